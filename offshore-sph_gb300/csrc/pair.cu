@@ -1,4 +1,5 @@
-// pair.cu -- the fused pair interaction of the WCSPH step.
+// pair.cu -- the fused pair interaction of the WCSPH step, mixed form (the
+// FP64 form's kernel is in pair64.cu).
 //
 // One thread per cell-sorted fluid particle i evaluates in one pass
 // everything _loop computes per particle (src/Tools/SolverTools.py:143-173):
@@ -17,128 +18,14 @@
 //      truncation bound) and append the survivors to a per-thread list in
 //      shared memory;
 //   2. evaluate the pair physics over the list, after the exact test.
-// FP64 form: phase 2 redoes the reference's neighbour test exactly
-// (q = r / h_ij <= 3 with correctly rounded operations) and its arithmetic.
-// Mixed form: phase 2 runs in FP32 on double-float differences of the FP64
-// state.
+// Phase 2 runs in FP32 on double-float differences of the FP64 state.
 #include <math.h>
 
 #include <type_traits>
 
-#include "sph_internal.cuh"
+#include "pair_common.cuh"
 
 namespace sph {
-
-constexpr int kPairBlock = 128;
-// per-thread neighbour-list capacity: above the typical number of pairs inside
-// the support (about 21 for the cubic spline at h = 1.3 dx, 43 for the
-// Gaussian cut at 3h), so that the mid-walk flush -- which runs divergently --
-// stays rare
-template <int KERNEL>
-struct ListCap {
-  static constexpr int value = Support<KERNEL>::q == 2 ? 32 : 64;
-};
-#ifndef SPH_PAIR_MIXED_BLOCKS
-#define SPH_PAIR_MIXED_BLOCKS 8
-#endif
-
-
-// Exact size of the reference's neighbour set of a query whose own cell is
-// not in its stencil (x-overflow alias) or whose h is not positive; those are
-// the only queries that can have an empty set (src/Tools/SolverTools.py:150-153).
-__device__ int exact_count(const StepArgs &a, const int *__restrict__ perm, const DevGrid &g, int2 qref, int qkey,
-                           int W, bool filter, const int2 *__restrict__ meta, const unsigned int *__restrict__ cstart,
-                           double xi, double yi, double hi) {
-  const Stencil sten(g, qref, qkey, W);
-  int cnt = 0;
-  for_stencil(sten, cstart, [&](unsigned int j) {
-    if (filter && !in_ref_stencil(meta, j, g, qref)) return;
-    const int pj = perm[j];
-    const double dx = xi - a.x[pj], dy = yi - a.y[pj];
-    const double r = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
-    const double q = __ddiv_rn(r, __dmul_rn(0.5, __dadd_rn(hi, a.h[pj])));
-    if (q <= 3.0) cnt++;
-  });
-  return cnt;
-}
-
-// TimeStep epilogue: the block's max a^2 over fluid; the last block computes
-// {dt, dt_courant, dt_force} (TimeStep.py:7-56) from the min h the records
-// pass gathered, and resets the slots.
-__device__ __forceinline__ void timestep_epilogue(DevCtrl *ctrl, unsigned long long ea, double co, double cfl_c,
-                                                  double cfl_f, double *dt_out, double *dt_hist,
-                                                  unsigned int *zero_on_last = nullptr,
-                                                  unsigned int nblocks = 0 /* 0: every block of the grid */) {
-  __shared__ unsigned long long red[kPairBlock / 32];
-  __shared__ bool last;
-  const unsigned int nb = nblocks ? nblocks : gridDim.x;
-  const unsigned long long wm = warp_max_u64(ea);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = wm;
-  __syncthreads();
-  unsigned long long ba = kEncMaxId;
-  if (threadIdx.x == 0) {
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) ba = red[w] > ba ? red[w] : ba;
-    if (nb == 1) {
-      last = true;
-    } else {
-      if (ba != kEncMaxId) atomicMax(&ctrl->pd_a2max, ba);
-      __threadfence();
-      last = atomicAdd(&ctrl->done_pair, 1u) == nb - 1;
-    }
-  }
-  __syncthreads();
-  if (last && threadIdx.x == 0) {
-    unsigned long long eh, ea2;
-    unsigned int cnt;
-    if (nb == 1) {
-      // the only block: the other contributions came from kernels that
-      // completed before this one started, so plain loads see them (one
-      // round trip instead of a fence and a chain of returning atomics)
-      eh = __ldcg(&ctrl->pd_hmin);
-      ea2 = __ldcg(&ctrl->pd_a2max);
-      cnt = __ldcg(&ctrl->pd_nfluid);
-      ea2 = ba > ea2 ? ba : ea2;
-      ctrl->pd_hmin = kEncMinId;
-      ctrl->pd_a2max = kEncMaxId;
-      ctrl->pd_nfluid = 0u;
-    } else {
-      __threadfence();
-      eh = atomicExch(&ctrl->pd_hmin, kEncMinId);
-      ea2 = atomicExch(&ctrl->pd_a2max, kEncMaxId);
-      cnt = atomicExch(&ctrl->pd_nfluid, 0u);
-      atomicExch(&ctrl->done_pair, 0u);
-    }
-    if (zero_on_last) *zero_on_last = 0u;
-    const double min_h = dec_d(eh);
-    const double max_a2 = dec_d(ea2);
-    const double max_c = co;  // compute_speed_of_sound gives co to every particle (WCSPH.py:110-129)
-    double dc = __ddiv_rn(__dmul_rn(cfl_c, min_h), max_c);
-    double df = max_a2 < 1e-12 ? 1e10 : __dmul_rn(cfl_f, __dsqrt_rn(__ddiv_rn(min_h, max_a2)));
-    double dt = (df < dc) ? df : dc;  // Python min(c, f) keeps c on ties
-    unsigned st = 0;
-    if (cnt == 0) {
-      st |= SPH_STATUS_NO_FLUID;
-      dt = dc = df = nan("");
-    }
-    if (dt < 1e-6) st |= SPH_STATUS_SMALL_DT;
-    if (st) atomicOr(&ctrl->status, st);
-    if (dt_out) {
-      dt_out[0] = dt;
-      dt_out[1] = dc;
-      dt_out[2] = df;
-    }
-    if (dt_hist) {
-      dt_hist[0] = dt;
-      dt_hist[1] = dc;
-      dt_hist[2] = df;
-    }
-  }
-}
-
-// a^2 as TimeStep.computeVars forms it (no contraction)
-__device__ __forceinline__ double accel2(double ax, double ay) {
-  return __dadd_rn(__dmul_rn(ax, ax), __dmul_rn(ay, ay));
-}
 
 // ---------------------------------------------------------------------------
 // Mixed-form pair physics, shared by the tile kernel and the global-path
@@ -370,27 +257,10 @@ __device__ __forceinline__ unsigned long long mixed_store(const MixedAcc &acc, c
   return enc_d(f2d(axs * axs + ayg * ayg));
 }
 
-struct PairPtrs {
-  const float4 *rec0, *rec1, *rec2;
-  const double4_32a *r64a, *r64b;
-  const int *perm, *keys_sorted;
-  const int2 *meta;
-  const unsigned int *cstart;
-  const DevGrid *grid;
-  DevCtrl *ctrl;
-};
-
-// resident blocks per SM the register allocation targets: the mixed form is
-// latency-bound and wants occupancy; the FP64 form is FP64-issue-bound
-template <bool MIXED>
-struct PairOcc {
-  static constexpr int blocks = MIXED ? SPH_PAIR_MIXED_BLOCKS : 4;
-};
-
 // Global-path evaluation of query slot k (all candidate records read from
 // global memory); returns the encoded a^2 of a fluid query, else the max
 // identity.  lists: the block's per-thread candidate lists.
-template <int KERNEL, bool XSPH, bool SUMDENS, bool MIXED, bool UH = false>
+template <int KERNEL, bool XSPH, bool SUMDENS, bool UH>
 __device__ __forceinline__ unsigned long long pair_query(const StepArgs &a, const PairPtrs &P, const PairParams &pp,
                                                          const DevGrid &g, bool filter, long long k,
                                                          unsigned int (*lists)[kPairBlock], int cell0 = 0) {
@@ -411,97 +281,16 @@ __device__ __forceinline__ unsigned long long pair_query(const StepArgs &a, cons
       const int qkey = P.keys_sorted[k] - cell0;
       const bool slow = qref.x >= g.ncx || !(hif > 0.f);
       const int W = g.mode == 0 ? 1 : (slow ? g.wide : g.wt);
-      // query state
-      double xi = 0, yi = 0, vxi = 0, vyi = 0, rhoi = 0, slf = 0, hi = 0;
-      float4 Ri = make_float4(0, 0, 0, 0), Vi = make_float4(0, 0, 0, 0);
-      if (MIXED) {
-        Ri = P.rec1[k];  // x_lo, y_lo, rho, p / rho^2
-        Vi = P.rec2[k];
-      } else {
-        const double4_32a A = P.r64a[k], B = P.r64b[k];
-        xi = A.x; yi = A.y; vxi = A.z; vyi = A.w;
-        rhoi = B.y; slf = B.z; hi = B.w;
-      }
-      // accumulators: FP32 (mixed) or FP64
+      const float4 Ri = P.rec1[k], Vi = P.rec2[k];  // x_lo, y_lo, rho, p / rho^2; velocities
       MixedAcc acc;
       const MixedConsts mc = mixed_consts<KERNEL>(pp);
       const UniformQ uq = uniform_q<KERNEL>(mc, hif);
-      double dd = 0.0, dax = 0.0, day = 0.0, dbx = 0.0, dby = 0.0, dsx = 0.0, dsy = 0.0, dfr = 0.0;
 
       // ---- phase 2: pair physics over the list
       auto physics = [&](int cnt) {
         for (int t = 0; t < cnt; t++) {
           const unsigned int j = lists[t][tid];
-          if (MIXED) {
-            mixed_entry<KERNEL, XSPH, SUMDENS, UH>(acc, mc, uq, Qi, Ri, Vi, P.rec0[j], P.rec1[j], P.rec2 + j);
-          } else {
-            const double4_32a A = P.r64a[j], B = P.r64b[j];
-            const double dx = xi - A.x, dy = yi - A.y;
-            const double d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
-            const double hij = __dmul_rn(0.5, __dadd_rn(hi, fabs(B.w)));
-            const double r = __dsqrt_rn(d2);
-            const double q = __ddiv_rn(r, hij);
-            if (!(q <= 3.0)) continue;  // NNLinkedList.py:74
-            const bool jf = !signbit(B.w);
-            const double mj = B.x, rhoj = B.y;
-            const double vxij = vxi - A.z, vyij = vyi - A.w;
-            double w = 0.0, coef = 0.0;
-            if (KERNEL == SPH_KERNEL_CUBIC) {
-              if (q <= 2.0) {
-                const double al = kCubicFac / (hij * hij);
-                if (q > 1.0) {
-                  const double t2 = 2.0 - q;
-                  w = al * 0.25 * (t2 * t2 * t2);
-                  if (r >= 1e-10) coef = al * (-0.75 * (t2 * t2)) / (hij * r);
-                } else {
-                  w = al * (1.0 - 1.5 * (q * q) * (1.0 - 0.5 * q));
-                  if (r >= 1e-10) coef = al * (-3.0 * q * (1.0 - 0.75 * q)) / (hij * r);
-                }
-              }
-            } else if (KERNEL == SPH_KERNEL_WENDLAND) {
-              w = wendland_w(r, hij);
-              coef = wendland_gcoef(r, hij);
-            } else {
-              const double ac = kInvPi / (hij * hij);
-              const double e = exp(-q * q);
-              w = ac * e;
-              const double tmp = r * hij;
-              if (tmp > 1e-12) coef = (-2.0 * q * ac * e) / tmp;
-            }
-            const double dwx = coef * dx, dwy = coef * dy;
-            if (jf) {
-              if (!SUMDENS) dd += mj * (vxij * dwx + vyij * dwy);
-              const double dot = vxij * dx + vyij * dy;
-              double PI = 0.0;
-              if (dot < 0.0) {
-                const double hb = 0.5 * (hi + hij);
-                const double mu = hb * dot / (r * r + 0.01 * hb * hb);
-                PI = mu * (pp.beta * mu - pp.alpha * (0.5 * pp.co)) / (0.5 * (rhoi + rhoj));
-              }
-              const double fac = slf + B.z + PI;
-              dax += -mj * fac * dwx;
-              day += -mj * fac * dwy;
-            } else if (r <= pp.r0 && r > 1e-12) {
-              const double frac = pp.r0 / r;
-              double tmp;
-              if (pp.lj_42) {
-                const double f2 = frac * frac;
-                tmp = f2 * f2 - f2;
-              } else {
-                tmp = pow(frac, pp.p1) - pow(frac, pp.p2);
-              }
-              const double fac = pp.D * tmp;
-              const double r2 = r * r;
-              dbx += fac * dx / r2;
-              dby += fac * dy / r2;
-              if (pp.fr && A.x >= pp.wall_x) dfr += fac * dx / r2;
-            }
-            if (XSPH) {
-              const double fac = -pp.eps * mj * w / (0.5 * (rhoi + rhoj));
-              dsx += fac * vxij;
-              dsy += fac * vyij;
-            }
-          }
+          mixed_entry<KERNEL, XSPH, SUMDENS, UH>(acc, mc, uq, Qi, Ri, Vi, P.rec0[j], P.rec1[j], P.rec2 + j);
         }
       };
 
@@ -530,48 +319,13 @@ __device__ __forceinline__ unsigned long long pair_query(const StepArgs &a, cons
 
       // the reference's set always holds the particle itself, except for the
       // slow queries, whose set size is counted exactly
-      bool any = true;
-      if (slow) {
-        if (MIXED) {
-          xi = a.x[i];
-          yi = a.y[i];
-          hi = a.h[i];
-        }
-        any = exact_count(a, P.perm, g, qref, qkey, W, g.mode == 1, P.meta, cst, xi, yi, hi) > 0;
-      }
-      if (any) {
-        if (MIXED) {
-          ea = mixed_store<XSPH, SUMDENS>(acc, a, i);
-        } else {
-          const double axf = dax + dbx;
-          const double ayf = (day - 9.81) + dby;
-          a.drho[i] = SUMDENS ? 0.0 : dd;
-          a.xsphx[i] = XSPH ? vxi + dsx : 0.0;
-          a.xsphy[i] = XSPH ? vyi + dsy : 0.0;
-          ea = enc_d(accel2(axf, ayf));
-          a.ax[i] = axf;
-          a.ay[i] = ayf;
-          if (pp.fr) pp.fr[i] = -P.r64b[k].x * dfr;
-        }
-      } else {
-        ea = enc_d(accel2(a.ax[i], a.ay[i]));  // keeps its previous values (SolverTools.py:150-153)
-        if (!MIXED && pp.fr) pp.fr[i] = 0.0;
-      }
+      const bool any = !slow || exact_count(a, P.perm, g, qref, qkey, W, g.mode == 1, P.meta, cst, a.x[i], a.y[i],
+                                            a.h[i]) > 0;
+      if (any) ea = mixed_store<XSPH, SUMDENS>(acc, a, i);
+      else ea = enc_d(accel2(a.ax[i], a.ay[i]));  // keeps its previous values (SolverTools.py:150-153)
     }
   }
   return ea;
-}
-
-template <int KERNEL, bool XSPH, bool SUMDENS, bool MIXED>
-__global__ void __launch_bounds__(kPairBlock, PairOcc<MIXED>::blocks)
-    k_pair(StepArgs a, PairPtrs P, PairParams pp, double *dt_out, double *dt_hist) {
-  __shared__ unsigned int lists[ListCap<KERNEL>::value][kPairBlock];
-  const DevGrid g = *P.grid;
-  const bool filter = g.mode == 1 && (g.need_filter || P.ctrl->alias_count > 0);
-  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  unsigned long long ea = kEncMaxId;
-  if (k < pp.n) ea = pair_query<KERNEL, XSPH, SUMDENS, MIXED>(a, P, pp, g, filter, k, lists);
-  if (pp.do_dt) timestep_epilogue(P.ctrl, ea, pp.co, pp.cfl_c, pp.cfl_f, dt_out, dt_hist);
 }
 
 // The queries the tile kernel left over (slot ranges of at most kPairBlock
@@ -600,7 +354,7 @@ __global__ void __launch_bounds__(kPairBlock, kListBlocks)
       const int2 r = fb[e];
       if ((int)threadIdx.x < r.y) {
         const unsigned long long q =
-            pair_query<KERNEL, XSPH, SUMDENS, true, UH>(a, P, pp, g, filter, r.x + threadIdx.x, lists);
+            pair_query<KERNEL, XSPH, SUMDENS, UH>(a, P, pp, g, filter, r.x + threadIdx.x, lists);
         ea = q > ea ? q : ea;
       }
     }
@@ -1265,8 +1019,8 @@ __global__ void __launch_bounds__(kPairBlock, kListBlocks)
     unsigned long long ea = kEncMaxId;
     if ((int)threadIdx.x < r.y)
       ea = pp.beta == 0.0
-               ? pair_query<KERNEL, XSPH, SUMDENS, true, true>(a, P, pp, g, filter, r.x + threadIdx.x, lists, B.coff[b])
-               : pair_query<KERNEL, XSPH, SUMDENS, true, false>(a, P, pp, g, filter, r.x + threadIdx.x, lists, B.coff[b]);
+               ? pair_query<KERNEL, XSPH, SUMDENS, true>(a, P, pp, g, filter, r.x + threadIdx.x, lists, B.coff[b])
+               : pair_query<KERNEL, XSPH, SUMDENS, false>(a, P, pp, g, filter, r.x + threadIdx.x, lists, B.coff[b]);
     const unsigned long long ba = block_max_u64<kPairBlock>(ea, red);
     if (threadIdx.x == 0 && ba != kEncMaxId) atomicMax(&B.sl[b].pd_a2max, ba);
   }
@@ -1414,27 +1168,6 @@ void launch_probe_density(const StepArgs &a, const WsPtrs &w, int kernel, long l
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
-static PairPtrs pair_ptrs(const WsPtrs &w) {
-  PairPtrs P;
-  P.rec0 = w.rec0; P.rec1 = w.rec1; P.rec2 = w.rec2; P.r64a = w.rec64a; P.r64b = w.rec64b;
-  P.perm = w.perm; P.keys_sorted = w.keys_sorted; P.meta = w.meta; P.cstart = w.cstart;
-  P.grid = w.grid; P.ctrl = w.ctrl;
-  return P;
-}
-
-static PairParams pair_params(const StepArgs &a, const sph_config_t &cfg, const sph_wcsph_t &wc, bool do_dt) {
-  PairParams pp;
-  pp.wall_x = 0.0;
-  pp.fr = nullptr;
-  pp.alpha = wc.alpha; pp.beta = wc.beta; pp.co = wc.co; pp.eps = wc.epsilon;
-  pp.r0 = wc.r0; pp.D = wc.D; pp.p1 = wc.p1; pp.p2 = wc.p2;
-  pp.lj_42 = (wc.p1 == 4.0 && wc.p2 == 2.0) ? 1 : 0;
-  pp.cfl_c = cfg.cfl_c; pp.cfl_f = cfg.cfl_f;
-  pp.do_dt = do_dt ? 1 : 0;
-  pp.n = a.n;
-  return pp;
-}
-
 int sm_count() {
   static int cache[64] = {0};
   int dev = 0;
@@ -1480,17 +1213,10 @@ static void mixed_pair_launch(const StepArgs &a, const WsPtrs &w, const PairPara
 template <int KERNEL, bool XSPH, bool SUMDENS>
 static void pair_dispatch(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, const PairParams &pp,
                           double *dt_out, double *dt_hist, cudaStream_t st) {
-  if (cfg.precision == SPH_PREC_MIXED) {
-    // a fixed h makes every fluid record's h the same (the uniform-h form,
-    // taken when the viscosity's beta is 0)
-    if (cfg.h_fixed > 0.0 && pp.beta == 0.0) mixed_pair_launch<KERNEL, XSPH, SUMDENS, true>(a, w, pp, dt_out, dt_hist, st);
-    else mixed_pair_launch<KERNEL, XSPH, SUMDENS, false>(a, w, pp, dt_out, dt_hist, st);
-  } else {
-    // one query per thread; below a few blocks per SM, one-warp blocks so
-    // that the FP64-bound work spreads evenly over the SMs
-    const int bs = a.n < (long long)sm_count() * kPairBlock * 8 ? 32 : kPairBlock;
-    k_pair<KERNEL, XSPH, SUMDENS, false><<<nblocks(a.n, bs), bs, 0, st>>>(a, pair_ptrs(w), pp, dt_out, dt_hist);
-  }
+  // a fixed h makes every fluid record's h the same (the uniform-h form,
+  // taken when the viscosity's beta is 0)
+  if (cfg.h_fixed > 0.0 && pp.beta == 0.0) mixed_pair_launch<KERNEL, XSPH, SUMDENS, true>(a, w, pp, dt_out, dt_hist, st);
+  else mixed_pair_launch<KERNEL, XSPH, SUMDENS, false>(a, w, pp, dt_out, dt_hist, st);
 }
 
 void launch_pair(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, const sph_wcsph_t &wc,
@@ -1499,6 +1225,10 @@ void launch_pair(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, co
   if (wall) {
     pp.wall_x = wall->wall_x;
     pp.fr = wall->fr;
+  }
+  if (cfg.precision != SPH_PREC_MIXED) {
+    launch_pair64(a, w, cfg, wc, pp, dt_out, dt_hist, st);
+    return;
   }
   const bool xs = wc.use_xsph != 0, sd = wc.use_summation_density != 0;
   auto go = [&](auto kern) {

@@ -1,0 +1,568 @@
+// pair64.cu -- the FP64 form of the fused pair interaction (the physics of
+// pair.cu's header comment, in FP64 arithmetic).
+//
+// What bounds it: the FP64 pipe.  It takes 16 cycles per warp instruction
+// (2 lanes per SM and cycle), so one FP64 operation costs as much issue time
+// as some sixty FP32 or integer ones, and the kernel's time is the number of
+// FP64 operations per pair.  So:
+//   - candidates are filtered in FP32 (padded) and compared on the integer
+//     pipe (positive doubles order like their bits);
+//   - reciprocals and square roots are one Halley step (cubic convergence)
+//     on the 2^-20 hardware estimate, not the compiler's divide and square
+//     root: 1/x in 3 operations, r and 1/r together in 6, each to about an
+//     ulp.  The neighbour test q = r / h_ij <= 3 (NNLinkedList.py:74) is redone
+//     with correctly rounded operations where an estimate could decide it
+//     differently;
+//   - with a uniform fluid h (Solver(h=...)) and beta = 0, the kernel gradient
+//     is a polynomial in r and 1/r whose coefficients are launch constants,
+//     and boundary neighbours beyond the Lennard-Jones reach are not listed
+//     (without XSPH they contribute nothing).
+// A pair of the cubic spline so takes 31 FP64 operations instead of about 90:
+// the 1M-fluid dam break's pair stage fell from 3.67 to 1.27 ms, and 20 steps
+// of 3200 fluid particles from 2.40 to 0.82 ms (with several lanes per query).
+#include <math.h>
+
+#include <type_traits>
+
+#include "pair_common.cuh"
+
+namespace sph {
+
+// ---------------------------------------------------------------------------
+// FP64 building blocks
+// ---------------------------------------------------------------------------
+// hardware estimates of 1/x and 1/sqrt(x) (normal x): the result's upper word
+__device__ __forceinline__ double rcp_est(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+__device__ __forceinline__ double rsqrt_est(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+// 1/x: y (1 + e + e^2), e = 1 - x y; the estimate's error cubed is far below
+// an ulp
+__device__ __forceinline__ double rcp64(double x) {
+  const double y = rcp_est(x);
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+// r = sqrt(x) and ir = 1/sqrt(x): y (1 + e/2 + 3/8 e^2), e = 1 - x y^2
+__device__ __forceinline__ void sqrt_rsqrt64(double x, double &r, double &ir) {
+  const double y = rsqrt_est(x);
+  const double t = x * y;
+  const double e = fma(-t, y, 1.0);
+  const double c = fma(0.375, e, 0.5) * e;
+  r = fma(t, c, t);
+  ir = fma(y, c, y);
+}
+
+// a <= b for non-negative doubles (false when either is NaN and a is not
+// below b's pattern), without an FP64 instruction
+__device__ __forceinline__ bool le_bits(double a, double b) {
+  return (unsigned long long)__double_as_longlong(a) <= (unsigned long long)__double_as_longlong(b);
+}
+
+// exp(-z) for 0 <= z < 16: table lookup and a short polynomial (P. T. P. Tang,
+// Table-driven implementation of the exponential function in IEEE
+// floating-point arithmetic, ACM TOMS 15, 1989), with 2048 entries so that a
+// cubic suffices: z = (n ln 2) / 2048 + s, |s| <= 1.7e-4,
+// exp(-z) = 2^(-n / 2048) (1 - s + s^2 / 2 - s^3 / 6) to 4e-17.  The index
+// comes from FP32, so the FP64 pipe sees 6 operations.
+constexpr int kExpN = 2048;
+struct ExpTable {
+  double v[kExpN];
+};
+struct DD {
+  double hi, lo;
+};
+constexpr DD dd_two_prod(double a, double b) {  // Dekker's product
+  const double p = a * b;
+  const double c1 = 134217729.0 * a, c2 = 134217729.0 * b;
+  const double ah = c1 - (c1 - a), bh = c2 - (c2 - b);
+  const double al = a - ah, bl = b - bh;
+  return {p, ((ah * bh - p) + ah * bl + al * bh) + al * bl};
+}
+constexpr DD dd_mul(DD a, DD b) {
+  const DD p = dd_two_prod(a.hi, b.hi);
+  const double l = p.lo + (a.hi * b.lo + a.lo * b.hi);
+  const double s = p.hi + l;
+  return {s, l - (s - p.hi)};
+}
+// ln 2 in three parts: the first with its last 20 bits zero, so that n times
+// it is exact for n < 2^16
+constexpr double kLn2Hi = 0x1.62e42fefp-1, kLn2Lo = 0x1.473de6af278edp-34;
+constexpr ExpTable make_exp_table() {
+  // c = 2^(-1/2048) = exp(-ln 2 / 2048) as a double-double Taylor sum
+  const DD x = {-0x1.62e42fefa39efp-1 / kExpN, -0x1.abc9e3b39803fp-56 / kExpN};
+  DD term = {1.0, 0.0}, c = {1.0, 0.0};
+  for (int k = 1; k <= 8; k++) {
+    term = dd_mul(term, x);
+    const DD inv = {1.0 / k, 0.0};
+    // term / k with one correction of the quotient
+    const DD q0 = dd_mul(term, inv);
+    const DD back = dd_mul(q0, DD{(double)k, 0.0});
+    const double fix = ((term.hi - back.hi) + (term.lo - back.lo)) / k;
+    const double qh = q0.hi + (q0.lo + fix);
+    term = DD{qh, (q0.lo + fix) - (qh - q0.hi)};
+    const double s = c.hi + term.hi;
+    const double err = (c.hi - s) + term.hi;
+    const double lo = err + (c.lo + term.lo);
+    const double s2 = s + lo;
+    c = DD{s2, lo - (s2 - s)};
+  }
+  ExpTable t = {};
+  DD v = {1.0, 0.0};
+  for (int i = 0; i < kExpN; i++) {
+    t.v[i] = v.hi;
+    v = dd_mul(v, c);
+  }
+  return t;
+}
+__device__ constexpr ExpTable g_exp_table = make_exp_table();
+
+__device__ __forceinline__ double exp_neg(double z) {
+  const float nf = fmaf(d2f_trunc(z), (float)(kExpN / 0.693147180559945309417), 12582912.0f);
+  const int n = (int)(__float_as_uint(nf) - 0x4B400000u);
+  const double nd = f2d(nf - 12582912.0f);
+  double s = fma(nd, -kLn2Hi / kExpN, z);
+  s = fma(nd, -kLn2Lo / kExpN, s);
+  const double p = fma(s, -1.0 / 6.0, 0.5);
+  const double t = fma(s * s, p, -s);
+  const double T = __ldg(&g_exp_table.v[n & (kExpN - 1)]);
+  const double b = __hiloint2double(__double2hiint(T) - ((n >> 11) << 20), __double2loint(T));
+  return fma(b, t, b);
+}
+
+// ---------------------------------------------------------------------------
+// Launch constants
+// ---------------------------------------------------------------------------
+struct Pair64 {
+  int xsph, sumdens;
+  // uniform fluid h (UH)
+  double h, ih, lim;           // h, 1/h, (support h)^2
+  double lim_lo, lim_hi;       // Gaussian: below / above, q <= 3 is decided
+  double h2;                   // cubic: d2 <= h^2 is the inner piece.  Gaussian: d2 <= h2 has no gradient
+  double o_ir, o_r, o_0;       // cubic, outer piece: o_ir / r + o_r r + o_0
+  double i_r, i_0;             // inner piece: i_r r + i_0.  Wendland: (i_r r + i_0) (1 + o_r r)^5
+  double al;                   // normalisation of W
+  double hb2, pic;             // viscosity: pic dot / ((d2 + hb2) (rho_i + rho_j))
+  double r02;                  // r0^2
+  int lj_free;                 // r0 < 1.5 h: the Lennard-Jones pairs all have q <= 3
+};
+
+static Pair64 pair64_consts(const sph_config_t &cfg, const sph_wcsph_t &wc) {
+  Pair64 c;
+  c.xsph = wc.use_xsph != 0;
+  c.sumdens = wc.use_summation_density != 0;
+  const double h = cfg.h_fixed > 0.0 ? cfg.h_fixed : 1.0;
+  const double ih = 1.0 / h, ih2 = ih * ih;
+  c.h = h;
+  c.ih = ih;
+  c.h2 = h * h;
+  c.o_ir = c.o_r = c.o_0 = c.i_r = c.i_0 = 0.0;
+  if (cfg.kernel == SPH_KERNEL_CUBIC) {
+    // al / (h r) times -0.75 (2 - q)^2 and -3 q (1 - 0.75 q) (CubicSpline.py:40-70)
+    c.al = kCubicFac * ih2;
+    c.lim = 4.0 * h * h;
+    c.o_ir = -3.0 * c.al * ih;
+    c.o_0 = 3.0 * c.al * ih2;
+    c.o_r = -0.75 * c.al * ih2 * ih;
+    c.i_0 = -3.0 * c.al * ih2;
+    c.i_r = 2.25 * c.al * ih2 * ih;
+  } else if (cfg.kernel == SPH_KERNEL_WENDLAND) {
+    // al / (h r) (1 - q/2)^5 (-14/3) q (1 + 2.5 q) (Wendland.py:36-64)
+    c.al = kWendFac * ih2;
+    c.lim = 4.0 * h * h;
+    c.o_r = -0.5 * ih;
+    c.i_0 = (-14.0 / 3.0) * c.al * ih2;
+    c.i_r = (-35.0 / 3.0) * c.al * ih2 * ih;
+  } else {
+    // -2 al / h^2 exp(-q^2) (Gaussian.py:37-59)
+    c.al = kInvPi * ih2;
+    c.lim = 9.0 * h * h;
+    c.i_0 = -2.0 * c.al * ih2;
+    c.h2 = 1e-24 * ih2;  // r h <= 1e-12: no gradient
+  }
+  c.lim_lo = c.lim * (1.0 - 1e-9);
+  c.lim_hi = c.lim * (1.0 + 1e-9);
+  c.hb2 = 0.01 * (h * h);
+  c.pic = -wc.alpha * wc.co * h;  // -2 alpha c_ij h with c_ij = co / 2
+  c.r02 = wc.r0 * wc.r0;
+  c.lj_free = cfg.h_fixed > 0.0 && wc.r0 < 1.5 * h * (1.0 - 1e-9);
+  return c;
+}
+
+// q = r / h_ij <= 3 as the reference decides it
+static __device__ __noinline__ bool near_exact(double dx, double dy, double hij) {
+  const double r = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
+  return __ddiv_rn(r, hij) <= 3.0;
+}
+
+struct Acc64 {
+  double dd = 0.0, ax = 0.0, ay = 0.0, sx = 0.0, sy = 0.0, fr = 0.0;
+};
+
+// The query's state (FP64 records).
+struct Query64 {
+  double x, y, vx, vy, rho, oth, h;
+};
+
+// One listed candidate j of query q: the exact support test, then
+// continuity, momentum with artificial viscosity, the Lennard-Jones boundary
+// force and XSPH.  UH: every fluid h is c.h and beta = 0.
+template <int KERNEL, bool UH>
+__device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 &c, const PairParams &pp,
+                                       const double4_32a &A, const double4_32a &B) {
+  constexpr bool gauss = KERNEL == SPH_KERNEL_GAUSSIAN;
+  const double dx = q.x - A.x, dy = q.y - A.y;
+  const double d2 = fma(dx, dx, dy * dy);
+  const bool fluid = !signbit(B.w);
+  if (fluid) {
+    double coef, w = 0.0, hij = c.h, ih = c.ih;
+    if constexpr (UH) {
+      if constexpr (gauss) {
+        if (!le_bits(d2, c.lim_lo) && (!le_bits(d2, c.lim_hi) || !near_exact(dx, dy, hij))) return;
+        const double e = exp_neg(d2 * (ih * ih));
+        coef = le_bits(d2, c.h2) ? 0.0 : c.i_0 * e;
+        if (c.xsph) w = c.al * e;
+      } else {
+        if (!le_bits(d2, c.lim)) return;  // W and its gradient are 0 at q >= 2
+        double r, ir;
+        sqrt_rsqrt64(d2, r, ir);
+        const bool tiny = le_bits(d2, 1e-20);  // r < 1e-10: no gradient
+        if (KERNEL == SPH_KERNEL_CUBIC) {
+          if (le_bits(d2, c.h2)) coef = fma(c.i_r, r, c.i_0);
+          else coef = fma(c.o_ir, ir, fma(c.o_r, r, c.o_0));
+        } else {
+          const double in = fma(c.o_r, r, 1.0), in2 = in * in;
+          coef = (in2 * in2) * (in * fma(c.i_r, r, c.i_0));
+        }
+        if (tiny) {
+          coef = 0.0;
+          r = 0.0;
+        }
+        if (c.xsph) {
+          const double qq = r * ih;
+          if (KERNEL == SPH_KERNEL_CUBIC) {
+            const double t = 2.0 - qq;
+            w = le_bits(d2, c.h2) ? c.al * (1.0 - 1.5 * (qq * qq) * (1.0 - 0.5 * qq)) : c.al * 0.25 * (t * t * t);
+          } else {
+            const double in = 1.0 - 0.5 * qq, in2 = in * in;
+            w = c.al * (in2 * in2 * in2 * ((35.0 / 12.0) * qq * qq + 3.0 * qq + 1.0));
+          }
+        }
+      }
+    } else {
+      hij = half_exact(q.h + B.w);  // both positive or zero
+      if (!(__double2hiint(hij) > 0)) return;  // q = r / 0
+      ih = rcp64(hij);
+      const double ih2 = ih * ih;
+      if constexpr (gauss) {
+        const double z = d2 * ih2;
+        if (!le_bits(z, 9.0 * (1.0 - 1e-9)) && (!le_bits(z, 9.0 * (1.0 + 1e-9)) || !near_exact(dx, dy, hij))) return;
+        const double e = kInvPi * ih2 * exp_neg(z);
+        coef = le_bits(d2, 1e-24 * ih2) ? 0.0 : -2.0 * e * ih2;
+        w = e;
+      } else {
+        double r, ir;
+        sqrt_rsqrt64(d2, r, ir);
+        const bool tiny = le_bits(d2, 1e-20);
+        if (tiny) r = 0.0;
+        const double qq = r * ih;
+        if (!le_bits(qq, 2.0)) return;
+        if (KERNEL == SPH_KERNEL_CUBIC) {
+          const double al = kCubicFac * ih2;
+          if (le_bits(qq, 1.0)) {
+            coef = (al * ih2) * fma(2.25, qq, -3.0);
+            if (c.xsph) w = al * (1.0 - 1.5 * (qq * qq) * (1.0 - 0.5 * qq));
+          } else {
+            const double t = 2.0 - qq, t2 = t * t;
+            coef = (-0.75 * al) * t2 * (ih * ir);
+            if (c.xsph) w = al * 0.25 * (t2 * t);
+          }
+        } else {
+          const double al = kWendFac * ih2;
+          const double in = fma(-0.5, qq, 1.0), in2 = in * in, in5 = in2 * in2 * in;
+          coef = (al * ih2) * in5 * fma(-35.0 / 3.0, qq, -14.0 / 3.0);
+          if (c.xsph) w = al * (in5 * in) * ((35.0 / 12.0) * qq * qq + 3.0 * qq + 1.0);
+        }
+        if (tiny) coef = 0.0;
+      }
+    }
+    const double vx = q.vx - A.z, vy = q.vy - A.w;
+    const double dot = fma(vx, dx, vy * dy);
+    const double mc = B.x * coef;
+    s.dd = fma(mc, dot, s.dd);
+    double S = q.oth + B.z;
+    const double rs = q.rho + B.y;  // 2 rho_ij
+    if (negative_bits(dot)) {
+      if constexpr (UH) {
+        S = fma(c.pic * dot, rcp64((d2 + c.hb2) * rs), S);
+      } else {
+        // mu = h v.r / (r^2 + 0.01 h^2), Pi = mu (beta mu - alpha c_ij) / rho_ij
+        const double hb = half_exact(q.h + hij);
+        const double den = fma(0.01 * hb, hb, d2);
+        const double inv = rcp64(den * rs);  // 1 / (den rs)
+        const double t = 2.0 * hb * dot * inv;  // mu / rho_ij
+        if (pp.beta == 0.0) S = fma(t, -0.5 * pp.alpha * pp.co, S);
+        else S = fma(t, fma(pp.beta, hb * dot * (inv * rs), -0.5 * pp.alpha * pp.co), S);
+      }
+    }
+    const double f = mc * S;
+    s.ax = fma(-f, dx, s.ax);
+    s.ay = fma(-f, dy, s.ay);
+    if (c.xsph) {
+      const double k = (-2.0 * pp.eps) * B.x * w * rcp64(rs);
+      s.sx = fma(k, vx, s.sx);
+      s.sy = fma(k, vy, s.sy);
+    }
+    return;
+  }
+  // a boundary neighbour: Lennard-Jones at 1e-12 < r <= r0 (the force is 0 at
+  // r0), and XSPH, which takes every neighbour (a massless one adds 0)
+  const bool lj = le_bits(d2, c.r02) && !le_bits(d2, 1e-24);
+  const bool xs = c.xsph && (B.x != 0.0);
+  if (!lj && !xs) return;
+  const double hj = fabs(B.w);
+  const double hij = 0.5 * (q.h + hj);
+  if (!(c.lj_free && lj) || xs) {  // the neighbour test
+    const double t = 3.0 * hij, t2 = t * t;
+    if (!le_bits(d2, t2 * (1.0 - 1e-9)) && (!le_bits(d2, t2 * (1.0 + 1e-9)) || !near_exact(dx, dy, hij))) return;
+    if (!(hij > 0.0)) return;
+  }
+  if (lj) {
+    const double ir2 = rcp64(d2);
+    double t;
+    if (pp.lj_42) {
+      const double f2 = c.r02 * ir2;
+      t = fma(f2, f2, -f2);
+    } else {
+      const double frac = pp.r0 / __dsqrt_rn(d2);
+      t = pow(frac, pp.p1) - pow(frac, pp.p2);
+    }
+    const double fac = pp.D * t * ir2;
+    s.ax = fma(fac, dx, s.ax);
+    s.ay = fma(fac, dy, s.ay);
+    if (pp.fr && A.x >= pp.wall_x) s.fr = fma(fac, dx, s.fr);
+  }
+  if (xs) {
+    const double r = __dsqrt_rn(d2);
+    const double w = KERNEL == SPH_KERNEL_CUBIC ? cubic_w(r, hij)
+                                                : (KERNEL == SPH_KERNEL_WENDLAND ? wendland_w(r, hij) : gauss_w(r, hij));
+    const double k = (-2.0 * pp.eps) * B.x * w * rcp64(q.rho + B.y);
+    s.sx = fma(k, q.vx - A.z, s.sx);
+    s.sy = fma(k, q.vy - A.w, s.sy);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The kernel.  G lanes share a query: they walk each stencil row G candidates
+// at a time, append the survivors of the FP32 test to the group's list in
+// candidate order (ballot), evaluate every G-th entry each and combine their
+// sums with shuffles.  G = 1 is one query per thread with a list of its own.
+// The sums of a query depend on G and its candidate order alone.
+// ---------------------------------------------------------------------------
+template <int KERNEL, bool UH, int G>
+__global__ void __launch_bounds__(kPairBlock, 4)
+    k_pair64(StepArgs a, PairPtrs P, PairParams pp, Pair64 c, double *dt_out, double *dt_hist) {
+  step_kernel_entry();
+  constexpr int kCap = (G == 1 ? 1 : 1.5) * ListCap<KERNEL>::value;
+  constexpr int kGroups = kPairBlock / G;
+  // G = 1: entry t of thread i at [t][i]; else entry t of group i at [i][t]
+  __shared__ unsigned int lists[kCap * kGroups];
+  const DevGrid &g = *P.grid;
+  const int tid = threadIdx.x;
+  const int gl = tid % G, grp = tid / G;
+  const long long k = ((long long)blockIdx.x * kPairBlock + tid) / G;
+  unsigned long long ea = kEncMaxId;
+  bool act = k < pp.n;
+  const float4 Qi = act ? P.rec0[k] : make_float4(0.f, 0.f, -1.f, 0.f);  // x_hi, y_hi, h (signed), m
+  const float hif = Qi.z;
+  act = act && !signbit(hif);
+  if (G > 1 ? __any_sync(0xffffffffu, act) : act) {
+    const bool filter = g.mode == 1 && (g.need_filter || P.ctrl->alias_count > 0);
+    const long long kq = act ? k : 0;
+    const int i = P.perm[kq];
+    const int2 qref = P.meta[kq];
+    const int qkey = P.keys_sorted[kq];
+    const bool slow = qref.x >= g.ncx || !(hif > 0.f);
+    const int W = g.mode == 0 ? 1 : (slow ? g.wide : g.wt);
+    const double4_32a A = P.r64a[kq], B = P.r64b[kq];
+    const Query64 q = {A.x, A.y, A.z, A.w, B.y, B.z, B.w};
+    Acc64 s;
+    // the FP32 test: the padded reach of the pair's h (kernel support; a
+    // boundary neighbour without XSPH: the Lennard-Jones reach min(r0, 3 h_ij))
+    const float SK = (float)Support<KERNEL>::q * 1.000002f;
+    const float r0f = (float)pp.r0, pad = g.pad_e;
+    const float rf = SK * hif + pad, rf2 = rf * rf;
+    auto near = [&](unsigned int j) {
+      if (j == (unsigned int)k) return false;  // the particle itself contributes zero
+      if (filter && !in_ref_stencil(P.meta, j, g, qref)) return false;
+      const float4 qj = P.rec0[j];
+      const float dx = Qi.x - qj.x, dy = Qi.y - qj.y;
+      const float d2 = dx * dx + dy * dy;
+      if (UH && !signbit(qj.z)) return d2 <= rf2;
+      const float hij = 0.5f * (hif + fabsf(qj.z));
+      float reach = SK * hij;
+      if (signbit(qj.z)) {
+        const float lj = fminf(r0f, 3.0f * hij) * 1.000002f;
+        reach = c.xsph ? fmaxf(reach, lj) : lj;
+      }
+      const float rp = reach + pad;
+      return d2 <= rp * rp;
+    };
+    const Stencil sten(g, qref, qkey, W);
+    if constexpr (G == 1) {
+      auto physics = [&](int cnt) {
+        for (int t = 0; t < cnt; t++) {
+          const unsigned int j = lists[t * kGroups + grp];
+          pair64<KERNEL, UH>(s, q, c, pp, P.r64a[j], P.r64b[j]);
+        }
+      };
+      int nl = 0;
+      for_stencil(sten, P.cstart, [&](unsigned int j) {
+        if (near(j)) {
+          lists[nl * kGroups + grp] = j;
+          if (++nl == kCap) {
+            physics(nl);
+            nl = 0;
+          }
+        }
+      });
+      physics(nl);
+    } else {
+      unsigned int *list = lists + grp * kCap;
+      const int lane = tid & 31;
+      const unsigned int gmask = (G == 32 ? 0xffffffffu : ((1u << G) - 1u)) << (lane & ~(G - 1));
+      const unsigned int below = gmask & ((1u << lane) - 1u);
+      int nl = 0;
+      auto physics = [&]() {
+        for (int t = gl; t < nl; t += G) {
+          const unsigned int j = list[t];
+          pair64<KERNEL, UH>(s, q, c, pp, P.r64a[j], P.r64b[j]);
+        }
+      };
+      // one run [j0, j1) of candidates per group and round; jump skips from
+      // e0 on (the second of two tile segments)
+      auto walk = [&](unsigned int j0, unsigned int j1, unsigned int e0, unsigned int jump) {
+        for (unsigned int j = j0 + gl; __any_sync(0xffffffffu, j - gl < j1); j += G) {
+          const unsigned int jj = j >= e0 ? j + jump : j;
+          const bool keep = j < j1 && near(jj);
+          const unsigned int b = __ballot_sync(0xffffffffu, keep) & gmask;
+          if (keep) list[nl + __popc(b & below)] = jj;
+          nl += __popc(b);
+          if (__any_sync(0xffffffffu, nl > kCap - G)) {  // no room for another round
+            __syncwarp();
+            if (nl > kCap - G) {
+              physics();
+              nl = 0;
+            }
+            __syncwarp();
+          }
+        }
+      };
+      const int rows = (int)__reduce_max_sync(0xffffffffu, (unsigned)max(act ? sten.y1 - sten.y0 + 1 : 0, 0));
+      const bool any_multi = __any_sync(0xffffffffu, act && sten.multi);
+      for (int r = 0; r < rows; r++) {
+        const int yy = sten.y0 + r;
+        const bool on = act && yy <= sten.y1;
+        const unsigned int *cs = P.cstart + (on ? sten.rowpart(yy) : 0);
+        if (!any_multi) {
+          unsigned int s0 = 0, e0 = 0, s1 = 0, e1 = 0;
+          if (on) {
+            s0 = __ldg(cs + sten.ca);
+            e0 = __ldg(cs + sten.cb);
+            s1 = __ldg(cs + sten.cc);
+            e1 = __ldg(cs + sten.cd);
+          }
+          walk(s0, e0 + (e1 - s1), e0, s1 - e0);
+        } else {
+          // columns over several tiles: the tiles one by one
+          const int m = (1 << sten.ts) - 1;
+          for (int xs = sten.x0; __any_sync(0xffffffffu, on && xs <= sten.x1); xs = (xs | m) + 1) {
+            unsigned int s0 = 0, e0 = 0;
+            if (on && xs <= sten.x1) {
+              s0 = __ldg(cs + Stencil::colpart(xs, sten.ts));
+              e0 = __ldg(cs + Stencil::colpart(min(sten.x1, xs | m), sten.ts) + 1);
+            }
+            walk(s0, e0, e0, 0u);
+          }
+        }
+      }
+      __syncwarp();
+      physics();
+      auto sum = [&](double &v) {
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      };
+      sum(s.dd);
+      sum(s.ax);
+      sum(s.ay);
+      if (c.xsph) {
+        sum(s.sx);
+        sum(s.sy);
+      }
+      if (pp.fr) sum(s.fr);
+    }
+    if (act && gl == 0) {
+      // the reference's set always holds the particle itself, except for the
+      // slow queries, whose set size is counted exactly
+      if (!slow || exact_count(a, P.perm, g, qref, qkey, W, g.mode == 1, P.meta, P.cstart, q.x, q.y, q.h) > 0) {
+        const double axf = s.ax, ayf = s.ay - 9.81;
+        a.drho[i] = c.sumdens ? 0.0 : s.dd;
+        a.xsphx[i] = c.xsph ? q.vx + s.sx : 0.0;
+        a.xsphy[i] = c.xsph ? q.vy + s.sy : 0.0;
+        ea = enc_d(accel2(axf, ayf));
+        a.ax[i] = axf;
+        a.ay[i] = ayf;
+        if (pp.fr) pp.fr[i] = -B.x * s.fr;
+      } else {
+        ea = enc_d(accel2(a.ax[i], a.ay[i]));  // keeps its previous values (SolverTools.py:150-153)
+        if (pp.fr) pp.fr[i] = 0.0;
+      }
+    }
+  }
+  if (pp.do_dt) timestep_epilogue(P.ctrl, ea, pp.co, pp.cfl_c, pp.cfl_f, dt_out, dt_hist);
+}
+
+template <int KERNEL, bool UH>
+static void pair64_launch(const StepArgs &a, const WsPtrs &w, const PairParams &pp, const Pair64 &c, double *dt_out,
+                          double *dt_hist, cudaStream_t st) {
+  // Lanes per query.  Sharing a query costs about a quarter more issue time
+  // (short groups, the final sums; dam break of 1M fluid particles: 1.27 ms
+  // with G = 1, 1.57 ms with G = 4) and divides the length of a thread's
+  // chain of dependent FP64 operations.  So G = 1 where the threads fill most
+  // of one wave of blocks (54K particles, Wendland: 786 us for 4 steps
+  // against 809 with G = 4) or several; G = 4 where the last wave would be
+  // nearly empty (99K, Gaussian: 361 us with G = 1, 325 with 4); G = 8 where
+  // the GPU is idle and the chain is the time (5K particles: 1415 us for 20
+  // steps with G = 1, 990 with 4, 820 with 8, 824 with 16).
+  const long long n = a.n, wave = (long long)sm_count() * kPairBlock * 4;
+  auto go = [&](auto lanes) {
+    constexpr int G = decltype(lanes)::value;
+    launch_pdl(k_pair64<KERNEL, UH, G>, dim3(nblocks(n * G, kPairBlock)), dim3(kPairBlock), 0, st, a, pair_ptrs(w), pp,
+               c, dt_out, dt_hist);
+  };
+  if (n < wave / 8) go(std::integral_constant<int, 8>());
+  else if (n < wave / 2 || (n > wave && n < 4 * wave)) go(std::integral_constant<int, 4>());
+  else go(std::integral_constant<int, 1>());
+}
+
+void launch_pair64(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, const sph_wcsph_t &wc,
+                   const PairParams &pp, double *dt_out, double *dt_hist, cudaStream_t st) {
+  const Pair64 c = pair64_consts(cfg, wc);
+  const bool uh = cfg.h_fixed > 0.0 && wc.beta == 0.0;
+  auto go = [&](auto kern) {
+    constexpr int K = decltype(kern)::value;
+    if (uh) pair64_launch<K, true>(a, w, pp, c, dt_out, dt_hist, st);
+    else pair64_launch<K, false>(a, w, pp, c, dt_out, dt_hist, st);
+  };
+  if (cfg.kernel == SPH_KERNEL_CUBIC) go(std::integral_constant<int, SPH_KERNEL_CUBIC>());
+  else if (cfg.kernel == SPH_KERNEL_WENDLAND) go(std::integral_constant<int, SPH_KERNEL_WENDLAND>());
+  else go(std::integral_constant<int, SPH_KERNEL_GAUSSIAN>());
+}
+
+}  // namespace sph

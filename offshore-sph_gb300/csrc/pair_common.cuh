@@ -1,0 +1,148 @@
+// pair_common.cuh -- what the pair kernels of both precision forms share:
+// their pointers and parameters, the exact neighbour count of the queries
+// that can have an empty set, and the TimeStep epilogue.
+#pragma once
+
+#include "sph_internal.cuh"
+
+namespace sph {
+
+constexpr int kPairBlock = 128;
+// per-thread neighbour-list capacity: above the typical number of pairs inside
+// the support (about 21 for the cubic spline at h = 1.3 dx, 43 for the
+// Gaussian cut at 3h), so that the mid-walk flush -- which runs divergently --
+// stays rare
+template <int KERNEL>
+struct ListCap {
+  static constexpr int value = Support<KERNEL>::q == 2 ? 32 : 64;
+};
+
+struct PairPtrs {
+  const float4 *rec0, *rec1, *rec2;
+  const double4_32a *r64a, *r64b;
+  const int *perm, *keys_sorted;
+  const int2 *meta;
+  const unsigned int *cstart;
+  const DevGrid *grid;
+  DevCtrl *ctrl;
+};
+
+inline PairPtrs pair_ptrs(const WsPtrs &w) {
+  PairPtrs P;
+  P.rec0 = w.rec0; P.rec1 = w.rec1; P.rec2 = w.rec2; P.r64a = w.rec64a; P.r64b = w.rec64b;
+  P.perm = w.perm; P.keys_sorted = w.keys_sorted; P.meta = w.meta; P.cstart = w.cstart;
+  P.grid = w.grid; P.ctrl = w.ctrl;
+  return P;
+}
+
+inline PairParams pair_params(const StepArgs &a, const sph_config_t &cfg, const sph_wcsph_t &wc, bool do_dt) {
+  PairParams pp;
+  pp.wall_x = 0.0;
+  pp.fr = nullptr;
+  pp.alpha = wc.alpha; pp.beta = wc.beta; pp.co = wc.co; pp.eps = wc.epsilon;
+  pp.r0 = wc.r0; pp.D = wc.D; pp.p1 = wc.p1; pp.p2 = wc.p2;
+  pp.lj_42 = (wc.p1 == 4.0 && wc.p2 == 2.0) ? 1 : 0;
+  pp.cfl_c = cfg.cfl_c; pp.cfl_f = cfg.cfl_f;
+  pp.do_dt = do_dt ? 1 : 0;
+  pp.n = a.n;
+  return pp;
+}
+
+// Exact size of the reference's neighbour set of a query whose own cell is
+// not in its stencil (x-overflow alias) or whose h is not positive; those are
+// the only queries that can have an empty set (src/Tools/SolverTools.py:150-153).
+static __device__ int exact_count(const StepArgs &a, const int *__restrict__ perm, const DevGrid &g, int2 qref, int qkey,
+                           int W, bool filter, const int2 *__restrict__ meta, const unsigned int *__restrict__ cstart,
+                           double xi, double yi, double hi) {
+  const Stencil sten(g, qref, qkey, W);
+  int cnt = 0;
+  for_stencil(sten, cstart, [&](unsigned int j) {
+    if (filter && !in_ref_stencil(meta, j, g, qref)) return;
+    const int pj = perm[j];
+    const double dx = xi - a.x[pj], dy = yi - a.y[pj];
+    const double r = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
+    const double q = __ddiv_rn(r, __dmul_rn(0.5, __dadd_rn(hi, a.h[pj])));
+    if (q <= 3.0) cnt++;
+  });
+  return cnt;
+}
+
+// TimeStep epilogue: the block's max a^2 over fluid; the last block computes
+// {dt, dt_courant, dt_force} (TimeStep.py:7-56) from the min h the records
+// pass gathered, and resets the slots.
+__device__ __forceinline__ void timestep_epilogue(DevCtrl *ctrl, unsigned long long ea, double co, double cfl_c,
+                                                  double cfl_f, double *dt_out, double *dt_hist,
+                                                  unsigned int *zero_on_last = nullptr,
+                                                  unsigned int nblocks = 0 /* 0: every block of the grid */) {
+  __shared__ unsigned long long red[kPairBlock / 32];
+  __shared__ bool last;
+  const unsigned int nb = nblocks ? nblocks : gridDim.x;
+  const unsigned long long wm = warp_max_u64(ea);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = wm;
+  __syncthreads();
+  unsigned long long ba = kEncMaxId;
+  if (threadIdx.x == 0) {
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++) ba = red[w] > ba ? red[w] : ba;
+    if (nb == 1) {
+      last = true;
+    } else {
+      if (ba != kEncMaxId) atomicMax(&ctrl->pd_a2max, ba);
+      __threadfence();
+      last = atomicAdd(&ctrl->done_pair, 1u) == nb - 1;
+    }
+  }
+  __syncthreads();
+  if (last && threadIdx.x == 0) {
+    unsigned long long eh, ea2;
+    unsigned int cnt;
+    if (nb == 1) {
+      // the only block: the other contributions came from kernels that
+      // completed before this one started, so plain loads see them (one
+      // round trip instead of a fence and a chain of returning atomics)
+      eh = __ldcg(&ctrl->pd_hmin);
+      ea2 = __ldcg(&ctrl->pd_a2max);
+      cnt = __ldcg(&ctrl->pd_nfluid);
+      ea2 = ba > ea2 ? ba : ea2;
+      ctrl->pd_hmin = kEncMinId;
+      ctrl->pd_a2max = kEncMaxId;
+      ctrl->pd_nfluid = 0u;
+    } else {
+      __threadfence();
+      eh = atomicExch(&ctrl->pd_hmin, kEncMinId);
+      ea2 = atomicExch(&ctrl->pd_a2max, kEncMaxId);
+      cnt = atomicExch(&ctrl->pd_nfluid, 0u);
+      atomicExch(&ctrl->done_pair, 0u);
+    }
+    if (zero_on_last) *zero_on_last = 0u;
+    const double min_h = dec_d(eh);
+    const double max_a2 = dec_d(ea2);
+    const double max_c = co;  // compute_speed_of_sound gives co to every particle (WCSPH.py:110-129)
+    double dc = __ddiv_rn(__dmul_rn(cfl_c, min_h), max_c);
+    double df = max_a2 < 1e-12 ? 1e10 : __dmul_rn(cfl_f, __dsqrt_rn(__ddiv_rn(min_h, max_a2)));
+    double dt = (df < dc) ? df : dc;  // Python min(c, f) keeps c on ties
+    unsigned st = 0;
+    if (cnt == 0) {
+      st |= SPH_STATUS_NO_FLUID;
+      dt = dc = df = nan("");
+    }
+    if (dt < 1e-6) st |= SPH_STATUS_SMALL_DT;
+    if (st) atomicOr(&ctrl->status, st);
+    if (dt_out) {
+      dt_out[0] = dt;
+      dt_out[1] = dc;
+      dt_out[2] = df;
+    }
+    if (dt_hist) {
+      dt_hist[0] = dt;
+      dt_hist[1] = dc;
+      dt_hist[2] = df;
+    }
+  }
+}
+
+// a^2 as TimeStep.computeVars forms it (no contraction)
+__device__ __forceinline__ double accel2(double ax, double ay) {
+  return __dadd_rn(__dmul_rn(ax, ax), __dmul_rn(ay, ay));
+}
+
+}  // namespace sph

@@ -879,6 +879,8 @@ struct WallLoad {
 void launch_pair(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, const sph_wcsph_t &wc,
                  double *dt_out, double *dt_hist, cudaStream_t st,
                  const WallLoad *wall = nullptr);
+void launch_pair64(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, const sph_wcsph_t &wc,
+                   const PairParams &pp, double *dt_out, double *dt_hist, cudaStream_t st);
 void launch_sum_fixed(const double *v, long long n, double *out, cudaStream_t st);
 void launch_adjoint_step(const StepArgs &s, const StepArgs &h, const WsPtrs &w, const sph_config_t &cfg,
                          const sph_wcsph_t &wc, const sph_adjoint_t &adj, cudaStream_t st);
