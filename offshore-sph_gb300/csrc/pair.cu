@@ -23,6 +23,7 @@
 
 #include <type_traits>
 
+#include "fp64_ops.cuh"
 #include "pair_common.cuh"
 
 namespace sph {
@@ -1054,9 +1055,10 @@ __device__ __forceinline__ int probe_cell(const DevGrid &g, double x, double y, 
   const float tx = fminf(fmaxf((d2f_trunc(x) - g.oxf) * g.inv_ctf, 0.f), g.txmaxf);
   const float ty = fminf(fmaxf((d2f_trunc(y) - g.oyf) * g.inv_ctf, 0.f), g.tymaxf);
   const int kx = min(max((int)floorf(tx), 0), g.ntx - 1), ky = min(max((int)floorf(ty), 0), g.nty - 1);
-  const double reach = 1.5 * (h + g.hmax) * (1.0 + 1e-6);
-  const double wd = ceil(reach / g.ct) + 1.0;
-  W = wd < 1.0 ? 1 : (wd > 1024.0 ? 1024 : (int)wd);
+  // in FP32, rounded up (a wider stencil has the same members)
+  const float reach = 1.5f * (d2f_trunc(h) + g.hmaxf) * 1.00001f;
+  const float wd = ceilf(reach * g.inv_ctf * 1.00001f) + 1.0f;
+  W = !(wd >= 1.0f) ? 1 : (wd > 1024.0f ? 1024 : (int)wd);
   return tiled_key(kx, ky, g.ts, g.ntlx);
 }
 
@@ -1102,44 +1104,177 @@ __global__ void __launch_bounds__(kPairBlock)
   sort_ref_order(idx + base, hij_out + base, q_out + base, r_out + base, cnt, refcell, g.ncx, qref);
 }
 
+// Every slot j of the stencil, spread over the lanes of a warp (all call it
+// with the same stencil; pre: 33 words of shared memory of the warp's own).
+// Up to 32 rows at a time: lane r loads row r's bounds, so a probe waits once
+// for all of them, and the lanes then share the rows' candidates as one
+// range: visit(j, valid), called by all lanes together.  Columns over several
+// tiles go by whole rows per lane: lone(j), called by each lane for itself.
+template <class F, class G>
+__device__ __forceinline__ void warp_stencil(const Stencil &sten, const unsigned int *__restrict__ cstart,
+                                             unsigned int *pre, F &&visit, G &&lone) {
+  const int lane = threadIdx.x & 31;
+  if (sten.multi) {
+    const int m = (1 << sten.ts) - 1;
+    for (int yy = sten.y0 + lane; yy <= sten.y1; yy += 32) {
+      const unsigned int *c = cstart + sten.rowpart(yy);
+      for (int xs = sten.x0; xs <= sten.x1; xs = (xs | m) + 1) {
+        const unsigned int e = __ldg(c + Stencil::colpart(min(sten.x1, xs | m), sten.ts) + 1);
+        for (unsigned int j = __ldg(c + Stencil::colpart(xs, sten.ts)); j < e; j++) lone(j);
+      }
+    }
+    return;
+  }
+  for (int y0 = sten.y0; y0 <= sten.y1; y0 += 32) {
+    const int yy = y0 + lane;
+    unsigned int s0 = 0, e0 = 0, jump = 0, len = 0;
+    if (yy <= sten.y1) {
+      const unsigned int *c = cstart + sten.rowpart(yy);
+      s0 = __ldg(c + sten.ca);
+      e0 = __ldg(c + sten.cb);
+      const unsigned int s1 = __ldg(c + sten.cc), e1 = __ldg(c + sten.cd);
+      jump = s1 - e0;
+      len = (e0 - s0) + (e1 - s1);
+    }
+    unsigned int inc = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    __syncwarp();
+    pre[lane + 1] = inc;
+    if (lane == 0) pre[0] = 0;
+    __syncwarp();
+    const unsigned int total = pre[32];
+    for (unsigned int t0 = 0; t0 < total; t0 += 32) {
+      const unsigned int t = t0 + lane;
+      int r = 0;  // the row of candidate t: the last whose prefix is <= t
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        if (pre[r + o] <= t) r += o;
+      const unsigned int rs0 = __shfl_sync(0xffffffffu, s0, r), re0 = __shfl_sync(0xffffffffu, e0, r);
+      const unsigned int rj = __shfl_sync(0xffffffffu, jump, r);
+      const unsigned int j = rs0 + (t - pre[r]);
+      visit(j >= re0 ? j + rj : j, t < total);
+    }
+  }
+}
+
 // rho = sum_fluid m_j W(r_j, hk) / sum_{fluid, rho_j >= 1e-3} W(r_j, hk) m_j / rho_j over
-// the nearPos set of (x, y, h_search); p = B ((rho / rho0)^gamma - 1)
+// the nearPos set of (x, y, h_search); p = B ((rho / rho0)^gamma - 1).
+// One warp per point: a probe has some 140 candidates, and walking them in
+// one thread was a serial chain of loads and FP64 square roots and divisions.
+// The FP64 pipe then bounds it, so the candidates first pass a test of 4 FP64
+// operations (the rest of it in FP32, padded), and the members that are left,
+// compacted into a list, take one round or two of the rest.  The q <= 3
+// decision takes the correctly rounded operations within 1e-9 of the edge.
+// 2000 points in a 200K-particle column: 757 us with a thread per point, 60
+// with a warp each and one pow per point, 38 so (ncu, cold caches).
+constexpr int kProbeBlock = 256;
 template <int KERNEL>
-__global__ void __launch_bounds__(kPairBlock)
+__global__ void __launch_bounds__(kProbeBlock)
     k_probe_density(const double *__restrict__ px, const double *__restrict__ py, const double *__restrict__ ph,
                     const double *__restrict__ hk, long long np, StepArgs a, const int *__restrict__ perm,
                     const int2 *__restrict__ meta, const unsigned int *__restrict__ cstart,
                     const DevGrid *__restrict__ gp, double rho0, double B, double gamma, double *rho_out,
                     double *p_out) {
-  const DevGrid g = *gp;
-  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= np) return;
+  constexpr int kList = 64;
+  __shared__ unsigned int pre_all[kProbeBlock / 32][33];
+  __shared__ int list_all[kProbeBlock / 32][kList];
+  const DevGrid &g = *gp;
+  __shared__ double rho_all[kProbeBlock / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long k0 = (long long)blockIdx.x * (kProbeBlock / 32);
+  const long long k = k0 + warp < np ? k0 + warp : np - 1;  // the last block's spare warps repeat the last point
+  int *list = list_all[warp];
   const double xi = px[k], yi = py[k], hi = ph[k], hw = hk[k];
+  const float hif = d2f_trunc(hi);
+  const double ihw = 1.0 / hw;
+  const double al = (KERNEL == SPH_KERNEL_CUBIC ? kCubicFac : (KERNEL == SPH_KERNEL_WENDLAND ? kWendFac : kInvPi)) /
+                    (hw * hw);
   int2 qref;
   int W;
   const int qkey = probe_cell(g, xi, yi, hi, qref, W);
   const bool filter = g.mode == 1;
   double shep = 0.0, sum = 0.0;
-  int nf = 0;
-  const Stencil sten(g, qref, qkey, W);
-  for_stencil(sten, cstart, [&](unsigned int j) {
-    if (filter && !in_ref_stencil(meta, j, g, qref)) return;
-    const int pj = perm[j];
-    const double dx = xi - a.x[pj], dy = yi - a.y[pj];
-    const double r = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
-    const double hij = __dmul_rn(0.5, __dadd_rn(hi, a.h[pj]));
-    if (!(__ddiv_rn(r, hij) <= 3.0)) return;
-    if (!is_fluid(a.label[pj])) return;  // Shepard and SummationDensity take fluid only
-    const double w = KERNEL == SPH_KERNEL_CUBIC ? cubic_w(r, hw)
-                                                : (KERNEL == SPH_KERNEL_WENDLAND ? wendland_w(r, hw) : gauss_w(r, hw));
-    const double m = a.m[pj], rho = a.rho[pj];
-    if (!(rho < 1e-3)) shep += w * m / rho;
-    sum += m * w;
+  unsigned int nf = 0;
+  // r <= 3 h_ij up to the padding; a negative h_ij (a negative search length)
+  // has every particle inside
+  auto close = [&](unsigned int j, int &pj) {
+    if (filter && !in_ref_stencil(meta, j, g, qref)) return false;
+    pj = perm[j];
+    const double xj = a.x[pj], yj = a.y[pj];
+    const float s = hif + d2f_trunc(a.h[pj]);
+    if (!is_fluid(a.label[pj])) return false;  // Shepard and SummationDensity take fluid only
+    const double dx = xi - xj, dy = yi - yj;
+    const float d2 = d2f_trunc(fma(dx, dx, dy * dy));
+    return hif < 0.f || !(d2 > 2.25f * 1.00001f * (s * s));
+  };
+  auto member = [&](int pj) {
+    const double xj = a.x[pj], yj = a.y[pj], hj = a.h[pj], m = a.m[pj], rho = a.rho[pj];
+    const double dx = xi - xj, dy = yi - yj;
+    const double d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
+    const double hij = __dmul_rn(0.5, __dadd_rn(hi, hj));
+    const double t = 9.0 * hij * hij;
+    if (!(d2 < t * (1.0 - 1e-9)) && !(__ddiv_rn(__dsqrt_rn(d2), hij) <= 3.0)) return;
+    double r = 0.0, ir;
+    if (d2 > 0.0) sqrt_rsqrt64(d2, r, ir);
+    // W(r, hw) (CubicSpline.py:12-36, Wendland.py:10-34, Gaussian.py:16-24)
+    const double q = r * ihw;
+    double w = 0.0;
+    if (KERNEL == SPH_KERNEL_CUBIC) {
+      const double c = 2.0 - q;
+      if (q <= 1.0) w = al * (1.0 - 1.5 * (q * q) * (1.0 - 0.5 * q));
+      else if (!(q > 2.0)) w = al * 0.25 * (c * c * c);
+    } else if (KERNEL == SPH_KERNEL_WENDLAND) {
+      const double c = 1.0 - 0.5 * q, c2 = c * c;
+      if (!(q >= 2.0)) w = al * (c2 * c2 * c2 * ((35.0 / 12.0) * q * q + 3.0 * q + 1.0));
+    } else if (fabs(q) < 3.0 * (1.0 - 1e-9) || r / hw <= 3.0) {
+      w = al * (q < 0.0 ? exp(-q * q) : exp_neg(q * q));
+    }
+    const double mw = m * w;
+    if (!(rho < 1e-3)) shep = rho < 1e300 ? fma(mw, rcp64(rho), shep) : shep + mw / rho;
+    sum += mw;
     nf++;
-  });
-  const double rho = nf ? sum / shep : 0.0;  // an empty sum without fluid neighbours
-  rho_out[k] = rho;
-  p_out[k] = (pow(rho / rho0, gamma) - 1.0) * B;
+  };
+  int nl = 0;
+  auto members = [&]() {
+    __syncwarp();
+    for (int t = lane; t < nl; t += 32) member(list[t]);
+    nl = 0;
+    __syncwarp();
+  };
+  const Stencil sten(g, qref, qkey, W);
+  warp_stencil(
+      sten, cstart, pre_all[warp],
+      [&](unsigned int j, bool valid) {
+        int pj = 0;
+        const bool in = valid && close(j, pj);
+        const unsigned int b = __ballot_sync(0xffffffffu, in);
+        if (in) list[nl + __popc(b & ((1u << lane) - 1u))] = pj;
+        nl += __popc(b);
+        if (nl > kList - 32) members();
+      },
+      [&](unsigned int j) {
+        int pj;
+        if (close(j, pj)) member(pj);
+      });
+  members();
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    shep += __shfl_xor_sync(0xffffffffu, shep, o);
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  }
+  nf = __reduce_add_sync(0xffffffffu, nf);
+  if (lane == 0) rho_all[warp] = nf ? sum / shep : 0.0;  // an empty sum without fluid neighbours
+  __syncthreads();
+  // the EOS of the block's points side by side: one pow for the block
+  if (threadIdx.x < kProbeBlock / 32 && k0 + threadIdx.x < np) {
+    const double rho = rho_all[threadIdx.x];
+    rho_out[k0 + threadIdx.x] = rho;
+    p_out[k0 + threadIdx.x] = (pow(rho / rho0, gamma) - 1.0) * B;
+  }
 }
 
 void launch_nn_probe(const StepArgs &a, const WsPtrs &w, long long np, const double *px, const double *py,
@@ -1153,15 +1288,15 @@ void launch_nn_probe(const StepArgs &a, const WsPtrs &w, long long np, const dou
 void launch_probe_density(const StepArgs &a, const WsPtrs &w, int kernel, long long np, const double *px,
                           const double *py, const double *ph, const double *hk, double rho0, double B, double gamma,
                           double *rho, double *p, cudaStream_t st) {
-  const unsigned nb = nblocks(np, kPairBlock);
+  const unsigned nb = nblocks(np * 32, kProbeBlock);
   if (kernel == SPH_KERNEL_CUBIC)
-    k_probe_density<SPH_KERNEL_CUBIC><<<nb, kPairBlock, 0, st>>>(px, py, ph, hk, np, a, w.perm, w.meta, w.cstart,
+    k_probe_density<SPH_KERNEL_CUBIC><<<nb, kProbeBlock, 0, st>>>(px, py, ph, hk, np, a, w.perm, w.meta, w.cstart,
                                                                   w.grid, rho0, B, gamma, rho, p);
   else if (kernel == SPH_KERNEL_WENDLAND)
-    k_probe_density<SPH_KERNEL_WENDLAND><<<nb, kPairBlock, 0, st>>>(px, py, ph, hk, np, a, w.perm, w.meta, w.cstart,
+    k_probe_density<SPH_KERNEL_WENDLAND><<<nb, kProbeBlock, 0, st>>>(px, py, ph, hk, np, a, w.perm, w.meta, w.cstart,
                                                                      w.grid, rho0, B, gamma, rho, p);
   else
-    k_probe_density<SPH_KERNEL_GAUSSIAN><<<nb, kPairBlock, 0, st>>>(px, py, ph, hk, np, a, w.perm, w.meta, w.cstart,
+    k_probe_density<SPH_KERNEL_GAUSSIAN><<<nb, kProbeBlock, 0, st>>>(px, py, ph, hk, np, a, w.perm, w.meta, w.cstart,
                                                                      w.grid, rho0, B, gamma, rho, p);
 }
 
