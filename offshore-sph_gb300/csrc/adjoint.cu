@@ -28,14 +28,16 @@
 // each thread's own outputs only, so each pair counts once.
 #include <math.h>
 
-#include "sph_internal.cuh"
+#include <type_traits>
+
+#include "fp64_ops.cuh"
+#include "pair_common.cuh"
 
 namespace sph {
 
-// one-warp blocks: the kernel is FP64-bound and a small case has few warps
-// per SM, so small blocks spread them evenly
-constexpr int kAdjBlock = 32;
-constexpr int kAdjSplit = 1;  // lanes per query
+// two-warp blocks: the kernels have few warps per SM, and small blocks spread
+// them evenly
+constexpr int kAdjBlock = 64;
 
 struct AdjParams {
   double alpha, beta, co, r0, D, p1, p2, gamma, B, inv_rho0;
@@ -60,69 +62,6 @@ __device__ __forceinline__ double dothr_drho(double rho, double othr, const AdjP
   return (dp - 2.0 * othr * rho) / (rho * rho);
 }
 
-// The adjoint needs about 1e-12 relative accuracy, not correct rounding, so
-// its reciprocals and square roots start from the FP32 hardware estimate
-// (reached through the integer-pipe truncating conversion) and take two
-// Newton-Raphson steps in FP64, each squaring the relative error:
-//   1/x:        y <- y + y (1 - x y)
-//   1/sqrt(x):  y <- y + y (1 - x y^2) / 2
-// (the FP64 pipe of GB300 issues few instructions per cycle; a correctly
-// rounded FP64 division or square root costs several times more).
-__device__ __forceinline__ double rcp_nr(double x) {
-  double y = f2d(__frcp_rn(d2f_trunc(x)));
-  double e = fma(-x, y, 1.0);
-  y = fma(y, e, y);
-  e = fma(-x, y, 1.0);
-  return fma(y, e, y);
-}
-__device__ __forceinline__ double rsqrt_nr(double x) {
-  double y = f2d(rsqrtf(d2f_trunc(x)));
-  double e = fma(-x * y, y, 1.0);
-  y = fma(0.5 * y, e, y);
-  e = fma(-x * y, y, 1.0);
-  return fma(0.5 * y, e, y);
-}
-
-// kernel gradient factor coef(r) (dW = coef * u) and its r-derivative, with
-// the reference's guards (CubicSpline.py:40-70, Gaussian.py:42-59)
-// (q = r / h, ih = 1 / h, ir = 1 / r; one reciprocal each per pair)
-template <int KERNEL>
-__device__ __forceinline__ void grad_coef(double r, double q, double ih, double ir, double &coef, double &dcoef) {
-  coef = 0.0;
-  dcoef = 0.0;
-  const double ih2 = ih * ih;
-  if (KERNEL == SPH_KERNEL_CUBIC) {
-    if (q > 2.0 || r < 1e-10) return;
-    const double al = kCubicFac * ih2;
-    double g, gp;
-    if (q > 1.0) {
-      const double t = 2.0 - q;
-      g = -0.75 * t * t;
-      gp = 1.5 * t;
-    } else {
-      g = -3.0 * q * (1.0 - 0.75 * q);
-      gp = -3.0 + 4.5 * q;
-    }
-    const double a = al * ih * ir;
-    coef = a * g;
-    dcoef = a * (gp * ih - g * ir);
-  } else if (KERNEL == SPH_KERNEL_WENDLAND) {
-    // g(q) = (1 - q/2)^5 (-14/3) q (1 + 2.5 q) (Wendland.py:58-60)
-    if (q >= 2.0 || r < 1e-10) return;
-    const double al = kWendFac * ih2;
-    const double in = 1.0 - 0.5 * q, in2 = in * in, in4 = in2 * in2;
-    const double g = in4 * in * (-14.0 / 3.0) * q * (1.0 + 2.5 * q);
-    const double gp = (-14.0 / 3.0) * (in4 * in * (1.0 + 5.0 * q) - 2.5 * in4 * q * (1.0 + 2.5 * q));
-    const double a = al * ih * ir;
-    coef = a * g;
-    dcoef = a * (gp * ih - g * ir);
-  } else {
-    if (!(q <= 3.0) || !(r > 1e-12 * ih)) return;
-    coef = -2.0 * kInvPi * ih2 * exp(-q * q) * ih2;
-    dcoef = coef * (-2.0 * r * ih2);
-  }
-}
-
 struct AdjPtrs {
   const float4 *rec0;  // FP32 positions and signed h (prefilter)
   const double4_32a *r64a, *r64b;
@@ -135,155 +74,179 @@ struct AdjPtrs {
   double *xhb, *yhb, *vxhb, *vyhb, *rhohb, *alb;  // outputs (caller order)
 };
 
-// the candidates of fluid query slot k that fall to lane `part`
-template <int KERNEL>
-__device__ __forceinline__ void adjoint_query(const AdjPtrs &P, const AdjParams &ap, long long k, int i,
-                                              unsigned int part, double &gx, double &gy, double &gvx, double &gvy,
-                                              double &grho, double &gal) {
+// The forward's padded FP32 reach test (kernel support for fluid, min(r0,
+// 3 h_ij) for boundary): a candidate outside it contributes nothing.
+struct AdjReach {
+  const AdjPtrs &P;
+  const DevGrid &g;
+  long long k;
+  int2 qref;
+  bool filter;
+  float4 Qi;
+  float rf2, pad, r0f;
+  __device__ __forceinline__ AdjReach(const AdjPtrs &P, const AdjParams &ap, const DevGrid &g, long long k, int2 qref,
+                                      float support)
+      : P(P), g(g), k(k), qref(qref) {
+    filter = g.mode == 1 && (g.need_filter || P.ctrl->alias_count > 0);
+    Qi = P.rec0[k];
+    pad = g.pad_e;
+    r0f = (float)ap.r0;
+    const float rf = support * 1.000002f * Qi.z + pad;
+    rf2 = rf * rf;
+  }
+  __device__ __forceinline__ bool operator()(unsigned int j) const {
+    if (j == (unsigned int)k) return false;
+    if (filter && !in_ref_stencil(P.meta, j, g, qref)) return false;
+    const float4 qj = P.rec0[j];
+    const float fx = Qi.x - qj.x, fy = Qi.y - qj.y;
+    const float d2 = fx * fx + fy * fy;
+    if (!signbit(qj.z)) return d2 <= rf2;  // every fluid h is the same
+    const float rp = fminf(r0f, 1.5f * (Qi.z + fabsf(qj.z))) * 1.000002f + pad;
+    return d2 <= rp * rp;
+  }
+};
+
+// G lanes per query (for_neighbours).  The FP64 pipe bounds it: about 70 FP64
+// operations per fluid pair, with the building blocks and launch constants of
+// the forward (pair64.cu).  Listing the pairs first keeps the lanes of a warp
+// together: evaluating each candidate as the walk met it ran 12.5 of 32 lanes
+// on average.  22K particles, one step: 297 us so, 100 us here (ncu).
+template <int KERNEL, int G>
+__global__ void __launch_bounds__(kAdjBlock, 6) k_pair_adjoint(AdjPtrs P, AdjParams ap, Pair64 c) {
+  constexpr int kCap = (G == 1 ? 1 : 1.5) * ListCap<KERNEL>::value;
+  constexpr bool gauss = KERNEL == SPH_KERNEL_GAUSSIAN;
+  __shared__ unsigned int lists[kCap * kAdjBlock / G];
   const DevGrid &g = *P.grid;
-  const double4_32a Ak = P.r64a[k], Bk = P.r64b[k];
-  const double xk = Ak.x, yk = Ak.y, vxk = Ak.z, vyk = Ak.w;
+  const long long k = ((long long)blockIdx.x * kAdjBlock + threadIdx.x) / G;
+  const long long kq = k < ap.n ? k : 0;
+  const int i = P.perm[kq];
+  const double4_32a Ak = P.r64a[kq], Bk = P.r64b[kq];
+  const bool act = k < ap.n && !signbit(Bk.w);
+  double gx = 0.0, gy = 0.0, gvx = 0.0, gvy = 0.0, glq = 0.0, grh = 0.0, gal = 0.0;
   const double mk = Bk.x, rhok = Bk.y, othrk = Bk.z, hk = Bk.w;
-  const double lAxk = P.lax[i], lAyk = P.lay[i], lDk = P.lad[i];
-  const double dothk = dothr_drho(rhok, othrk, ap);
-  const double ihk = 1.0 / hk;  // 1 / h_ij of pairs with h_j == h_k
-  const double cbar = 0.5 * ap.co;
-  const int2 qref = P.meta[k];
-  const int qkey = P.keys_sorted[k];
-  const bool slow = qref.x >= g.ncx || !(hk > 0.0);
-  const int W = g.mode == 0 ? 1 : (slow ? g.wide : g.wt);
-  const bool filter = g.mode == 1 && (g.need_filter || P.ctrl->alias_count > 0);
-  unsigned int cnt = 0;
-  // the forward's padded FP32 reach test: a candidate outside it contributes
-  // nothing (kernel support for fluid, min(r0, 3 h_ij) for boundary)
-  const float4 Qi = P.rec0[k];
-  const float hif = Qi.z, r0f = (float)ap.r0, pad = g.pad_e;
-  const float SK = (float)Support<KERNEL>::q * 1.000002f;
-  const Stencil sten(g, qref, qkey, W);
-  for_stencil(sten, P.cstart, [&](unsigned int j) {
-    if ((cnt++ % kAdjSplit) != part) return;
-    if (j == (unsigned int)k) return;
-    if (filter && !in_ref_stencil(P.meta, j, g, qref)) return;
-    {
-      const float4 qj = P.rec0[j];
-      const float fx = Qi.x - qj.x, fy = Qi.y - qj.y;
-      const float hijf = 0.5f * (hif + fabsf(qj.z));
-      float reach = SK * hijf;
-      if (signbit(qj.z)) reach = fmaxf(reach, fminf(r0f, 3.0f * hijf) * 1.000002f);
-      const float rp = reach + pad;
-      if (fx * fx + fy * fy > rp * rp) return;
-    }
-    const double4_32a Aj = P.r64a[j], Bj = P.r64b[j];
-    const double dx = xk - Aj.x, dy = yk - Aj.y;
-    const double d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
-    if (!(d2 > 1e-24)) return;  // coincident: no kernel gradient, no boundary force
-    const double ir = rsqrt_nr(d2);
-    double r = d2 * ir;
-    const double hj = fabs(Bj.w);
-    const double hij = __dmul_rn(0.5, __dadd_rn(hk, hj));
-    // h_j == h_k (fluid pairs at a fixed h) and h_j == 0 (boundary) are exact
-    const double ih = hj == hk ? ihk : (hj == 0.0 ? 2.0 * ihk : rcp_nr(hij));
-    double q = r * ih;
-    // the forward's neighbour test q = r / h_ij <= 3 (NNLinkedList.py:74),
-    // redone with its correctly rounded operations where the estimate could
-    // decide differently
-    if (fabs(q - 3.0) < 1e-9) {
-      r = __dsqrt_rn(d2);
-      q = __ddiv_rn(r, hij);
-    }
-    if (!(q <= 3.0)) return;
-    if (!signbit(Bj.w)) {
-      // fluid pair: continuity + momentum with artificial viscosity
-      const double mj = Bj.x, rhoj = Bj.y, othrj = Bj.z;
-      const double vxij = vxk - Aj.z, vyij = vyk - Aj.w;
-      double coef, dcoef;
-      grad_coef<KERNEL>(r, q, ih, ir, coef, dcoef);
-      if (coef == 0.0 && dcoef == 0.0) return;
-      const double dWx = coef * dx, dWy = coef * dy;
-      const double dot = vxij * dx + vyij * dy;
-      const double irbar = 2.0 * rcp_nr(rhok + rhoj);
-      double Pi = 0.0, dPi_dmu = 0.0, mu = 0.0, iden = 0.0, hb = 0.0;
-      if (dot < 0.0) {
-        hb = 0.5 * (hk + hij);
-        iden = rcp_nr(d2 + 0.01 * hb * hb);
-        mu = hb * dot * iden;
-        Pi = mu * (ap.beta * mu - ap.alpha * cbar) * irbar;
-        dPi_dmu = (2.0 * ap.beta * mu - ap.alpha * cbar) * irbar;
+  if (G > 1 ? __any_sync(0xffffffffu, act) : act) {
+    const double lAxk = P.lax[i], lAyk = P.lay[i], lDk = P.lad[i];
+    const double ac = ap.alpha * 0.5 * ap.co;
+    const int2 qref = P.meta[kq];
+    const bool slow = qref.x >= g.ncx;
+    const int W = g.mode == 0 ? 1 : (slow ? g.wide : g.wt);
+    const AdjReach near(P, ap, g, kq, qref, (float)Support<KERNEL>::q);
+    const Stencil sten(g, qref, P.keys_sorted[kq], W);
+    for_neighbours<G, kCap, kAdjBlock>(sten, P.cstart, act, lists, near, [&](unsigned int j) {
+      const double4_32a Aj = P.r64a[j], Bj = P.r64b[j];
+      const double dx = Ak.x - Aj.x, dy = Ak.y - Aj.y;
+      const double d2 = fma(dx, dx, dy * dy);
+      if (le_bits(d2, 1e-24)) return;  // coincident: no kernel gradient, no boundary force
+      if (!signbit(Bj.w)) {
+        // fluid pair: continuity + momentum with artificial viscosity.
+        // dW = coef u; dci = (d coef / d r) / r
+        double coef, dci;
+        if constexpr (gauss) {
+          if (!le_bits(d2, c.lim_lo) && (!le_bits(d2, c.lim_hi) || !near_exact(dx, dy, hk))) return;
+          if (le_bits(d2, c.h2)) return;
+          const double ih2 = c.ih * c.ih;
+          coef = c.i_0 * exp_neg(d2 * ih2);
+          dci = coef * (-2.0 * ih2);
+        } else {
+          if (!le_bits(d2, c.lim) || le_bits(d2, 1e-20)) return;
+          double r, ir;
+          sqrt_rsqrt64(d2, r, ir);
+          if (KERNEL == SPH_KERNEL_CUBIC) {
+            if (le_bits(d2, c.h2)) {
+              coef = fma(c.i_r, r, c.i_0);
+              dci = c.i_r * ir;
+            } else {
+              coef = fma(c.o_ir, ir, fma(c.o_r, r, c.o_0));
+              dci = ir * fma(-c.o_ir * ir, ir, c.o_r);
+            }
+          } else {
+            const double in = fma(c.o_r, r, 1.0), in2 = in * in, in4 = in2 * in2;
+            const double l = fma(c.i_r, r, c.i_0);
+            coef = in4 * (in * l);
+            dci = ir * in4 * fma(5.0 * c.o_r, l, in * c.i_r);
+          }
+        }
+        const double mj = Bj.x;
+        const int pj = P.perm[j];
+        const double lAxj = P.lax[pj], lAyj = P.lay[pj], lDj = P.lad[pj];
+        const double vx = Ak.z - Aj.z, vy = Ak.w - Aj.w;
+        const double dot = fma(vx, dx, vy * dy);
+        const double lQx = fma(mk, lAxj, -mj * lAxk), lQy = fma(mk, lAyj, -mj * lAyk);
+        const double lC = fma(mk, lDj, mj * lDk);
+        const double lQu = fma(lQx, dx, lQy * dy), lQdW = coef * lQu;
+        double S = othrk + Bj.z;
+        glq += lQdW;
+        if (negative_bits(dot)) {
+          const double rs = rhok + Bj.y;  // 2 rho_kj
+          const double den = d2 + c.hb2;
+          const double inv = rcp64(den * rs);
+          const double a = dot * inv, irs = inv * den;
+          double Pi, f;  // Pi, and lQdW times d Pi / d (dot)
+          if (ap.beta == 0.0) {
+            Pi = (-2.0 * ac * c.h) * a;
+            f = lQdW * ((-2.0 * ac * c.h) * inv);
+          } else {
+            const double mu = c.h * (a * rs);
+            Pi = 2.0 * mu * fma(ap.beta, mu, -ac) * irs;
+            f = lQdW * (2.0 * c.h * fma(2.0 * ap.beta, mu, -ac) * inv);
+          }
+          S += Pi;
+          const double c2 = 2.0 * (a * rs);  // 2 dot / (r^2 + 0.01 h^2)
+          gx = fma(f, fma(-c2, dx, vx), gx);
+          gy = fma(f, fma(-c2, dy, vy), gy);
+          gvx = fma(f, dx, gvx);
+          gvy = fma(f, dy, gvy);
+          gal = fma((mj * coef) * fma(lAxk, dx, lAyk * dy), a, gal);
+          grh = fma(-lQdW, Pi * irs, grh);  // d rbar / d rho_k = 1/2
+        }
+        // (d dW / d u)^T z = coef z + (dcoef / r) (u . z) u
+        const double cq = dci * fma(S, lQu, lC * dot);
+        const double lCc = lC * coef, Sc = S * coef;
+        gx = fma(cq, dx, fma(Sc, lQx, fma(lCc, vx, gx)));
+        gy = fma(cq, dy, fma(Sc, lQy, fma(lCc, vy, gy)));
+        gvx = fma(lCc, dx, gvx);
+        gvy = fma(lCc, dy, gvy);
+        return;
       }
-      const double S = othrk + othrj + Pi;
-      const int pj = P.perm[j];
-      const double lAxj = P.lax[pj], lAyj = P.lay[pj], lDj = P.lad[pj];
-      const double lQx = -mj * lAxk + mk * lAxj, lQy = -mj * lAyk + mk * lAyj;
-      const double lC = mj * lDk + mk * lDj;
-      const double lQdW = lQx * dWx + lQy * dWy;
-      // (d dW / d u)^T z = coef z + dcoef (u . z) u / r
-      const double cq = S * dcoef * (dx * lQx + dy * lQy) * ir + lC * dcoef * dot * ir;
-      gx += S * coef * lQx + lC * coef * vxij + cq * dx;
-      gy += S * coef * lQy + lC * coef * vyij + cq * dy;
-      gvx += lC * dWx;
-      gvy += lC * dWy;
-      if (dot < 0.0) {
-        const double f = lQdW * dPi_dmu * hb * iden;
-        const double c2 = 2.0 * dot * iden;
-        gx += f * (vxij - c2 * dx);
-        gy += f * (vyij - c2 * dy);
-        gvx += f * dx;
-        gvy += f * dy;
-        gal += mj * (lAxk * dWx + lAyk * dWy) * (mu * cbar * irbar);
-      }
-      grho += lQdW * (dothk - 0.5 * Pi * irbar);  // d rbar / d rho_k = 1/2
-    } else if (r <= ap.r0 && r > 1e-12) {
       // boundary pair: Lennard-Jones force b = D phi(r) u, phi = ((r0/r)^p1 - (r0/r)^p2) / r^2,
       // and the wall load -m_k b.x when j is on the loaded wall
-      const double s = ap.r0 * ir;
+      if (!le_bits(d2, c.r02)) return;
+      if (!c.lj_free) {  // the neighbour test
+        const double hij = 0.5 * (hk + fabs(Bj.w)), t = 3.0 * hij, t2 = t * t;
+        if (!le_bits(d2, t2 * (1.0 - 1e-9)) && (!le_bits(d2, t2 * (1.0 + 1e-9)) || !near_exact(dx, dy, hij))) return;
+      }
+      const double ir2 = rcp64(d2);
       double sp1, sp2;
       if (ap.lj_42) {
-        sp2 = s * s;
+        sp2 = c.r02 * ir2;
         sp1 = sp2 * sp2;
       } else {
+        const double s = ap.r0 / __dsqrt_rn(d2);
         sp1 = pow(s, ap.p1);
         sp2 = pow(s, ap.p2);
       }
-      const double ir2 = ir * ir;
       const double phi = (sp1 - sp2) * ir2;
-      const double dphi = ((-ap.p1 - 2.0) * sp1 + (ap.p2 + 2.0) * sp2) * ir2 * ir;
+      const double dphi = fma(-ap.p1 - 2.0, sp1, (ap.p2 + 2.0) * sp2) * (ir2 * ir2);  // phi' / r
       const double zx = lAxk - ((ap.omega != 0.0 && Aj.x >= ap.wall_x) ? ap.omega * mk : 0.0), zy = lAyk;
-      const double c = dphi * (dx * zx + dy * zy) * ir;
-      gx += ap.D * (phi * zx + c * dx);
-      gy += ap.D * (phi * zy + c * dy);
-    }
-  });
-}
-
-template <int KERNEL>
-__global__ void __launch_bounds__(kAdjBlock, 12) k_pair_adjoint(AdjPtrs P, AdjParams ap) {
-  // kAdjSplit adjacent lanes share a query and take every kAdjSplit-th
-  // candidate of its stencil; their sums are combined with shuffles
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long k = t / kAdjSplit;
-  const unsigned int part = (unsigned int)(t % kAdjSplit);
-  double gx = 0.0, gy = 0.0, gvx = 0.0, gvy = 0.0, grho = 0.0, gal = 0.0;
-  int i = -1;
-  if (k < ap.n) {
-    i = P.perm[k];
-    if (!signbit(P.r64b[k].w)) adjoint_query<KERNEL>(P, ap, k, i, part, gx, gy, gvx, gvy, grho, gal);
+      const double q = dphi * fma(dx, zx, dy * zy);
+      gx = fma(ap.D, fma(phi, zx, q * dx), gx);
+      gy = fma(ap.D, fma(phi, zy, q * dy), gy);
+    });
   }
-#pragma unroll
-  for (int o = 1; o < kAdjSplit; o <<= 1) {
-    gx += __shfl_xor_sync(0xffffffffu, gx, o);
-    gy += __shfl_xor_sync(0xffffffffu, gy, o);
-    gvx += __shfl_xor_sync(0xffffffffu, gvx, o);
-    gvy += __shfl_xor_sync(0xffffffffu, gvy, o);
-    grho += __shfl_xor_sync(0xffffffffu, grho, o);
-    gal += __shfl_xor_sync(0xffffffffu, gal, o);
-  }
-  if (i >= 0 && part == 0) {  // non-fluid particles get zeros: no outputs, their adjoint is not used
+  group_sum<G>(gx);
+  group_sum<G>(gy);
+  group_sum<G>(gvx);
+  group_sum<G>(gvy);
+  group_sum<G>(glq);
+  group_sum<G>(grh);
+  group_sum<G>(gal);
+  if (k < ap.n && threadIdx.x % G == 0) {  // non-fluid particles get zeros: no outputs, their adjoint is not used
     P.xhb[i] = gx;
     P.yhb[i] = gy;
     P.vxhb[i] = gvx;
     P.vyhb[i] = gvy;
-    P.rhohb[i] = grho;
-    P.alb[i] = gal;
+    P.rhohb[i] = act ? fma(glq, dothr_drho(rhok, othrk, ap), grh) : 0.0;
+    P.alb[i] = gal * (ap.co * c.h);  // mu cbar / rho_kj = 2 cbar h a
   }
 }
 
@@ -332,129 +295,119 @@ __device__ __forceinline__ void grad_coef_f(float r, float q, float ih, float ir
   }
 }
 
-template <int KERNEL>
-__device__ __forceinline__ void adjoint_query_mixed(const AdjPtrs &P, const AdjParams &ap, long long k, int i,
-                                                    float &gx, float &gy, float &gvx, float &gvy, float &grho,
-                                                    float &gal) {
+template <int KERNEL, int G>
+__global__ void __launch_bounds__(kAdjBlock) k_pair_adjoint_mixed(AdjPtrs P, AdjParams ap) {
+  constexpr int kCap = (G == 1 ? 1 : 1.5) * ListCap<KERNEL>::value;
+  __shared__ unsigned int lists[kCap * kAdjBlock / G];
   const DevGrid &g = *P.grid;
-  const double4_32a Ak = P.r64a[k], Bk = P.r64b[k];
-  const double xk = Ak.x, yk = Ak.y, vxk = Ak.z, vyk = Ak.w;
-  const double hk = Bk.w;
-  const float mk = d2f_trunc(Bk.x), rhok = d2f_trunc(Bk.y), othrk = d2f_trunc(Bk.z), hkf = d2f_trunc(hk);
-  const float lAxk = d2f_trunc(P.lax[i]), lAyk = d2f_trunc(P.lay[i]), lDk = d2f_trunc(P.lad[i]);
-  const float dothk = d2f_trunc(dothr_drho(Bk.y, Bk.z, ap));
-  const float ihk = __fdividef(1.0f, hkf);
-  const float cbar = 0.5f * (float)ap.co, alpha = (float)ap.alpha, beta = (float)ap.beta;
-  const float r0 = (float)ap.r0, D = (float)ap.D, p1 = (float)ap.p1, p2 = (float)ap.p2;
-  const float omega_m = (float)ap.omega * mk;
-  const int2 qref = P.meta[k];
-  const int qkey = P.keys_sorted[k];
-  const bool slow = qref.x >= g.ncx || !(hk > 0.0);
-  const int W = g.mode == 0 ? 1 : (slow ? g.wide : g.wt);
-  const bool filter = g.mode == 1 && (g.need_filter || P.ctrl->alias_count > 0);
-  const float4 Qi = P.rec0[k];
-  const float hif = Qi.z, pad = g.pad_e;
-  const float SK = (float)Support<KERNEL>::q * 1.000002f;
-  const Stencil sten(g, qref, qkey, W);
-  for_stencil(sten, P.cstart, [&](unsigned int j) {
-    if (j == (unsigned int)k) return;
-    if (filter && !in_ref_stencil(P.meta, j, g, qref)) return;
-    {
-      const float4 qj = P.rec0[j];
-      const float fx = Qi.x - qj.x, fy = Qi.y - qj.y;
-      const float hijf = 0.5f * (hif + fabsf(qj.z));
-      float reach = SK * hijf;
-      if (signbit(qj.z)) reach = fmaxf(reach, fminf(r0, 3.0f * hijf) * 1.000002f);
-      const float rp = reach + pad;
-      if (fx * fx + fy * fy > rp * rp) return;
-    }
-    const double4_32a Aj = P.r64a[j], Bj = P.r64b[j];
-    const double dxd = xk - Aj.x, dyd = yk - Aj.y;
-    const float dx = d2f_trunc(dxd), dy = d2f_trunc(dyd);
-    const float d2 = dx * dx + dy * dy;
-    if (!(d2 > 1e-24f)) return;  // coincident: no kernel gradient, no boundary force
-    const float ir = rsqrtf(d2);
-    const float r = d2 * ir;
-    const double hj = fabs(Bj.w);
-    const float hjf = d2f_trunc(hj);
-    const float hij = 0.5f * (hkf + hjf);
-    const float ih = hj == hk ? ihk : (hj == 0.0 ? 2.0f * ihk : __fdividef(1.0f, hij));
-    const float q = r * ih;
-    bool in = q <= 3.0f;
-    if (fabsf(q - 3.0f) < 1e-4f) {  // the forward's neighbour test (NNLinkedList.py:74), exactly
-      const double rd = __dsqrt_rn(__dadd_rn(__dmul_rn(dxd, dxd), __dmul_rn(dyd, dyd)));
-      in = __ddiv_rn(rd, __dmul_rn(0.5, __dadd_rn(hk, hj))) <= 3.0;
-    }
-    if (!in) return;
-    if (!signbit(Bj.w)) {
-      // fluid pair: continuity + momentum with artificial viscosity
-      const float mj = d2f_trunc(Bj.x), rhoj = d2f_trunc(Bj.y), othrj = d2f_trunc(Bj.z);
-      const float vxij = d2f_trunc(vxk - Aj.z), vyij = d2f_trunc(vyk - Aj.w);
-      float coef, dcoef;
-      grad_coef_f<KERNEL>(r, q, ih, ir, coef, dcoef);
-      if (coef == 0.f && dcoef == 0.f) return;
-      const float dWx = coef * dx, dWy = coef * dy;
-      const float dot = vxij * dx + vyij * dy;
-      const float irbar = __fdividef(2.0f, rhok + rhoj);
-      float Pi = 0.f, dPi_dmu = 0.f, mu = 0.f, iden = 0.f, hb = 0.f;
-      if (dot < 0.f) {
-        hb = 0.5f * (hkf + hij);
-        iden = __fdividef(1.0f, d2 + 0.01f * hb * hb);
-        mu = hb * dot * iden;
-        Pi = mu * (beta * mu - alpha * cbar) * irbar;
-        dPi_dmu = (2.0f * beta * mu - alpha * cbar) * irbar;
-      }
-      const float S = othrk + othrj + Pi;
-      const int pj = P.perm[j];
-      const float lAxj = d2f_trunc(P.lax[pj]), lAyj = d2f_trunc(P.lay[pj]), lDj = d2f_trunc(P.lad[pj]);
-      const float lQx = -mj * lAxk + mk * lAxj, lQy = -mj * lAyk + mk * lAyj;
-      const float lC = mj * lDk + mk * lDj;
-      const float lQdW = lQx * dWx + lQy * dWy;
-      // (d dW / d u)^T z = coef z + dcoef (u . z) u / r
-      const float cq = S * dcoef * (dx * lQx + dy * lQy) * ir + lC * dcoef * dot * ir;
-      gx += S * coef * lQx + lC * coef * vxij + cq * dx;
-      gy += S * coef * lQy + lC * coef * vyij + cq * dy;
-      gvx += lC * dWx;
-      gvy += lC * dWy;
-      if (dot < 0.f) {
-        const float f = lQdW * dPi_dmu * hb * iden;
-        const float c2 = 2.0f * dot * iden;
-        gx += f * (vxij - c2 * dx);
-        gy += f * (vyij - c2 * dy);
-        gvx += f * dx;
-        gvy += f * dy;
-        gal += mj * (lAxk * dWx + lAyk * dWy) * (mu * cbar * irbar);
-      }
-      grho += lQdW * (dothk - 0.5f * Pi * irbar);
-    } else if (r <= r0 && r > 1e-12f) {
-      // boundary pair: Lennard-Jones force and the wall load
-      const float s = r0 * ir;
-      float sp1, sp2;
-      if (ap.lj_42) {
-        sp2 = s * s;
-        sp1 = sp2 * sp2;
-      } else {
-        sp1 = __powf(s, p1);
-        sp2 = __powf(s, p2);
-      }
-      const float ir2 = ir * ir;
-      const float phi = (sp1 - sp2) * ir2;
-      const float dphi = ((-p1 - 2.0f) * sp1 + (p2 + 2.0f) * sp2) * ir2 * ir;
-      const float zx = lAxk - ((ap.omega != 0.0 && Aj.x >= ap.wall_x) ? omega_m : 0.f), zy = lAyk;
-      const float c = dphi * (dx * zx + dy * zy) * ir;
-      gx += D * (phi * zx + c * dx);
-      gy += D * (phi * zy + c * dy);
-    }
-  });
-}
-
-template <int KERNEL>
-__global__ void __launch_bounds__(kBlock) k_pair_adjoint_mixed(AdjPtrs P, AdjParams ap) {
-  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= ap.n) return;
-  const int i = P.perm[k];
+  const long long k = ((long long)blockIdx.x * kAdjBlock + threadIdx.x) / G;
+  const long long kq = k < ap.n ? k : 0;
+  const int i = P.perm[kq];
+  const double4_32a Ak = P.r64a[kq], Bk = P.r64b[kq];
+  const bool act = k < ap.n && !signbit(Bk.w);
   float gx = 0.f, gy = 0.f, gvx = 0.f, gvy = 0.f, grho = 0.f, gal = 0.f;
-  if (!signbit(P.r64b[k].w)) adjoint_query_mixed<KERNEL>(P, ap, k, i, gx, gy, gvx, gvy, grho, gal);
+  if (G > 1 ? __any_sync(0xffffffffu, act) : act) {
+    const double xk = Ak.x, yk = Ak.y, vxk = Ak.z, vyk = Ak.w;
+    const double hk = Bk.w;
+    const float mk = d2f_trunc(Bk.x), rhok = d2f_trunc(Bk.y), othrk = d2f_trunc(Bk.z), hkf = d2f_trunc(hk);
+    const float lAxk = d2f_trunc(P.lax[i]), lAyk = d2f_trunc(P.lay[i]), lDk = d2f_trunc(P.lad[i]);
+    const float dothk = d2f_trunc(dothr_drho(Bk.y, Bk.z, ap));
+    const float ihk = __fdividef(1.0f, hkf);
+    const float cbar = 0.5f * (float)ap.co, alpha = (float)ap.alpha, beta = (float)ap.beta;
+    const float r0 = (float)ap.r0, D = (float)ap.D, p1 = (float)ap.p1, p2 = (float)ap.p2;
+    const float omega_m = (float)ap.omega * mk;
+    const int2 qref = P.meta[kq];
+    const bool slow = qref.x >= g.ncx || !(hk > 0.0);
+    const int W = g.mode == 0 ? 1 : (slow ? g.wide : g.wt);
+    const AdjReach near(P, ap, g, kq, qref, (float)Support<KERNEL>::q);
+    const Stencil sten(g, qref, P.keys_sorted[kq], W);
+    for_neighbours<G, kCap, kAdjBlock>(sten, P.cstart, act, lists, near, [&](unsigned int j) {
+      const double4_32a Aj = P.r64a[j], Bj = P.r64b[j];
+      const double dxd = xk - Aj.x, dyd = yk - Aj.y;
+      const float dx = d2f_trunc(dxd), dy = d2f_trunc(dyd);
+      const float d2 = dx * dx + dy * dy;
+      if (!(d2 > 1e-24f)) return;  // coincident: no kernel gradient, no boundary force
+      const float ir = rsqrtf(d2);
+      const float r = d2 * ir;
+      const double hj = fabs(Bj.w);
+      const float hjf = d2f_trunc(hj);
+      const float hij = 0.5f * (hkf + hjf);
+      const float ih = hj == hk ? ihk : (hj == 0.0 ? 2.0f * ihk : __fdividef(1.0f, hij));
+      const float q = r * ih;
+      bool in = q <= 3.0f;
+      if (fabsf(q - 3.0f) < 1e-4f) {  // the forward's neighbour test (NNLinkedList.py:74), exactly
+        const double rd = __dsqrt_rn(__dadd_rn(__dmul_rn(dxd, dxd), __dmul_rn(dyd, dyd)));
+        in = __ddiv_rn(rd, __dmul_rn(0.5, __dadd_rn(hk, hj))) <= 3.0;
+      }
+      if (!in) return;
+      if (!signbit(Bj.w)) {
+        // fluid pair: continuity + momentum with artificial viscosity
+        const float mj = d2f_trunc(Bj.x), rhoj = d2f_trunc(Bj.y), othrj = d2f_trunc(Bj.z);
+        const float vxij = d2f_trunc(vxk - Aj.z), vyij = d2f_trunc(vyk - Aj.w);
+        float coef, dcoef;
+        grad_coef_f<KERNEL>(r, q, ih, ir, coef, dcoef);
+        if (coef == 0.f && dcoef == 0.f) return;
+        const float dWx = coef * dx, dWy = coef * dy;
+        const float dot = vxij * dx + vyij * dy;
+        const float irbar = __fdividef(2.0f, rhok + rhoj);
+        float Pi = 0.f, dPi_dmu = 0.f, mu = 0.f, iden = 0.f, hb = 0.f;
+        if (dot < 0.f) {
+          hb = 0.5f * (hkf + hij);
+          iden = __fdividef(1.0f, d2 + 0.01f * hb * hb);
+          mu = hb * dot * iden;
+          Pi = mu * (beta * mu - alpha * cbar) * irbar;
+          dPi_dmu = (2.0f * beta * mu - alpha * cbar) * irbar;
+        }
+        const float S = othrk + othrj + Pi;
+        const int pj = P.perm[j];
+        const float lAxj = d2f_trunc(P.lax[pj]), lAyj = d2f_trunc(P.lay[pj]), lDj = d2f_trunc(P.lad[pj]);
+        const float lQx = -mj * lAxk + mk * lAxj, lQy = -mj * lAyk + mk * lAyj;
+        const float lC = mj * lDk + mk * lDj;
+        const float lQdW = lQx * dWx + lQy * dWy;
+        // (d dW / d u)^T z = coef z + dcoef (u . z) u / r
+        const float cq = S * dcoef * (dx * lQx + dy * lQy) * ir + lC * dcoef * dot * ir;
+        gx += S * coef * lQx + lC * coef * vxij + cq * dx;
+        gy += S * coef * lQy + lC * coef * vyij + cq * dy;
+        gvx += lC * dWx;
+        gvy += lC * dWy;
+        if (dot < 0.f) {
+          const float f = lQdW * dPi_dmu * hb * iden;
+          const float c2 = 2.0f * dot * iden;
+          gx += f * (vxij - c2 * dx);
+          gy += f * (vyij - c2 * dy);
+          gvx += f * dx;
+          gvy += f * dy;
+          gal += mj * (lAxk * dWx + lAyk * dWy) * (mu * cbar * irbar);
+        }
+        grho += lQdW * (dothk - 0.5f * Pi * irbar);
+      } else if (r <= r0 && r > 1e-12f) {
+        // boundary pair: Lennard-Jones force and the wall load
+        const float s = r0 * ir;
+        float sp1, sp2;
+        if (ap.lj_42) {
+          sp2 = s * s;
+          sp1 = sp2 * sp2;
+        } else {
+          sp1 = __powf(s, p1);
+          sp2 = __powf(s, p2);
+        }
+        const float ir2 = ir * ir;
+        const float phi = (sp1 - sp2) * ir2;
+        const float dphi = ((-p1 - 2.0f) * sp1 + (p2 + 2.0f) * sp2) * ir2 * ir;
+        const float zx = lAxk - ((ap.omega != 0.0 && Aj.x >= ap.wall_x) ? omega_m : 0.f), zy = lAyk;
+        const float c = dphi * (dx * zx + dy * zy) * ir;
+        gx += D * (phi * zx + c * dx);
+        gy += D * (phi * zy + c * dy);
+      }
+    });
+  }
+  group_sum<G>(gx);
+  group_sum<G>(gy);
+  group_sum<G>(gvx);
+  group_sum<G>(gvy);
+  group_sum<G>(grho);
+  group_sum<G>(gal);
+  if (k >= ap.n || threadIdx.x % G != 0) return;
   P.xhb[i] = f2d(gx);
   P.yhb[i] = f2d(gy);
   P.vxhb[i] = f2d(gvx);
@@ -595,17 +548,22 @@ void launch_adjoint_step(const StepArgs &s, const StepArgs &h, const WsPtrs &w, 
   ap.wall_x = adj.wall_x;
   ap.dt = dt;
   ap.n = n;
-  if (cfg.precision == SPH_PREC_MIXED) {
-    const unsigned nbm = nblocks(n, kBlock);
-    if (cfg.kernel == SPH_KERNEL_CUBIC) k_pair_adjoint_mixed<SPH_KERNEL_CUBIC><<<nbm, kBlock, 0, st>>>(P, ap);
-    else if (cfg.kernel == SPH_KERNEL_WENDLAND) k_pair_adjoint_mixed<SPH_KERNEL_WENDLAND><<<nbm, kBlock, 0, st>>>(P, ap);
-    else k_pair_adjoint_mixed<SPH_KERNEL_GAUSSIAN><<<nbm, kBlock, 0, st>>>(P, ap);
-  } else {
-    const unsigned nbp = nblocks(n * kAdjSplit, kAdjBlock);
-    if (cfg.kernel == SPH_KERNEL_CUBIC) k_pair_adjoint<SPH_KERNEL_CUBIC><<<nbp, kAdjBlock, 0, st>>>(P, ap);
-    else if (cfg.kernel == SPH_KERNEL_WENDLAND) k_pair_adjoint<SPH_KERNEL_WENDLAND><<<nbp, kAdjBlock, 0, st>>>(P, ap);
-    else k_pair_adjoint<SPH_KERNEL_GAUSSIAN><<<nbp, kAdjBlock, 0, st>>>(P, ap);
-  }
+  const Pair64 c = pair64_consts(cfg, wc);
+  const int lanes = lanes_per_query(n);
+  auto go = [&](auto kern, auto l) {
+    constexpr int K = decltype(kern)::value, G = decltype(l)::value;
+    const unsigned nbp = nblocks(n * G, kAdjBlock);
+    if (cfg.precision == SPH_PREC_MIXED) k_pair_adjoint_mixed<K, G><<<nbp, kAdjBlock, 0, st>>>(P, ap);
+    else k_pair_adjoint<K, G><<<nbp, kAdjBlock, 0, st>>>(P, ap, c);
+  };
+  auto go_lanes = [&](auto kern) {
+    if (lanes == 8) go(kern, std::integral_constant<int, 8>());
+    else if (lanes == 4) go(kern, std::integral_constant<int, 4>());
+    else go(kern, std::integral_constant<int, 1>());
+  };
+  if (cfg.kernel == SPH_KERNEL_CUBIC) go_lanes(std::integral_constant<int, SPH_KERNEL_CUBIC>());
+  else if (cfg.kernel == SPH_KERNEL_WENDLAND) go_lanes(std::integral_constant<int, SPH_KERNEL_WENDLAND>());
+  else go_lanes(std::integral_constant<int, SPH_KERNEL_GAUSSIAN>());
   k_adj_post<<<nb, kBlock, 0, st>>>(s.label, n, dt, adj.xb, adj.yb, adj.vxb, adj.vyb, adj.rhob, adj.axb, adj.ayb,
                                     adj.drhob, adj.xhb, adj.yhb, adj.vxhb, adj.vyhb, adj.rhohb, adj.alb, adj.alphab);
 }

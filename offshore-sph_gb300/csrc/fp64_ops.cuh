@@ -1,5 +1,6 @@
 // fp64_ops.cuh -- reciprocal, square root and exponential in few FP64
-// operations, for the kernels that the FP64 pipe bounds.
+// operations, and the launch constants of the FP64 pair kernels, for the
+// kernels that the FP64 pipe bounds.
 #pragma once
 
 #include "sph_internal.cuh"
@@ -112,6 +113,71 @@ __device__ __forceinline__ double exp_neg(double z) {
   const double T = __ldg(&g_exp_table.v[n & (kExpN - 1)]);
   const double b = __hiloint2double(__double2hiint(T) - ((n >> 11) << 20), __double2loint(T));
   return fma(b, t, b);
+}
+
+// ---------------------------------------------------------------------------
+// Launch constants of the FP64 pair kernels
+// ---------------------------------------------------------------------------
+struct Pair64 {
+  int xsph, sumdens;
+  // uniform fluid h (UH)
+  double h, ih, lim;           // h, 1/h, (support h)^2
+  double lim_lo, lim_hi;       // Gaussian: below / above, q <= 3 is decided
+  double h2;                   // cubic: d2 <= h^2 is the inner piece.  Gaussian: d2 <= h2 has no gradient
+  double o_ir, o_r, o_0;       // cubic, outer piece: o_ir / r + o_r r + o_0
+  double i_r, i_0;             // inner piece: i_r r + i_0.  Wendland: (i_r r + i_0) (1 + o_r r)^5
+  double al;                   // normalisation of W
+  double hb2, pic;             // viscosity: pic dot / ((d2 + hb2) (rho_i + rho_j))
+  double r02;                  // r0^2
+  int lj_free;                 // r0 < 1.5 h: the Lennard-Jones pairs all have q <= 3
+};
+
+inline Pair64 pair64_consts(const sph_config_t &cfg, const sph_wcsph_t &wc) {
+  Pair64 c;
+  c.xsph = wc.use_xsph != 0;
+  c.sumdens = wc.use_summation_density != 0;
+  const double h = cfg.h_fixed > 0.0 ? cfg.h_fixed : 1.0;
+  const double ih = 1.0 / h, ih2 = ih * ih;
+  c.h = h;
+  c.ih = ih;
+  c.h2 = h * h;
+  c.o_ir = c.o_r = c.o_0 = c.i_r = c.i_0 = 0.0;
+  if (cfg.kernel == SPH_KERNEL_CUBIC) {
+    // al / (h r) times -0.75 (2 - q)^2 and -3 q (1 - 0.75 q) (CubicSpline.py:40-70)
+    c.al = kCubicFac * ih2;
+    c.lim = 4.0 * h * h;
+    c.o_ir = -3.0 * c.al * ih;
+    c.o_0 = 3.0 * c.al * ih2;
+    c.o_r = -0.75 * c.al * ih2 * ih;
+    c.i_0 = -3.0 * c.al * ih2;
+    c.i_r = 2.25 * c.al * ih2 * ih;
+  } else if (cfg.kernel == SPH_KERNEL_WENDLAND) {
+    // al / (h r) (1 - q/2)^5 (-14/3) q (1 + 2.5 q) (Wendland.py:36-64)
+    c.al = kWendFac * ih2;
+    c.lim = 4.0 * h * h;
+    c.o_r = -0.5 * ih;
+    c.i_0 = (-14.0 / 3.0) * c.al * ih2;
+    c.i_r = (-35.0 / 3.0) * c.al * ih2 * ih;
+  } else {
+    // -2 al / h^2 exp(-q^2) (Gaussian.py:37-59)
+    c.al = kInvPi * ih2;
+    c.lim = 9.0 * h * h;
+    c.i_0 = -2.0 * c.al * ih2;
+    c.h2 = 1e-24 * ih2;  // r h <= 1e-12: no gradient
+  }
+  c.lim_lo = c.lim * (1.0 - 1e-9);
+  c.lim_hi = c.lim * (1.0 + 1e-9);
+  c.hb2 = 0.01 * (h * h);
+  c.pic = -wc.alpha * wc.co * h;  // -2 alpha c_ij h with c_ij = co / 2
+  c.r02 = wc.r0 * wc.r0;
+  c.lj_free = cfg.h_fixed > 0.0 && wc.r0 < 1.5 * h * (1.0 - 1e-9);
+  return c;
+}
+
+// q = r / h_ij <= 3 as the reference decides it
+static __device__ __noinline__ bool near_exact(double dx, double dy, double hij) {
+  const double r = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
+  return __ddiv_rn(r, hij) <= 3.0;
 }
 
 }  // namespace sph

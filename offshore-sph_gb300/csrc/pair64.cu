@@ -27,71 +27,6 @@
 
 namespace sph {
 
-// ---------------------------------------------------------------------------
-// Launch constants
-// ---------------------------------------------------------------------------
-struct Pair64 {
-  int xsph, sumdens;
-  // uniform fluid h (UH)
-  double h, ih, lim;           // h, 1/h, (support h)^2
-  double lim_lo, lim_hi;       // Gaussian: below / above, q <= 3 is decided
-  double h2;                   // cubic: d2 <= h^2 is the inner piece.  Gaussian: d2 <= h2 has no gradient
-  double o_ir, o_r, o_0;       // cubic, outer piece: o_ir / r + o_r r + o_0
-  double i_r, i_0;             // inner piece: i_r r + i_0.  Wendland: (i_r r + i_0) (1 + o_r r)^5
-  double al;                   // normalisation of W
-  double hb2, pic;             // viscosity: pic dot / ((d2 + hb2) (rho_i + rho_j))
-  double r02;                  // r0^2
-  int lj_free;                 // r0 < 1.5 h: the Lennard-Jones pairs all have q <= 3
-};
-
-static Pair64 pair64_consts(const sph_config_t &cfg, const sph_wcsph_t &wc) {
-  Pair64 c;
-  c.xsph = wc.use_xsph != 0;
-  c.sumdens = wc.use_summation_density != 0;
-  const double h = cfg.h_fixed > 0.0 ? cfg.h_fixed : 1.0;
-  const double ih = 1.0 / h, ih2 = ih * ih;
-  c.h = h;
-  c.ih = ih;
-  c.h2 = h * h;
-  c.o_ir = c.o_r = c.o_0 = c.i_r = c.i_0 = 0.0;
-  if (cfg.kernel == SPH_KERNEL_CUBIC) {
-    // al / (h r) times -0.75 (2 - q)^2 and -3 q (1 - 0.75 q) (CubicSpline.py:40-70)
-    c.al = kCubicFac * ih2;
-    c.lim = 4.0 * h * h;
-    c.o_ir = -3.0 * c.al * ih;
-    c.o_0 = 3.0 * c.al * ih2;
-    c.o_r = -0.75 * c.al * ih2 * ih;
-    c.i_0 = -3.0 * c.al * ih2;
-    c.i_r = 2.25 * c.al * ih2 * ih;
-  } else if (cfg.kernel == SPH_KERNEL_WENDLAND) {
-    // al / (h r) (1 - q/2)^5 (-14/3) q (1 + 2.5 q) (Wendland.py:36-64)
-    c.al = kWendFac * ih2;
-    c.lim = 4.0 * h * h;
-    c.o_r = -0.5 * ih;
-    c.i_0 = (-14.0 / 3.0) * c.al * ih2;
-    c.i_r = (-35.0 / 3.0) * c.al * ih2 * ih;
-  } else {
-    // -2 al / h^2 exp(-q^2) (Gaussian.py:37-59)
-    c.al = kInvPi * ih2;
-    c.lim = 9.0 * h * h;
-    c.i_0 = -2.0 * c.al * ih2;
-    c.h2 = 1e-24 * ih2;  // r h <= 1e-12: no gradient
-  }
-  c.lim_lo = c.lim * (1.0 - 1e-9);
-  c.lim_hi = c.lim * (1.0 + 1e-9);
-  c.hb2 = 0.01 * (h * h);
-  c.pic = -wc.alpha * wc.co * h;  // -2 alpha c_ij h with c_ij = co / 2
-  c.r02 = wc.r0 * wc.r0;
-  c.lj_free = cfg.h_fixed > 0.0 && wc.r0 < 1.5 * h * (1.0 - 1e-9);
-  return c;
-}
-
-// q = r / h_ij <= 3 as the reference decides it
-static __device__ __noinline__ bool near_exact(double dx, double dy, double hij) {
-  const double r = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
-  return __ddiv_rn(r, hij) <= 3.0;
-}
-
 struct Acc64 {
   double dd = 0.0, ax = 0.0, ay = 0.0, sx = 0.0, sy = 0.0, fr = 0.0;
 };
@@ -250,23 +185,17 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
 }
 
 // ---------------------------------------------------------------------------
-// The kernel.  G lanes share a query: they walk each stencil row G candidates
-// at a time, append the survivors of the FP32 test to the group's list in
-// candidate order (ballot), evaluate every G-th entry each and combine their
-// sums with shuffles.  G = 1 is one query per thread with a list of its own.
-// The sums of a query depend on G and its candidate order alone.
+// The kernel: G lanes per query (for_neighbours).
 // ---------------------------------------------------------------------------
 template <int KERNEL, bool UH, int G>
 __global__ void __launch_bounds__(kPairBlock, 4)
     k_pair64(StepArgs a, PairPtrs P, PairParams pp, Pair64 c, double *dt_out, double *dt_hist) {
   step_kernel_entry();
   constexpr int kCap = (G == 1 ? 1 : 1.5) * ListCap<KERNEL>::value;
-  constexpr int kGroups = kPairBlock / G;
-  // G = 1: entry t of thread i at [t][i]; else entry t of group i at [i][t]
-  __shared__ unsigned int lists[kCap * kGroups];
+  __shared__ unsigned int lists[kCap * kPairBlock / G];
   const DevGrid &g = *P.grid;
   const int tid = threadIdx.x;
-  const int gl = tid % G, grp = tid / G;
+  const int gl = tid % G;
   const long long k = ((long long)blockIdx.x * kPairBlock + tid) / G;
   unsigned long long ea = kEncMaxId;
   bool act = k < pp.n;
@@ -306,98 +235,17 @@ __global__ void __launch_bounds__(kPairBlock, 4)
       return d2 <= rp * rp;
     };
     const Stencil sten(g, qref, qkey, W);
-    if constexpr (G == 1) {
-      auto physics = [&](int cnt) {
-        for (int t = 0; t < cnt; t++) {
-          const unsigned int j = lists[t * kGroups + grp];
-          pair64<KERNEL, UH>(s, q, c, pp, P.r64a[j], P.r64b[j]);
-        }
-      };
-      int nl = 0;
-      for_stencil(sten, P.cstart, [&](unsigned int j) {
-        if (near(j)) {
-          lists[nl * kGroups + grp] = j;
-          if (++nl == kCap) {
-            physics(nl);
-            nl = 0;
-          }
-        }
-      });
-      physics(nl);
-    } else {
-      unsigned int *list = lists + grp * kCap;
-      const int lane = tid & 31;
-      const unsigned int gmask = (G == 32 ? 0xffffffffu : ((1u << G) - 1u)) << (lane & ~(G - 1));
-      const unsigned int below = gmask & ((1u << lane) - 1u);
-      int nl = 0;
-      auto physics = [&]() {
-        for (int t = gl; t < nl; t += G) {
-          const unsigned int j = list[t];
-          pair64<KERNEL, UH>(s, q, c, pp, P.r64a[j], P.r64b[j]);
-        }
-      };
-      // one run [j0, j1) of candidates per group and round; jump skips from
-      // e0 on (the second of two tile segments)
-      auto walk = [&](unsigned int j0, unsigned int j1, unsigned int e0, unsigned int jump) {
-        for (unsigned int j = j0 + gl; __any_sync(0xffffffffu, j - gl < j1); j += G) {
-          const unsigned int jj = j >= e0 ? j + jump : j;
-          const bool keep = j < j1 && near(jj);
-          const unsigned int b = __ballot_sync(0xffffffffu, keep) & gmask;
-          if (keep) list[nl + __popc(b & below)] = jj;
-          nl += __popc(b);
-          if (__any_sync(0xffffffffu, nl > kCap - G)) {  // no room for another round
-            __syncwarp();
-            if (nl > kCap - G) {
-              physics();
-              nl = 0;
-            }
-            __syncwarp();
-          }
-        }
-      };
-      const int rows = (int)__reduce_max_sync(0xffffffffu, (unsigned)max(act ? sten.y1 - sten.y0 + 1 : 0, 0));
-      const bool any_multi = __any_sync(0xffffffffu, act && sten.multi);
-      for (int r = 0; r < rows; r++) {
-        const int yy = sten.y0 + r;
-        const bool on = act && yy <= sten.y1;
-        const unsigned int *cs = P.cstart + (on ? sten.rowpart(yy) : 0);
-        if (!any_multi) {
-          unsigned int s0 = 0, e0 = 0, s1 = 0, e1 = 0;
-          if (on) {
-            s0 = __ldg(cs + sten.ca);
-            e0 = __ldg(cs + sten.cb);
-            s1 = __ldg(cs + sten.cc);
-            e1 = __ldg(cs + sten.cd);
-          }
-          walk(s0, e0 + (e1 - s1), e0, s1 - e0);
-        } else {
-          // columns over several tiles: the tiles one by one
-          const int m = (1 << sten.ts) - 1;
-          for (int xs = sten.x0; __any_sync(0xffffffffu, on && xs <= sten.x1); xs = (xs | m) + 1) {
-            unsigned int s0 = 0, e0 = 0;
-            if (on && xs <= sten.x1) {
-              s0 = __ldg(cs + Stencil::colpart(xs, sten.ts));
-              e0 = __ldg(cs + Stencil::colpart(min(sten.x1, xs | m), sten.ts) + 1);
-            }
-            walk(s0, e0, e0, 0u);
-          }
-        }
-      }
-      __syncwarp();
-      physics();
-      auto sum = [&](double &v) {
-#pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      };
-      sum(s.dd);
-      sum(s.ax);
-      sum(s.ay);
-      if (c.xsph) {
-        sum(s.sx);
-        sum(s.sy);
-      }
-      if (pp.fr) sum(s.fr);
+    for_neighbours<G, kCap, kPairBlock>(sten, P.cstart, act, lists, near, [&](unsigned int j) {
+      pair64<KERNEL, UH>(s, q, c, pp, P.r64a[j], P.r64b[j]);
+    });
+    group_sum<G>(s.dd);
+    group_sum<G>(s.ax);
+    group_sum<G>(s.ay);
+    if (c.xsph) {
+      group_sum<G>(s.sx);
+      group_sum<G>(s.sy);
     }
+    if (pp.fr) group_sum<G>(s.fr);
     if (act && gl == 0) {
       // the reference's set always holds the particle itself, except for the
       // slow queries, whose set size is counted exactly
@@ -422,23 +270,14 @@ __global__ void __launch_bounds__(kPairBlock, 4)
 template <int KERNEL, bool UH>
 static void pair64_launch(const StepArgs &a, const WsPtrs &w, const PairParams &pp, const Pair64 &c, double *dt_out,
                           double *dt_hist, cudaStream_t st) {
-  // Lanes per query.  Sharing a query costs about a quarter more issue time
-  // (short groups, the final sums; dam break of 1M fluid particles: 1.27 ms
-  // with G = 1, 1.57 ms with G = 4) and divides the length of a thread's
-  // chain of dependent FP64 operations.  So G = 1 where the threads fill most
-  // of one wave of blocks (54K particles, Wendland: 786 us for 4 steps
-  // against 809 with G = 4) or several; G = 4 where the last wave would be
-  // nearly empty (99K, Gaussian: 361 us with G = 1, 325 with 4); G = 8 where
-  // the GPU is idle and the chain is the time (5K particles: 1415 us for 20
-  // steps with G = 1, 990 with 4, 820 with 8, 824 with 16).
-  const long long n = a.n, wave = (long long)sm_count() * kPairBlock * 4;
   auto go = [&](auto lanes) {
     constexpr int G = decltype(lanes)::value;
-    launch_pdl(k_pair64<KERNEL, UH, G>, dim3(nblocks(n * G, kPairBlock)), dim3(kPairBlock), 0, st, a, pair_ptrs(w), pp,
+    launch_pdl(k_pair64<KERNEL, UH, G>, dim3(nblocks(a.n * G, kPairBlock)), dim3(kPairBlock), 0, st, a, pair_ptrs(w), pp,
                c, dt_out, dt_hist);
   };
-  if (n < wave / 8) go(std::integral_constant<int, 8>());
-  else if (n < wave / 2 || (n > wave && n < 4 * wave)) go(std::integral_constant<int, 4>());
+  const int lanes = lanes_per_query(a.n);
+  if (lanes == 8) go(std::integral_constant<int, 8>());
+  else if (lanes == 4) go(std::integral_constant<int, 4>());
   else go(std::integral_constant<int, 1>());
 }
 

@@ -48,6 +48,117 @@ inline PairParams pair_params(const StepArgs &a, const sph_config_t &cfg, const 
   return pp;
 }
 
+// The neighbours of a query, for the kernels whose work per pair is long: the
+// candidates of its stencil that pass near(j) are listed first, in candidate
+// order, and pair(j) then runs over the list, so that the lanes of a warp run
+// the long part together.  G lanes share a query (all lanes of the warp call
+// this; act: the query exists): they walk each stencil row G candidates at a
+// time, append by ballot, and take every G-th entry each, so a query's sums
+// depend on G and its candidate order alone.  G = 1 is one query per thread.
+// lists: CAP * BLOCK / G words of shared memory of the block.
+template <int G, int CAP, int BLOCK, class Near, class Pair>
+__device__ __forceinline__ void for_neighbours(const Stencil &sten, const unsigned int *__restrict__ cstart, bool act,
+                                               unsigned int *lists, Near &&near, Pair &&pair) {
+  const int tid = threadIdx.x;
+  if constexpr (G == 1) {
+    if (!act) return;
+    auto physics = [&](int cnt) {
+      for (int t = 0; t < cnt; t++) pair(lists[t * BLOCK + tid]);
+    };
+    int nl = 0;
+    for_stencil(sten, cstart, [&](unsigned int j) {
+      if (near(j)) {
+        lists[nl * BLOCK + tid] = j;
+        if (++nl == CAP) {
+          physics(nl);
+          nl = 0;
+        }
+      }
+    });
+    physics(nl);
+  } else {
+    const int gl = tid % G, lane = tid & 31;
+    unsigned int *list = lists + tid / G * CAP;
+    const unsigned int gmask = (G == 32 ? 0xffffffffu : ((1u << (G % 32)) - 1u)) << (lane & ~(G - 1));
+    const unsigned int below = gmask & ((1u << lane) - 1u);
+    int nl = 0;
+    auto physics = [&]() {
+      for (int t = gl; t < nl; t += G) pair(list[t]);
+    };
+    // candidates [j0, j1), those from e0 on moved by jump (the second of two
+    // tile segments)
+    auto walk = [&](unsigned int j0, unsigned int j1, unsigned int e0, unsigned int jump) {
+      for (unsigned int j = j0 + gl; __any_sync(0xffffffffu, j - gl < j1); j += G) {
+        const unsigned int jj = j >= e0 ? j + jump : j;
+        const bool keep = j < j1 && near(jj);
+        const unsigned int b = __ballot_sync(0xffffffffu, keep) & gmask;
+        if (keep) list[nl + __popc(b & below)] = jj;
+        nl += __popc(b);
+        if (__any_sync(0xffffffffu, nl > CAP - G)) {  // no room for another round
+          __syncwarp();
+          if (nl > CAP - G) {
+            physics();
+            nl = 0;
+          }
+          __syncwarp();
+        }
+      }
+    };
+    const int rows = (int)__reduce_max_sync(0xffffffffu, (unsigned)max(act ? sten.y1 - sten.y0 + 1 : 0, 0));
+    const bool any_multi = __any_sync(0xffffffffu, act && sten.multi);
+    for (int r = 0; r < rows; r++) {
+      const int yy = sten.y0 + r;
+      const bool on = act && yy <= sten.y1;
+      const unsigned int *cs = cstart + (on ? sten.rowpart(yy) : 0);
+      if (!any_multi) {
+        unsigned int s0 = 0, e0 = 0, s1 = 0, e1 = 0;
+        if (on) {
+          s0 = __ldg(cs + sten.ca);
+          e0 = __ldg(cs + sten.cb);
+          s1 = __ldg(cs + sten.cc);
+          e1 = __ldg(cs + sten.cd);
+        }
+        walk(s0, e0 + (e1 - s1), e0, s1 - e0);
+      } else {
+        // columns over several tiles: the tiles one by one
+        const int m = (1 << sten.ts) - 1;
+        for (int xs = sten.x0; __any_sync(0xffffffffu, on && xs <= sten.x1); xs = (xs | m) + 1) {
+          unsigned int s0 = 0, e0 = 0;
+          if (on && xs <= sten.x1) {
+            s0 = __ldg(cs + Stencil::colpart(xs, sten.ts));
+            e0 = __ldg(cs + Stencil::colpart(min(sten.x1, xs | m), sten.ts) + 1);
+          }
+          walk(s0, e0, e0, 0u);
+        }
+      }
+    }
+    __syncwarp();
+    physics();
+  }
+}
+
+// sum over the G lanes of a query
+template <int G, class T>
+__device__ __forceinline__ void group_sum(T &v) {
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+}
+
+// Lanes per query of the FP64 kernels for n particles.  Sharing a query costs
+// about a quarter more issue time (short groups, the final sums; dam break of
+// 1M fluid particles: 1.27 ms with G = 1, 1.57 ms with G = 4) and divides the
+// length of a thread's chain of dependent FP64 operations.  So G = 1 where the
+// threads fill most of one wave of blocks (54K particles, Wendland: 786 us for
+// 4 steps against 809 with G = 4) or several; G = 4 where the last wave would
+// be nearly empty (99K, Gaussian: 361 us with G = 1, 325 with 4); G = 8 where
+// the GPU is idle and the chain is the time (5K particles: 1415 us for 20
+// steps with G = 1, 990 with 4, 820 with 8, 824 with 16).
+inline int lanes_per_query(long long n) {
+  const long long wave = (long long)sm_count() * kPairBlock * 4;
+  if (n < wave / 8) return 8;
+  return n < wave / 2 || (n > wave && n < 4 * wave) ? 4 : 1;
+}
+
 // Exact size of the reference's neighbour set of a query whose own cell is
 // not in its stencil (x-overflow alias) or whose h is not positive; those are
 // the only queries that can have an empty set (src/Tools/SolverTools.py:150-153).
