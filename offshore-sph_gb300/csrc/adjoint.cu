@@ -94,10 +94,10 @@ struct AdjReach {
     const float rf = support * 1.000002f * Qi.z + pad;
     rf2 = rf * rf;
   }
-  __device__ __forceinline__ bool operator()(unsigned int j) const {
+  __device__ __forceinline__ float4 load(unsigned int j) const { return __ldg(P.rec0 + j); }
+  __device__ __forceinline__ bool test(unsigned int j, float4 qj) const {
     if (j == (unsigned int)k) return false;
     if (filter && !in_ref_stencil(P.meta, j, g, qref)) return false;
-    const float4 qj = P.rec0[j];
     const float fx = Qi.x - qj.x, fy = Qi.y - qj.y;
     const float d2 = fx * fx + fy * fy;
     if (!signbit(qj.z)) return d2 <= rf2;  // every fluid h is the same
@@ -113,7 +113,7 @@ struct AdjReach {
 // on average.  22K particles, one step: 297 us so, 100 us here (ncu).
 template <int KERNEL, int G>
 __global__ void __launch_bounds__(kAdjBlock, 6) k_pair_adjoint(AdjPtrs P, AdjParams ap, Pair64 c) {
-  constexpr int kCap = (G == 1 ? 1 : 1.5) * ListCap<KERNEL>::value;
+  constexpr int kCap = list_words<G>(ListCap<KERNEL>::value);
   constexpr bool gauss = KERNEL == SPH_KERNEL_GAUSSIAN;
   __shared__ unsigned int lists[kCap * kAdjBlock / G];
   const DevGrid &g = *P.grid;
@@ -297,7 +297,7 @@ __device__ __forceinline__ void grad_coef_f(float r, float q, float ih, float ir
 
 template <int KERNEL, int G>
 __global__ void __launch_bounds__(kAdjBlock) k_pair_adjoint_mixed(AdjPtrs P, AdjParams ap) {
-  constexpr int kCap = (G == 1 ? 1 : 1.5) * ListCap<KERNEL>::value;
+  constexpr int kCap = list_words<G>(ListCap<KERNEL>::value);
   __shared__ unsigned int lists[kCap * kAdjBlock / G];
   const DevGrid &g = *P.grid;
   const long long k = ((long long)blockIdx.x * kAdjBlock + threadIdx.x) / G;

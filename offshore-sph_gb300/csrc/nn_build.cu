@@ -18,6 +18,7 @@
 
 #include <string.h>
 
+#include "fp64_ops.cuh"
 #include "sph_internal.cuh"
 
 namespace sph {
@@ -819,7 +820,9 @@ __device__ __forceinline__ void record_fp64(const StepArgs &a, long long k, int 
   double h = a.h[i];
   if (fl && !rp.from_state) h = rp.h_fixed_on ? rp.h_fixed : compute_h_call(m, rho);
   const double p = rp.from_state ? a.p[i] : tait_p(rho, lab, rp.gamma, rp.B, rp.inv_rho0, rp.Pb);
-  const double othr = p / (rho * rho);
+  // p / rho^2 of a fluid particle; no kernel reads a boundary particle's,
+  // whose 0 / 0 took the division's slow path
+  const double othr = !fl ? 0.0 : (rho > 0.0 ? p * rcp64(rho * rho) : p / (rho * rho));
   const double hs = fl ? h : -h;
   r64a[k] = make_double4_32a(x, y, a.vx[i], a.vy[i]);
   r64b[k] = make_double4_32a(m, rho, othr, (!fl && h == 0.0) ? -0.0 : hs);

@@ -187,11 +187,39 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
 // ---------------------------------------------------------------------------
 // The kernel: G lanes per query (for_neighbours).
 // ---------------------------------------------------------------------------
+template <int KERNEL, bool UH>
+struct Near64 {
+  const float4 *rec0;
+  const int2 *meta;
+  const DevGrid &g;
+  float4 Qi;
+  int2 qref;
+  unsigned int k;
+  float rf2, r0f, pad;
+  bool filter, xsph;
+  __device__ __forceinline__ float4 load(unsigned int j) const { return __ldg(rec0 + j); }
+  __device__ __forceinline__ bool test(unsigned int j, float4 qj) const {
+    if (j == k) return false;  // the particle itself contributes zero
+    if (filter && !in_ref_stencil(meta, j, g, qref)) return false;
+    const float dx = Qi.x - qj.x, dy = Qi.y - qj.y;
+    const float d2 = dx * dx + dy * dy;
+    if (UH && !signbit(qj.z)) return d2 <= rf2;
+    const float hij = 0.5f * (Qi.z + fabsf(qj.z));
+    float reach = (float)Support<KERNEL>::q * 1.000002f * hij;
+    if (signbit(qj.z)) {
+      const float lj = fminf(r0f, 3.0f * hij) * 1.000002f;
+      reach = xsph ? fmaxf(reach, lj) : lj;
+    }
+    const float rp = reach + pad;
+    return d2 <= rp * rp;
+  }
+};
+
 template <int KERNEL, bool UH, int G>
 __global__ void __launch_bounds__(kPairBlock, 4)
     k_pair64(StepArgs a, PairPtrs P, PairParams pp, Pair64 c, double *dt_out, double *dt_hist) {
   step_kernel_entry();
-  constexpr int kCap = (G == 1 ? 1 : 1.5) * ListCap<KERNEL>::value;
+  constexpr int kCap = list_words<G>(ListCap<KERNEL>::value);
   __shared__ unsigned int lists[kCap * kPairBlock / G];
   const DevGrid &g = *P.grid;
   const int tid = threadIdx.x;
@@ -218,22 +246,7 @@ __global__ void __launch_bounds__(kPairBlock, 4)
     const float SK = (float)Support<KERNEL>::q * 1.000002f;
     const float r0f = (float)pp.r0, pad = g.pad_e;
     const float rf = SK * hif + pad, rf2 = rf * rf;
-    auto near = [&](unsigned int j) {
-      if (j == (unsigned int)k) return false;  // the particle itself contributes zero
-      if (filter && !in_ref_stencil(P.meta, j, g, qref)) return false;
-      const float4 qj = P.rec0[j];
-      const float dx = Qi.x - qj.x, dy = Qi.y - qj.y;
-      const float d2 = dx * dx + dy * dy;
-      if (UH && !signbit(qj.z)) return d2 <= rf2;
-      const float hij = 0.5f * (hif + fabsf(qj.z));
-      float reach = SK * hij;
-      if (signbit(qj.z)) {
-        const float lj = fminf(r0f, 3.0f * hij) * 1.000002f;
-        reach = c.xsph ? fmaxf(reach, lj) : lj;
-      }
-      const float rp = reach + pad;
-      return d2 <= rp * rp;
-    };
+    const Near64<KERNEL, UH> near{P.rec0, P.meta, g, Qi, qref, (unsigned int)kq, rf2, r0f, pad, filter, c.xsph != 0};
     const Stencil sten(g, qref, qkey, W);
     for_neighbours<G, kCap, kPairBlock>(sten, P.cstart, act, lists, near, [&](unsigned int j) {
       pair64<KERNEL, UH>(s, q, c, pp, P.r64a[j], P.r64b[j]);

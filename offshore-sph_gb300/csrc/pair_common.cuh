@@ -48,17 +48,30 @@ inline PairParams pair_params(const StepArgs &a, const sph_config_t &cfg, const 
   return pp;
 }
 
+// Entries of a query's list for G lanes per query, cap being one thread's: a
+// round adds up to G entries, and the list is evaluated early when another
+// round might not fit.
+template <int G>
+constexpr int list_words(int cap) {
+  return G == 1 ? cap : (G == 32 ? 3 * cap : cap + cap / 2);
+}
+
 // The neighbours of a query, for the kernels whose work per pair is long: the
-// candidates of its stencil that pass near(j) are listed first, in candidate
+// candidates of its stencil that near accepts are listed first, in candidate
 // order, and pair(j) then runs over the list, so that the lanes of a warp run
-// the long part together.  G lanes share a query (all lanes of the warp call
-// this; act: the query exists): they walk each stencil row G candidates at a
-// time, append by ballot, and take every G-th entry each, so a query's sums
-// depend on G and its candidate order alone.  G = 1 is one query per thread.
+// the long part together.  near.load(j) reads what near.test(j, record)
+// decides on.  G lanes share a query (all lanes of the warp call this; act: the
+// query exists): they test G candidates at a time, append by ballot, and take
+// every G-th entry each, so a query's sums depend on G and its candidate order
+// alone.  G = 1 is one query per thread.
+// With G lanes the scene is small and latency is the time: the lanes load the
+// stencil rows' bounds together and walk the rows as one range, two rounds of
+// candidate loads in flight.  Row by row, the walk took 11.4K of the 27K cycles
+// of a block of the FP64 kernel (3200-particle tank, G = 8).
 // lists: CAP * BLOCK / G words of shared memory of the block.
 template <int G, int CAP, int BLOCK, class Near, class Pair>
 __device__ __forceinline__ void for_neighbours(const Stencil &sten, const unsigned int *__restrict__ cstart, bool act,
-                                               unsigned int *lists, Near &&near, Pair &&pair) {
+                                               unsigned int *lists, const Near &near, Pair &&pair) {
   const int tid = threadIdx.x;
   if constexpr (G == 1) {
     if (!act) return;
@@ -67,7 +80,7 @@ __device__ __forceinline__ void for_neighbours(const Stencil &sten, const unsign
     };
     int nl = 0;
     for_stencil(sten, cstart, [&](unsigned int j) {
-      if (near(j)) {
+      if (near.test(j, near.load(j))) {
         lists[nl * BLOCK + tid] = j;
         if (++nl == CAP) {
           physics(nl);
@@ -77,58 +90,81 @@ __device__ __forceinline__ void for_neighbours(const Stencil &sten, const unsign
     });
     physics(nl);
   } else {
+    constexpr unsigned int full = 0xffffffffu;
     const int gl = tid % G, lane = tid & 31;
     unsigned int *list = lists + tid / G * CAP;
-    const unsigned int gmask = (G == 32 ? 0xffffffffu : ((1u << (G % 32)) - 1u)) << (lane & ~(G - 1));
+    const unsigned int gmask = (G == 32 ? full : ((1u << (G % 32)) - 1u)) << (lane & ~(G - 1));
     const unsigned int below = gmask & ((1u << lane) - 1u);
     int nl = 0;
     auto physics = [&]() {
       for (int t = gl; t < nl; t += G) pair(list[t]);
     };
-    // candidates [j0, j1), those from e0 on moved by jump (the second of two
-    // tile segments)
-    auto walk = [&](unsigned int j0, unsigned int j1, unsigned int e0, unsigned int jump) {
-      for (unsigned int j = j0 + gl; __any_sync(0xffffffffu, j - gl < j1); j += G) {
-        const unsigned int jj = j >= e0 ? j + jump : j;
-        const bool keep = j < j1 && near(jj);
-        const unsigned int b = __ballot_sync(0xffffffffu, keep) & gmask;
-        if (keep) list[nl + __popc(b & below)] = jj;
-        nl += __popc(b);
-        if (__any_sync(0xffffffffu, nl > CAP - G)) {  // no room for another round
-          __syncwarp();
-          if (nl > CAP - G) {
-            physics();
-            nl = 0;
-          }
-          __syncwarp();
+    auto append = [&](unsigned int j, bool keep) {
+      const unsigned int b = __ballot_sync(full, keep) & gmask;
+      if (keep) list[nl + __popc(b & below)] = j;
+      nl += __popc(b);
+      if (__any_sync(full, nl > CAP - G)) {  // no room for another round
+        __syncwarp();
+        if (nl > CAP - G) {
+          physics();
+          nl = 0;
         }
+        __syncwarp();
       }
     };
-    const int rows = (int)__reduce_max_sync(0xffffffffu, (unsigned)max(act ? sten.y1 - sten.y0 + 1 : 0, 0));
-    const bool any_multi = __any_sync(0xffffffffu, act && sten.multi);
-    for (int r = 0; r < rows; r++) {
-      const int yy = sten.y0 + r;
-      const bool on = act && yy <= sten.y1;
-      const unsigned int *cs = cstart + (on ? sten.rowpart(yy) : 0);
-      if (!any_multi) {
-        unsigned int s0 = 0, e0 = 0, s1 = 0, e1 = 0;
-        if (on) {
-          s0 = __ldg(cs + sten.ca);
-          e0 = __ldg(cs + sten.cb);
-          s1 = __ldg(cs + sten.cc);
-          e1 = __ldg(cs + sten.cd);
-        }
-        walk(s0, e0 + (e1 - s1), e0, s1 - e0);
-      } else {
-        // columns over several tiles: the tiles one by one
-        const int m = (1 << sten.ts) - 1;
-        for (int xs = sten.x0; __any_sync(0xffffffffu, on && xs <= sten.x1); xs = (xs | m) + 1) {
-          unsigned int s0 = 0, e0 = 0;
+    const int nr = act ? max(sten.y1 - sten.y0 + 1, 0) : 0;
+    if (!__any_sync(full, nr > G || (act && sten.multi))) {
+      // lane r holds row r: candidates [first, last) of the flat range are
+      // slots base + t, from e0 on moved by jump (the second tile segment)
+      unsigned int s0 = 0, e0 = 0, jump = 0, len = 0;
+      if (gl < nr) {
+        const unsigned int *c = cstart + sten.rowpart(sten.y0 + gl);
+        s0 = __ldg(c + sten.ca);
+        e0 = __ldg(c + sten.cb);
+        const unsigned int s1 = __ldg(c + sten.cc), e1 = __ldg(c + sten.cd);
+        jump = s1 - e0;
+        len = (e0 - s0) + (e1 - s1);
+      }
+      unsigned int last = len;
+#pragma unroll
+      for (int o = 1; o < G; o <<= 1) {
+        const unsigned int v = __shfl_up_sync(full, last, o, G);
+        if (gl >= o) last += v;
+      }
+      const unsigned int base = s0 - (last - len), total = __shfl_sync(full, last, G - 1, G);
+      const int rows = (int)__reduce_max_sync(full, (unsigned)nr);
+      auto slot = [&](unsigned int t) {
+        int r = 0;
+        for (int q = 0; q < rows - 1; q++) r += t >= __shfl_sync(full, last, q, G) ? 1 : 0;
+        const unsigned int j = __shfl_sync(full, base, r, G) + t;
+        const unsigned int e = __shfl_sync(full, e0, r, G), s = __shfl_sync(full, jump, r, G);
+        return j >= e ? j + s : j;
+      };
+      for (unsigned int t0 = 0; __any_sync(full, t0 < total); t0 += 2 * G) {
+        const unsigned int ta = t0 + gl, tb = ta + G;
+        const unsigned int ja = slot(ta), jb = slot(tb);
+        float4 qa = make_float4(0.f, 0.f, 0.f, 0.f), qb = qa;
+        if (ta < total) qa = near.load(ja);
+        if (tb < total) qb = near.load(jb);
+        append(ja, ta < total && near.test(ja, qa));
+        append(jb, tb < total && near.test(jb, qb));
+      }
+    } else {
+      // wide stencils (queries whose own cell is not in theirs) or columns
+      // over several tiles: row by row, tile by tile
+      const int rows = (int)__reduce_max_sync(full, (unsigned)nr);
+      const int m = (1 << sten.ts) - 1;
+      for (int r = 0; r < rows; r++) {
+        const bool on = r < nr;
+        const unsigned int *c = cstart + (on ? sten.rowpart(sten.y0 + r) : 0);
+        for (int xs = sten.x0; __any_sync(full, on && xs <= sten.x1); xs = (xs | m) + 1) {
+          unsigned int j = 0, e = 0;
           if (on && xs <= sten.x1) {
-            s0 = __ldg(cs + Stencil::colpart(xs, sten.ts));
-            e0 = __ldg(cs + Stencil::colpart(min(sten.x1, xs | m), sten.ts) + 1);
+            j = __ldg(c + Stencil::colpart(xs, sten.ts));
+            e = __ldg(c + Stencil::colpart(min(sten.x1, xs | m), sten.ts) + 1);
           }
-          walk(s0, e0, e0, 0u);
+          for (j += gl; __any_sync(full, j - gl < e); j += G)
+            append(j, j < e && near.test(j, near.load(j)));
         }
       }
     }
@@ -148,11 +184,11 @@ __device__ __forceinline__ void group_sum(T &v) {
 // about a quarter more issue time (short groups, the final sums; dam break of
 // 1M fluid particles: 1.27 ms with G = 1, 1.57 ms with G = 4) and divides the
 // length of a thread's chain of dependent FP64 operations.  So G = 1 where the
-// threads fill most of one wave of blocks (54K particles, Wendland: 786 us for
-// 4 steps against 809 with G = 4) or several; G = 4 where the last wave would
-// be nearly empty (99K, Gaussian: 361 us with G = 1, 325 with 4); G = 8 where
-// the GPU is idle and the chain is the time (5K particles: 1415 us for 20
-// steps with G = 1, 990 with 4, 820 with 8, 824 with 16).
+// threads fill most of one wave of blocks (54K particles, Wendland: 784 us for
+// 4 steps against 817 with G = 4) or several; G = 4 where the last wave would
+// be nearly empty (99K, Gaussian: 356 us with G = 1, 327 with 4, 355 with 8);
+// G = 8 where the GPU is idle and the chain is the time (5K particles: 1393 us
+// for 20 steps with G = 1, 858 with 4, 732 with 8, 793 with 16, 914 with 32).
 inline int lanes_per_query(long long n) {
   const long long wave = (long long)sm_count() * kPairBlock * 4;
   if (n < wave / 8) return 8;
@@ -214,16 +250,17 @@ __device__ __forceinline__ void timestep_epilogue(DevCtrl *ctrl, unsigned long l
       ea2 = __ldcg(&ctrl->pd_a2max);
       cnt = __ldcg(&ctrl->pd_nfluid);
       ea2 = ba > ea2 ? ba : ea2;
-      ctrl->pd_hmin = kEncMinId;
-      ctrl->pd_a2max = kEncMaxId;
-      ctrl->pd_nfluid = 0u;
     } else {
+      // every other block has added its share (and fenced): L2 loads see it
       __threadfence();
-      eh = atomicExch(&ctrl->pd_hmin, kEncMinId);
-      ea2 = atomicExch(&ctrl->pd_a2max, kEncMaxId);
-      cnt = atomicExch(&ctrl->pd_nfluid, 0u);
-      atomicExch(&ctrl->done_pair, 0u);
+      eh = __ldcg(&ctrl->pd_hmin);
+      ea2 = __ldcg(&ctrl->pd_a2max);
+      cnt = __ldcg(&ctrl->pd_nfluid);
+      ctrl->done_pair = 0u;
     }
+    ctrl->pd_hmin = kEncMinId;
+    ctrl->pd_a2max = kEncMaxId;
+    ctrl->pd_nfluid = 0u;
     if (zero_on_last) *zero_on_last = 0u;
     const double min_h = dec_d(eh);
     const double max_a2 = dec_d(ea2);
