@@ -65,6 +65,7 @@ __device__ __forceinline__ double dothr_drho(double rho, double othr, const AdjP
 struct AdjPtrs {
   const float4 *rec0;  // FP32 positions and signed h (prefilter)
   const double4_32a *r64a, *r64b;
+  const longlong2 *fix;  // integer positions (fp64_ops.cuh)
   const int *perm, *keys_sorted;
   const int2 *meta;
   const unsigned int *cstart;
@@ -115,6 +116,7 @@ template <int KERNEL, int G>
 __global__ void __launch_bounds__(kAdjBlock, 6) k_pair_adjoint(AdjPtrs P, AdjParams ap, Pair64 c) {
   constexpr int kCap = list_words<G>(ListCap<KERNEL>::value);
   constexpr bool gauss = KERNEL == SPH_KERNEL_GAUSSIAN;
+  constexpr bool kFix = G < 8;  // integer differences, as in the forward
   __shared__ unsigned int lists[kCap * kAdjBlock / G];
   const DevGrid &g = *P.grid;
   const long long k = ((long long)blockIdx.x * kAdjBlock + threadIdx.x) / G;
@@ -127,6 +129,9 @@ __global__ void __launch_bounds__(kAdjBlock, 6) k_pair_adjoint(AdjPtrs P, AdjPar
   if (G > 1 ? __any_sync(0xffffffffu, act) : act) {
     const double lAxk = P.lax[i], lAyk = P.lay[i], lDk = P.lad[i];
     const double ac = ap.alpha * 0.5 * ap.co;
+    const longlong2 pk = kFix ? P.fix[kq] : longlong2();
+    const int fix_s = g.fix_s;
+    const bool wide = g.pad_e > 0.5f * (float)g.r_search;
     const int2 qref = P.meta[kq];
     const bool slow = qref.x >= g.ncx;
     const int W = g.mode == 0 ? 1 : (slow ? g.wide : g.wt);
@@ -134,15 +139,17 @@ __global__ void __launch_bounds__(kAdjBlock, 6) k_pair_adjoint(AdjPtrs P, AdjPar
     const Stencil sten(g, qref, P.keys_sorted[kq], W);
     for_neighbours<G, kCap, kAdjBlock>(sten, P.cstart, act, lists, near, [&](unsigned int j) {
       const double4_32a Aj = P.r64a[j], Bj = P.r64b[j];
-      const double dx = Ak.x - Aj.x, dy = Ak.y - Aj.y;
-      const double d2 = fma(dx, dx, dy * dy);
+      PairGeom geo;
+      if constexpr (kFix) geo = wide ? pair_geom_wide(Ak.x - Aj.x, Ak.y - Aj.y) : pair_geom(pk, P.fix[j], fix_s);
+      else geo = pair_geom_fp64(Ak.x - Aj.x, Ak.y - Aj.y);
+      const double dx = geo.dx, dy = geo.dy, d2 = geo.d2;
       if (le_bits(d2, 1e-24)) return;  // coincident: no kernel gradient, no boundary force
       if (!signbit(Bj.w)) {
         // fluid pair: continuity + momentum with artificial viscosity.
         // dW = coef u; dci = (d coef / d r) / r
         double coef, dci;
         if constexpr (gauss) {
-          if (!le_bits(d2, c.lim_lo) && (!le_bits(d2, c.lim_hi) || !near_exact(dx, dy, hk))) return;
+          if (!le_bits(d2, c.lim_lo) && (!le_bits(d2, c.lim_hi) || !near_exact(Ak.x - Aj.x, Ak.y - Aj.y, hk))) return;
           if (le_bits(d2, c.h2)) return;
           const double ih2 = c.ih * c.ih;
           coef = c.i_0 * exp_neg(d2 * ih2);
@@ -150,7 +157,7 @@ __global__ void __launch_bounds__(kAdjBlock, 6) k_pair_adjoint(AdjPtrs P, AdjPar
         } else {
           if (!le_bits(d2, c.lim) || le_bits(d2, 1e-20)) return;
           double r, ir;
-          sqrt_rsqrt64(d2, r, ir);
+          sqrt_rsqrt64(geo.v, r, ir);
           if (KERNEL == SPH_KERNEL_CUBIC) {
             if (le_bits(d2, c.h2)) {
               coef = fma(c.i_r, r, c.i_0);
@@ -213,7 +220,7 @@ __global__ void __launch_bounds__(kAdjBlock, 6) k_pair_adjoint(AdjPtrs P, AdjPar
       if (!le_bits(d2, c.r02)) return;
       if (!c.lj_free) {  // the neighbour test
         const double hij = 0.5 * (hk + fabs(Bj.w)), t = 3.0 * hij, t2 = t * t;
-        if (!le_bits(d2, t2 * (1.0 - 1e-9)) && (!le_bits(d2, t2 * (1.0 + 1e-9)) || !near_exact(dx, dy, hij))) return;
+        if (!le_bits(d2, t2 * (1.0 - 1e-9)) && (!le_bits(d2, t2 * (1.0 + 1e-9)) || !near_exact(Ak.x - Aj.x, Ak.y - Aj.y, hij))) return;
       }
       const double ir2 = rcp64(d2);
       double sp1, sp2;
@@ -516,6 +523,7 @@ void launch_adjoint_step(const StepArgs &s, const StepArgs &h, const WsPtrs &w, 
   AdjPtrs P;
   P.rec0 = w.rec0;
   P.r64a = w.rec64a;
+  P.fix = reinterpret_cast<const longlong2 *>(w.rec1);
   P.r64b = w.rec64b;
   P.perm = w.perm;
   P.keys_sorted = w.keys_sorted;

@@ -428,7 +428,7 @@ static void compute_body(const StepArgs &a, const WsPtrs &w, const sph_wcsph_t &
                          double *dt_out, double *dt_hist, cudaStream_t st, const WallLoad *wall = nullptr,
                          bool write_state = true) {
   const bool do_dt = dt_out != nullptr || dt_hist != nullptr;
-  const RecParams rp = rec_params(cfg, wc, write_state, false, do_dt);
+  const RecParams rp = rec_params(a.n, cfg, wc, write_state, false, do_dt);
   launch_build(a, w, cfg, wc, st, &rp);
   if (wc.use_summation_density) {
     launch_sumdens(a, w, cfg, wc, st);
@@ -633,7 +633,7 @@ int sph_run_profiled(sph_particles_t *pa, const sph_wcsph_t *w, const sph_config
     double *nxt = ring + 3 * ((s + 1) & 1);
     launch_bounds(a, wp, *cfg, *w, s == 0 ? kStagePredict : kStageCorrectPredict, true, prev, cur, st);
     lap(SPH_STAGE_PREDICT);
-    const RecParams rp = rec_params(*cfg, *w, step_writes_state(*w, *cfg, s, nsteps), false, !fixed);
+    const RecParams rp = rec_params(a.n, *cfg, *w, step_writes_state(*w, *cfg, s, nsteps), false, !fixed);
     launch_build(a, wp, *cfg, *w, st, &rp);  // the records pass is fused into the build's last kernel
     lap(SPH_STAGE_BUILD);
     if (w->use_summation_density) {

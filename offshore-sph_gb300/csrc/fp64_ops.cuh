@@ -10,33 +10,235 @@ namespace sph {
 // ---------------------------------------------------------------------------
 // FP64 building blocks
 // ---------------------------------------------------------------------------
-// hardware estimates of 1/x and 1/sqrt(x) (normal x): the result's upper word
-__device__ __forceinline__ double rcp_est(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+// One FP64 instruction costs the SM as much issue time as 64 integer or FP32
+// ones, so reciprocal and square root run on the integer pipe: a 24-bit FP32
+// estimate and one Newton-type step of third order on 64-bit fixed-point
+// mantissas,
+//   1/x:        y (1 + e + e^2),          e = 1 - x y
+//   1/sqrt(x):  y (1 + e/2 + 3/8 e^2),    e = 1 - x y^2
+// (the binomial series of (1 - e)^-1 and (1 - e)^-1/2), rounded once to 53
+// bits.  The error before that rounding is below 2^-60, so the results are
+// within 0.51 ulp.  About 35 and 57 instructions instead of 3 and 6 FP64 ones
+// (Halley steps on the hardware's 2^-20 estimates).
+static __device__ __noinline__ double rcp64_slow(double x) { return 1.0 / x; }
+
+__device__ __forceinline__ float rcp_est_f(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ double rsqrt_est(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+__device__ __forceinline__ float rsqrt_est_f(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// 1/x: y (1 + e + e^2), e = 1 - x y; the estimate's error cubed is far below
-// an ulp
+// an estimate y0 in about [0.5, 1] as a fraction of 2^32 (24 bits of it)
+__device__ __forceinline__ unsigned int est_q32(float y0) {
+  y0 = fminf(fmaxf(y0, 0.5f), 0.99999994f);
+  return (__float_as_uint(y0) << 8) | 0x80000000u;
+}
+// y0 (1 + c) in units of 2^-63 from y0 in units of 2^-32 and c in units of
+// 2^-CB, |c| < 2^-20
+template <int CB>
+__device__ __forceinline__ unsigned long long refine_q63(unsigned int y0, long long c) {
+  const unsigned int ys = y0 >> 1;  // y0 in units of 2^-31
+  const unsigned long long lo = (unsigned long long)ys * (unsigned int)c;
+  const long long s = (long long)(int)ys * (int)(c >> 32) + (long long)(lo >> 32);  // units of 2^(1 - CB)
+  return ((unsigned long long)y0 << 31) + (unsigned long long)(s << (64 - CB));
+}
+// the double with 53-bit integer significand (m rounded to bit `drop`) whose
+// leading bit has the biased exponent e
+template <int DROP>
+__device__ __forceinline__ double pack64(unsigned long long m, int e, unsigned int sign = 0u) {
+  const unsigned long long r = (m + (1ull << (DROP - 1))) >> DROP;  // may carry into the exponent
+  const unsigned int hi = (unsigned int)(r >> 32) + ((unsigned int)(e - 1) << 20);
+  return __hiloint2double((int)(hi | sign), (int)(unsigned int)r);
+}
+
+// the product of two 64-bit fractions, within 3 units
+__device__ __forceinline__ unsigned long long mul_hi(unsigned long long a, unsigned long long b) {
+  const unsigned int a1 = (unsigned int)(a >> 32), a0 = (unsigned int)a;
+  const unsigned int b1 = (unsigned int)(b >> 32), b0 = (unsigned int)b;
+  return (unsigned long long)a1 * b1 + (((unsigned long long)a1 * b0) >> 32) + (((unsigned long long)a0 * b1) >> 32);
+}
+// 1 / v for v in [1, 2) in units of 2^-63, in units of 2^-63
+__device__ __forceinline__ unsigned long long rcp_q63(unsigned int vh, unsigned int vl) {
+  const unsigned int y0 = est_q32(rcp_est_f(__uint_as_float(0x3f800000u | ((vh >> 8) & 0x7fffffu))));
+  const unsigned long long p = (unsigned long long)vh * y0 + (((unsigned long long)vl * y0) >> 32);
+  const long long e1 = (long long)(0x8000000000000000ull - p);  // 1 - x y, units of 2^-63
+  const int eh = (int)(e1 >> 21);
+  const long long c = e1 + (long long)(((unsigned long long)((long long)eh * eh)) >> 21);
+  return refine_q63<63>(y0, c);
+}
+
 __device__ __forceinline__ double rcp64(double x) {
-  const double y = rcp_est(x);
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
+  const unsigned int hi = (unsigned int)__double2hiint(x), lo = (unsigned int)__double2loint(x);
+  const unsigned int e = (hi >> 20) & 0x7ffu;
+  if (e - 2u > 2042u) return rcp64_slow(x);  // zero, denormal, infinite, NaN, or a denormal result
+  const unsigned int mh = (hi & 0xfffffu) | 0x100000u;
+  return pack64<10>(rcp_q63(__funnelshift_l(lo, mh, 11), lo << 11), 2045 - (int)e, hi & 0x80000000u);
 }
-// r = sqrt(x) and ir = 1/sqrt(x): y (1 + e/2 + 3/8 e^2), e = 1 - x y^2
-__device__ __forceinline__ void sqrt_rsqrt64(double x, double &r, double &ir) {
-  const double y = rsqrt_est(x);
-  const double t = x * y;
-  const double e = fma(-t, y, 1.0);
-  const double c = fma(0.375, e, 0.5) * e;
-  r = fma(t, c, t);
-  ir = fma(y, c, y);
+
+// A positive number v 4^k, v in [1, 4) in units of 2^-62.
+struct Quad64 {
+  unsigned int vh, vl;
+  int k;
+};
+__device__ __forceinline__ Quad64 quad64(double x) {  // x > 0 normal
+  const unsigned int hi = (unsigned int)__double2hiint(x), lo = (unsigned int)__double2loint(x);
+  const int ue = (int)(hi >> 20) - 1023;
+  const unsigned int odd = (unsigned int)ue & 1u;
+  const unsigned int mh = (hi & 0xfffffu) | 0x100000u;
+  return {__funnelshift_l(lo, mh, 10u + odd), lo << (10u + odd), ue >> 1};
 }
+
+// y = 1 / sqrt(v 4^-k), in [0.5, 1], in units of 2^-63
+__device__ __forceinline__ unsigned long long rsqrt_q63(const Quad64 &v) {
+  const unsigned int vh = v.vh, vl = v.vl;
+  // v in FP32, truncated: its leading bit is bit 31 or 30 of vh
+  const unsigned int odd = vh >> 31;
+  const float vf = __uint_as_float(((126u + odd) << 23) + (vh >> (7u + odd)));
+  const unsigned int y0 = est_q32(rsqrt_est_f(vf));
+  const unsigned long long t = (unsigned long long)y0 * y0;  // y^2, units of 2^-64
+  const unsigned long long p = mul_hi(((unsigned long long)vh << 32) | vl, t);
+  const long long e1 = (long long)(0x4000000000000000ull - p);  // 1 - x y^2, units of 2^-62
+  const int eh = (int)(e1 >> 20);
+  const unsigned int e2 = (unsigned int)(((unsigned long long)((long long)eh * eh)) >> 22);  // e^2, units of 2^-62
+  const long long c = (e1 >> 1) + (long long)((3u * e2) >> 3);
+  return refine_q63<62>(y0, c);
+}
+// sqrt(v 4^-k) in units of 2^-61 from it
+__device__ __forceinline__ unsigned long long sqrt_q61(const Quad64 &v, unsigned long long y) {
+  return mul_hi(((unsigned long long)v.vh << 32) | v.vl, y);
+}
+// r = sqrt(v) and ir = 1 / sqrt(v)
+__device__ __forceinline__ void sqrt_rsqrt64(const Quad64 &v, double &r, double &ir) {
+  const unsigned long long y = rsqrt_q63(v);
+  ir = pack64<10>(y, 1022 - v.k);
+  r = pack64<9>(sqrt_q61(v, y), 1023 + v.k);
+}
+
+// A positive constant m 2^(e - 62), m in [2^62, 2^63).
+struct Fix64 {
+  unsigned long long m;
+  int e;
+};
+inline Fix64 fix64(double x) {
+  int e = 0;
+  const double f = frexp(x, &e);  // [0.5, 1)
+  return {(unsigned long long)ldexp(f, 63), e - 1};
+}
+
+// 1 / ((v + c) r), v a pair's squared distance, c > 0, r > 0: sum and product
+// on the integers as well, one rounding in all
+static __device__ __noinline__ double rcp_sum_slow(double d2, double c, double r) { return 1.0 / ((d2 + c) * r); }
+__device__ __forceinline__ double rcp_sum_prod(const Quad64 &v, const Fix64 &c, double r, double d2, double cd) {
+  const unsigned int rh = (unsigned int)__double2hiint(r), rl = (unsigned int)__double2loint(r);
+  const int er = (int)(rh >> 20);  // sign included: a negative r is out of range
+  if ((unsigned int)(er - 2) > 2042u) return rcp_sum_slow(d2, cd, r);
+  const int e = max(2 * v.k + 2, c.e + 1);
+  const unsigned long long vm = ((unsigned long long)v.vh << 32) | v.vl;
+  const unsigned long long s = (vm >> min(e - 2 * v.k, 63)) + (c.m >> min(e - c.e, 63));  // units of 2^(e - 62)
+  const int n = __clz((int)(s >> 32));  // 1 to 3
+  const unsigned long long rm = ((unsigned long long)(((rh & 0xfffffu) << 11) | 0x80000000u | (rl >> 21)) << 32) | (rl << 11);
+  unsigned long long p = mul_hi(s << n, rm);  // [2^62, 2^64)
+  const int lead = (int)(p >> 63);
+  p <<= 1 - lead;
+  // (v + c) r = (p / 2^63) 2^(e + 1 - n + er - 1023 + lead)
+  return pack64<10>(rcp_q63((unsigned int)(p >> 32), (unsigned int)p), 2044 - (e - n + er + lead));
+}
+
+// g(q) of the cubic spline's gradient factor -(al / h^2) g, q = r / h:
+// 3 - 2.25 q for q <= 1, 3 / q + 0.75 q - 3 = 0.75 (2 - q)^2 / q up to 2, from
+// the pair's squared distance and ih = 1 / h, h; q < 2 + 2^-40.  Fixed point,
+// absolute error below 2^-58.
+__device__ __forceinline__ double cubic_g(const Quad64 &v, const Fix64 &ih, const Fix64 &h) {
+  const unsigned long long y = rsqrt_q63(v);
+  // q = r ih in units of 2^-61: r = s 2^k, s in [1, 2) in units of 2^-61
+  const int sq = v.k + ih.e;  // q = (s ih.m) 2^sq, the product in [1, 4)
+  const unsigned long long q = mul_hi(sqrt_q61(v, y) << 2, ih.m << 1) >> min(max(1 - sq, 0), 63);
+  constexpr unsigned long long three = 3ull << 61;
+  unsigned long long g;
+  if (q <= 1ull << 61) {
+    g = three - 2 * q - (q >> 2);
+  } else {
+    // 1 / q = y h 2^-k in units of 2^-61: y in [0.5, 1], h.m / 2^62 in [1, 2)
+    const unsigned long long iq = mul_hi(y, h.m << 1) >> min(max(1 - (h.e - v.k), 0), 63);
+    const unsigned long long t = 3 * iq + (q >> 1) + (q >> 2);
+    g = t > three ? t - three : 0ull;
+  }
+  if (g == 0ull) return 0.0;
+  const int n = __clzll((long long)g);
+  return pack64<10>(g << (n - 1), 1086 - n - 61);
+}
+
+// ---------------------------------------------------------------------------
+// Positions as 64-bit integers, for pair differences on the integer pipe: a
+// position in units of 2^-s modulo 2^64, with s such that the interaction
+// radius is below 2^62 units (fix_shift), so that the difference of two
+// candidates' integers is that of their positions: exact for coordinates with
+// no bits below 2^-s (|x| > R / 512), within R 2^-61 for the others.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ int fix_shift(double R) {
+  return 61 - ((int)(((unsigned int)__double2hiint(R) >> 20) & 0x7ffu) - 1023);
+}
+__device__ __forceinline__ long long to_fix(double x, int s) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+  const int e = (int)((u >> 52) & 0x7ffu);
+  unsigned long long m = (u & 0xfffffffffffffull) | (e ? 0x10000000000000ull : 0ull);
+  const int sh = e - 1075 + s;
+  if (sh >= 0) m = sh < 64 ? m << sh : 0ull;
+  else m = sh > -64 ? m >> -sh : 0ull;
+  return (u >> 63) ? -(long long)m : (long long)m;
+}
+
+// A pair's geometry: the differences, the squared distance (each rounded once)
+// and the latter's significand for sqrt_rsqrt64.
+struct PairGeom {
+  double dx, dy, d2;
+  Quad64 v;
+};
+// |d| < 2^63 units of 2^-s as a double
+__device__ __forceinline__ double fix_diff(unsigned long long a, int s, bool neg) {
+  if (a == 0ull) return 0.0;
+  const int n = __clzll((long long)a);
+  return pack64<10>(a << (n - 1), 1086 - n - s, neg ? 0x80000000u : 0u);
+}
+// u^2 / 2^64, within 2 units
+__device__ __forceinline__ unsigned long long square_hi(unsigned long long u) {
+  const unsigned int u1 = (unsigned int)(u >> 32), u0 = (unsigned int)u;
+  return (unsigned long long)u1 * u1 + (((unsigned long long)u1 * u0) >> 31);
+}
+__device__ __forceinline__ PairGeom pair_geom(longlong2 a, longlong2 b, int s) {
+  PairGeom p;
+  const long long ix = (long long)((unsigned long long)a.x - (unsigned long long)b.x);
+  const long long iy = (long long)((unsigned long long)a.y - (unsigned long long)b.y);
+  const unsigned long long ux = ix < 0 ? -(unsigned long long)ix : (unsigned long long)ix;
+  const unsigned long long uy = iy < 0 ? -(unsigned long long)iy : (unsigned long long)iy;
+  p.dx = fix_diff(ux, s, ix < 0);
+  p.dy = fix_diff(uy, s, iy < 0);
+  // both shifted so that the larger's leading bit is bit 62
+  const int sh = __clzll((long long)(ux | uy | 1ull)) - 1;
+  const unsigned long long d = square_hi(ux << sh) + square_hi(uy << sh);  // [2^60, 2^63)
+  const bool big = (d >> 62) != 0ull;
+  const unsigned long long v = big ? d : d << 2;
+  p.v = {(unsigned int)(v >> 32), (unsigned int)v, (big ? 63 : 62) - sh - s};
+  const unsigned int odd = (unsigned int)(v >> 63);
+  p.d2 = (ux | uy) == 0ull ? 0.0 : pack64<10>(v >> odd, 1023 + 2 * p.v.k + (int)odd);
+  return p;
+}
+// the same by FP64 operations
+__device__ __forceinline__ PairGeom pair_geom_fp64(double dx, double dy) {
+  PairGeom p;
+  p.dx = dx;
+  p.dy = dy;
+  p.d2 = fma(dx, dx, dy * dy);
+  p.v = quad64(p.d2);
+  return p;
+}
+// out of line: where the padding of the FP32 test could let differences past
+// the integers' range through (a domain of some millions of radii)
+static __device__ __noinline__ PairGeom pair_geom_wide(double dx, double dy) { return pair_geom_fp64(dx, dy); }
 
 // a <= b for non-negative doubles (false when either is NaN and a is not
 // below b's pattern), without an FP64 instruction
@@ -126,6 +328,8 @@ struct Pair64 {
   double h2;                   // cubic: d2 <= h^2 is the inner piece.  Gaussian: d2 <= h2 has no gradient
   double o_ir, o_r, o_0;       // cubic, outer piece: o_ir / r + o_r r + o_0
   double i_r, i_0;             // inner piece: i_r r + i_0.  Wendland: (i_r r + i_0) (1 + o_r r)^5
+  double scale;                // FIX: of the gradient factor that is summed (cubic: -al / h^2)
+  Fix64 hf, ihf, hb2f;         // h, 1/h, hb2
   double al;                   // normalisation of W
   double hb2, pic;             // viscosity: pic dot / ((d2 + hb2) (rho_i + rho_j))
   double r02;                  // r0^2
@@ -168,6 +372,10 @@ inline Pair64 pair64_consts(const sph_config_t &cfg, const sph_wcsph_t &wc) {
   c.lim_lo = c.lim * (1.0 - 1e-9);
   c.lim_hi = c.lim * (1.0 + 1e-9);
   c.hb2 = 0.01 * (h * h);
+  c.hf = fix64(h);
+  c.ihf = fix64(ih);
+  c.hb2f = fix64(c.hb2);
+  c.scale = cfg.kernel == SPH_KERNEL_CUBIC ? -c.al * ih2 : 1.0;
   c.pic = -wc.alpha * wc.co * h;  // -2 alpha c_ij h with c_ij = co / 2
   c.r02 = wc.r0 * wc.r0;
   c.lj_free = cfg.h_fixed > 0.0 && wc.r0 < 1.5 * h * (1.0 - 1e-9);

@@ -19,7 +19,7 @@
 #include <string.h>
 
 #include "fp64_ops.cuh"
-#include "sph_internal.cuh"
+#include "pair_common.cuh"
 
 namespace sph {
 
@@ -390,6 +390,7 @@ __device__ unsigned grid_setup(double xmin, double xmax, double ymin, double yma
   double ext = fmax(xmax - xmin, ymax - ymin);
   R = fmax(R, fmax(ext * 1e-7, 1e-300));
   g->r_search = R;
+  g->fix_s = fix_shift(R);
   // the FP32 hi parts of the positions are truncated to 24 bits: a pair
   // distance formed from them is off by at most 2^-22 sqrt(2) max|coordinate|
   {
@@ -805,8 +806,8 @@ __device__ __forceinline__ void record_mixed(const StepArgs &a, long long k, int
 }
 
 // The FP64 form's records of slot k (particle i), the reference's arithmetic.
-__device__ __forceinline__ void record_fp64(const StepArgs &a, long long k, int i, const RecParams &rp,
-                                            float4 *__restrict__ rec0, double4_32a *__restrict__ r64a,
+__device__ __forceinline__ void record_fp64(const StepArgs &a, long long k, int i, const RecParams &rp, int fix_s,
+                                            float4 *__restrict__ rec0, float4 *__restrict__ rec1, double4_32a *__restrict__ r64a,
                                             double4_32a *__restrict__ r64b, unsigned long long &eh,
                                             unsigned int &nf) {
   const int8_t lab = a.label[i];
@@ -825,6 +826,7 @@ __device__ __forceinline__ void record_fp64(const StepArgs &a, long long k, int 
   const double othr = !fl ? 0.0 : (rho > 0.0 ? p * rcp64(rho * rho) : p / (rho * rho));
   const double hs = fl ? h : -h;
   r64a[k] = make_double4_32a(x, y, a.vx[i], a.vy[i]);
+  if (rp.fix) reinterpret_cast<longlong2 *>(rec1)[k] = make_longlong2(to_fix(x, fix_s), to_fix(y, fix_s));
   r64b[k] = make_double4_32a(m, rho, othr, (!fl && h == 0.0) ? -0.0 : hs);
   const float hf = d2f_trunc(h);
   rec0[k] = make_float4(xh, yh, fl ? hf : -hf, mf);
@@ -958,12 +960,12 @@ __global__ void __launch_bounds__(kBlock) k_cellsort(const int *__restrict__ per
     perm[slot] = v;
     meta[slot] = refcell[v];
     if (REC == kRecMixed) record_mixed_t<HSRC, PB>(a, slot, v, rp, rec0, rec1, rec2, eh, nf);
-    if (REC == kRecFp64) record_fp64(a, slot, v, rp, rec0, r64a, r64b, eh, nf);
+    if (REC == kRecFp64) record_fp64(a, slot, v, rp, gp->fix_s, rec0, rec1, r64a, r64b, eh, nf);
   }
   if (REC != kRecNone && rp.reduce_h) reduce_h_block(eh, nf, red, redn, ctrl);
 }
 
-RecParams rec_params(const sph_config_t &cfg, const sph_wcsph_t &wc, bool write_state, bool p_from_state,
+RecParams rec_params(long long n, const sph_config_t &cfg, const sph_wcsph_t &wc, bool write_state, bool p_from_state,
                      bool reduce_h) {
   RecParams rp;
   rp.h_fixed = cfg.h_fixed;
@@ -980,6 +982,7 @@ RecParams rec_params(const sph_config_t &cfg, const sph_wcsph_t &wc, bool write_
   rp.write_state = write_state ? 1 : 0;
   rp.from_state = p_from_state ? 1 : 0;
   rp.reduce_h = reduce_h ? 1 : 0;
+  rp.fix = lanes_per_query(n) < 8 ? 1 : 0;
   return rp;
 }
 
@@ -1032,7 +1035,7 @@ void launch_build(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, c
 // ---------------------------------------------------------------------------
 template <bool MIXED>
 __global__ void __launch_bounds__(kBlock) k_records(StepArgs a, const int *__restrict__ perm, RecParams rp,
-                                                    DevCtrl *ctrl, float4 *__restrict__ rec0,
+                                                    const DevGrid *__restrict__ gp, DevCtrl *ctrl, float4 *__restrict__ rec0,
                                                     float4 *__restrict__ rec1, float4 *__restrict__ rec2,
                                                     double4_32a *__restrict__ r64a,
                                                     double4_32a *__restrict__ r64b) {
@@ -1044,19 +1047,19 @@ __global__ void __launch_bounds__(kBlock) k_records(StepArgs a, const int *__res
   if (k < a.n) {
     const int i = perm[k];
     if (MIXED) record_mixed(a, k, i, rp, rec0, rec1, rec2, eh, nf);
-    else record_fp64(a, k, i, rp, rec0, r64a, r64b, eh, nf);
+    else record_fp64(a, k, i, rp, gp->fix_s, rec0, rec1, r64a, r64b, eh, nf);
   }
   if (rp.reduce_h) reduce_h_block(eh, nf, red, redn, ctrl);
 }
 
 void launch_records(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, const sph_wcsph_t &wc,
                     bool write_state, bool p_from_state, bool reduce_h, cudaStream_t st) {
-  const RecParams rp = rec_params(cfg, wc, write_state, p_from_state, reduce_h);
+  const RecParams rp = rec_params(a.n, cfg, wc, write_state, p_from_state, reduce_h);
   if (cfg.precision == SPH_PREC_MIXED)
-    k_records<true><<<nblocks(a.n), kBlock, 0, st>>>(a, w.perm, rp, w.ctrl, w.rec0, w.rec1, w.rec2, w.rec64a,
+    k_records<true><<<nblocks(a.n), kBlock, 0, st>>>(a, w.perm, rp, w.grid, w.ctrl, w.rec0, w.rec1, w.rec2, w.rec64a,
                                                      w.rec64b);
   else
-    k_records<false><<<nblocks(a.n), kBlock, 0, st>>>(a, w.perm, rp, w.ctrl, w.rec0, w.rec1, w.rec2, w.rec64a,
+    k_records<false><<<nblocks(a.n), kBlock, 0, st>>>(a, w.perm, rp, w.grid, w.ctrl, w.rec0, w.rec1, w.rec2, w.rec64a,
                                                       w.rec64b);
 }
 

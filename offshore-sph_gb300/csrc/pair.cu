@@ -1219,7 +1219,7 @@ __global__ void __launch_bounds__(kProbeBlock)
     const double t = 9.0 * hij * hij;
     if (!(d2 < t * (1.0 - 1e-9)) && !(__ddiv_rn(__dsqrt_rn(d2), hij) <= 3.0)) return;
     double r = 0.0, ir;
-    if (d2 > 0.0) sqrt_rsqrt64(d2, r, ir);
+    if (d2 > 0.0) sqrt_rsqrt64(quad64(d2), r, ir);
     // W(r, hw) (CubicSpline.py:12-36, Wendland.py:10-34, Gaussian.py:16-24)
     const double q = r * ihw;
     double w = 0.0;

@@ -3,23 +3,25 @@
 //
 // What bounds it: the FP64 pipe.  It takes 16 cycles per warp instruction
 // (2 lanes per SM and cycle), so one FP64 operation costs as much issue time
-// as some sixty FP32 or integer ones, and the kernel's time is the number of
-// FP64 operations per pair.  So:
+// as some sixty FP32 or integer ones.  So whatever has a cheap equal goes to the
+// other pipes (fp64_ops.cuh):
 //   - candidates are filtered in FP32 (padded) and compared on the integer
 //     pipe (positive doubles order like their bits);
-//   - reciprocals and square roots are one Halley step (cubic convergence)
-//     on the 2^-20 hardware estimate, not the compiler's divide and square
-//     root: 1/x in 3 operations, r and 1/r together in 6, each to about an
-//     ulp.  The neighbour test q = r / h_ij <= 3 (NNLinkedList.py:74) is redone
-//     with correctly rounded operations where an estimate could decide it
-//     differently;
-//   - with a uniform fluid h (Solver(h=...)) and beta = 0, the kernel gradient
-//     is a polynomial in r and 1/r whose coefficients are launch constants,
-//     and boundary neighbours beyond the Lennard-Jones reach are not listed
-//     (without XSPH they contribute nothing).
-// A pair of the cubic spline so takes 31 FP64 operations instead of about 90:
-// the 1M-fluid dam break's pair stage fell from 3.67 to 1.27 ms, and 20 steps
-// of 3200 fluid particles from 2.40 to 0.82 ms (with several lanes per query).
+//   - position differences and the squared distance come from 64-bit integer
+//     positions, reciprocals and square roots from 64-bit fixed-point Newton
+//     steps, each rounded once.  The neighbour test q = r / h_ij <= 3
+//     (NNLinkedList.py:74) is redone with correctly rounded operations where
+//     an estimate could decide it differently;
+//   - with a uniform fluid h (Solver(h=...)) and beta = 0, the cubic's gradient
+//     factor and the viscosity's reciprocal are fixed-point too, and boundary
+//     neighbours beyond the Lennard-Jones reach are not listed (without XSPH
+//     they contribute nothing).
+// A pair of the cubic spline so takes 13 FP64 operations instead of about 90.
+// 1M-fluid dam break, pair stage: 3.67 ms at 90, 1.27 ms at 31 (Halley steps and
+// launch-constant gradient polynomials in FP64), 0.76 ms now; the FP64 pipe
+// is busy 70% of it and 27% of the issue slots are used.  20 steps of 3200
+// fluid particles, where latency decides (several lanes per query): 2.40 ms,
+// 0.71 and 0.69.
 #include <type_traits>
 
 #include "fp64_ops.cuh"
@@ -28,38 +30,46 @@
 namespace sph {
 
 struct Acc64 {
-  double dd = 0.0, ax = 0.0, ay = 0.0, sx = 0.0, sy = 0.0, fr = 0.0;
+  double dd = 0.0, ax = 0.0, ay = 0.0, bx = 0.0, by = 0.0, sx = 0.0, sy = 0.0, fr = 0.0;
 };
 
 // The query's state (FP64 records).
 struct Query64 {
   double x, y, vx, vy, rho, oth, h;
+  longlong2 p;  // integer position
+  int fix_s;
+  bool wide;    // the integers' differences could wrap
 };
 
 // One listed candidate j of query q: the exact support test, then
 // continuity, momentum with artificial viscosity, the Lennard-Jones boundary
 // force and XSPH.  UH: every fluid h is c.h and beta = 0.
-template <int KERNEL, bool UH>
+// FIX: differences from the integer positions.
+template <int KERNEL, bool UH, bool FIX>
 __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 &c, const PairParams &pp,
-                                       const double4_32a &A, const double4_32a &B) {
+                                       longlong2 pj, const double4_32a &A, const double4_32a &B) {
   constexpr bool gauss = KERNEL == SPH_KERNEL_GAUSSIAN;
-  const double dx = q.x - A.x, dy = q.y - A.y;
-  const double d2 = fma(dx, dx, dy * dy);
+  PairGeom geo;
+  if constexpr (FIX) geo = q.wide ? pair_geom_wide(q.x - A.x, q.y - A.y) : pair_geom(q.p, pj, q.fix_s);
+  else geo = pair_geom_fp64(q.x - A.x, q.y - A.y);
+  const double dx = geo.dx, dy = geo.dy, d2 = geo.d2;
   const bool fluid = !signbit(B.w);
   if (fluid) {
     double coef, w = 0.0, hij = c.h, ih = c.ih;
     if constexpr (UH) {
       if constexpr (gauss) {
-        if (!le_bits(d2, c.lim_lo) && (!le_bits(d2, c.lim_hi) || !near_exact(dx, dy, hij))) return;
+        if (!le_bits(d2, c.lim_lo) && (!le_bits(d2, c.lim_hi) || !near_exact(q.x - A.x, q.y - A.y, hij))) return;
         const double e = exp_neg(d2 * (ih * ih));
         coef = le_bits(d2, c.h2) ? 0.0 : c.i_0 * e;
         if (c.xsph) w = c.al * e;
       } else {
         if (!le_bits(d2, c.lim)) return;  // W and its gradient are 0 at q >= 2
-        double r, ir;
-        sqrt_rsqrt64(d2, r, ir);
         const bool tiny = le_bits(d2, 1e-20);  // r < 1e-10: no gradient
-        if (KERNEL == SPH_KERNEL_CUBIC) {
+        double r = 0.0, ir;
+        if (!(FIX && KERNEL == SPH_KERNEL_CUBIC) || c.xsph) sqrt_rsqrt64(geo.v, r, ir);
+        if (FIX && KERNEL == SPH_KERNEL_CUBIC) {
+          coef = cubic_g(geo.v, c.ihf, c.hf);
+        } else if (KERNEL == SPH_KERNEL_CUBIC) {
           if (le_bits(d2, c.h2)) coef = fma(c.i_r, r, c.i_0);
           else coef = fma(c.o_ir, ir, fma(c.o_r, r, c.o_0));
         } else {
@@ -88,13 +98,13 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
       const double ih2 = ih * ih;
       if constexpr (gauss) {
         const double z = d2 * ih2;
-        if (!le_bits(z, 9.0 * (1.0 - 1e-9)) && (!le_bits(z, 9.0 * (1.0 + 1e-9)) || !near_exact(dx, dy, hij))) return;
+        if (!le_bits(z, 9.0 * (1.0 - 1e-9)) && (!le_bits(z, 9.0 * (1.0 + 1e-9)) || !near_exact(q.x - A.x, q.y - A.y, hij))) return;
         const double e = kInvPi * ih2 * exp_neg(z);
         coef = le_bits(d2, 1e-24 * ih2) ? 0.0 : -2.0 * e * ih2;
         w = e;
       } else {
         double r, ir;
-        sqrt_rsqrt64(d2, r, ir);
+        sqrt_rsqrt64(geo.v, r, ir);
         const bool tiny = le_bits(d2, 1e-20);
         if (tiny) r = 0.0;
         const double qq = r * ih;
@@ -119,14 +129,15 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
       }
     }
     const double vx = q.vx - A.z, vy = q.vy - A.w;
-    const double dot = fma(vx, dx, vy * dy);
+    const double dot = fma(vy, dy, vx * dx);
     const double mc = B.x * coef;
     s.dd = fma(mc, dot, s.dd);
     double S = q.oth + B.z;
     const double rs = q.rho + B.y;  // 2 rho_ij
     if (negative_bits(dot)) {
       if constexpr (UH) {
-        S = fma(c.pic * dot, rcp64((d2 + c.hb2) * rs), S);
+        const double inv = FIX ? rcp_sum_prod(geo.v, c.hb2f, rs, d2, c.hb2) : rcp64((d2 + c.hb2) * rs);
+        S = fma(c.pic * dot, inv, S);
       } else {
         // mu = h v.r / (r^2 + 0.01 h^2), Pi = mu (beta mu - alpha c_ij) / rho_ij
         const double hb = half_exact(q.h + hij);
@@ -156,7 +167,7 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
   const double hij = 0.5 * (q.h + hj);
   if (!(c.lj_free && lj) || xs) {  // the neighbour test
     const double t = 3.0 * hij, t2 = t * t;
-    if (!le_bits(d2, t2 * (1.0 - 1e-9)) && (!le_bits(d2, t2 * (1.0 + 1e-9)) || !near_exact(dx, dy, hij))) return;
+    if (!le_bits(d2, t2 * (1.0 - 1e-9)) && (!le_bits(d2, t2 * (1.0 + 1e-9)) || !near_exact(q.x - A.x, q.y - A.y, hij))) return;
     if (!(hij > 0.0)) return;
   }
   if (lj) {
@@ -170,8 +181,8 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
       t = pow(frac, pp.p1) - pow(frac, pp.p2);
     }
     const double fac = pp.D * t * ir2;
-    s.ax = fma(fac, dx, s.ax);
-    s.ay = fma(fac, dy, s.ay);
+    s.bx = fma(fac, dx, s.bx);
+    s.by = fma(fac, dy, s.by);
     if (pp.fr && A.x >= pp.wall_x) s.fr = fma(fac, dx, s.fr);
   }
   if (xs) {
@@ -216,9 +227,13 @@ struct Near64 {
 };
 
 template <int KERNEL, bool UH, int G>
-__global__ void __launch_bounds__(kPairBlock, 4)
+__global__ void __launch_bounds__(kPairBlock, G == 8 ? 4 : kPair64Blocks)
     k_pair64(StepArgs a, PairPtrs P, PairParams pp, Pair64 c, double *dt_out, double *dt_hist) {
   step_kernel_entry();
+  // Integer differences save FP64 issue time and lengthen a pair's chain: not
+  // where a query's latency is the time (20 steps of 3200 fluid particles 674
+  // us without, 695 with; 4 steps of 1M: 5117 and 4601)
+  constexpr bool kFix = G < 8;
   constexpr int kCap = list_words<G>(ListCap<KERNEL>::value);
   __shared__ unsigned int lists[kCap * kPairBlock / G];
   const DevGrid &g = *P.grid;
@@ -239,7 +254,8 @@ __global__ void __launch_bounds__(kPairBlock, 4)
     const bool slow = qref.x >= g.ncx || !(hif > 0.f);
     const int W = g.mode == 0 ? 1 : (slow ? g.wide : g.wt);
     const double4_32a A = P.r64a[kq], B = P.r64b[kq];
-    const Query64 q = {A.x, A.y, A.z, A.w, B.y, B.z, B.w};
+    const longlong2 *fix = reinterpret_cast<const longlong2 *>(P.rec1);
+    const Query64 q = {A.x, A.y, A.z, A.w, B.y, B.z, B.w, fix[kq], g.fix_s, g.pad_e > 0.5f * (float)g.r_search};
     Acc64 s;
     // the FP32 test: the padded reach of the pair's h (kernel support; a
     // boundary neighbour without XSPH: the Lennard-Jones reach min(r0, 3 h_ij))
@@ -249,8 +265,15 @@ __global__ void __launch_bounds__(kPairBlock, 4)
     const Near64<KERNEL, UH> near{P.rec0, P.meta, g, Qi, qref, (unsigned int)kq, rf2, r0f, pad, filter, c.xsph != 0};
     const Stencil sten(g, qref, qkey, W);
     for_neighbours<G, kCap, kPairBlock>(sten, P.cstart, act, lists, near, [&](unsigned int j) {
-      pair64<KERNEL, UH>(s, q, c, pp, P.r64a[j], P.r64b[j]);
+      pair64<KERNEL, UH, kFix>(s, q, c, pp, kFix ? fix[j] : longlong2(), P.r64a[j], P.r64b[j]);
     });
+    if (UH && kFix && KERNEL == SPH_KERNEL_CUBIC) {
+      s.dd *= c.scale;
+      s.ax *= c.scale;
+      s.ay *= c.scale;
+    }
+    s.ax += s.bx;
+    s.ay += s.by;
     group_sum<G>(s.dd);
     group_sum<G>(s.ax);
     group_sum<G>(s.ay);

@@ -8,6 +8,7 @@
 namespace sph {
 
 constexpr int kPairBlock = 128;
+constexpr int kPair64Blocks = 5;  // resident blocks per SM of the FP64 kernel (registers)
 // per-thread neighbour-list capacity: above the typical number of pairs inside
 // the support (about 21 for the cubic spline at h = 1.3 dx, 43 for the
 // Gaussian cut at 3h), so that the mid-walk flush -- which runs divergently --
@@ -190,7 +191,7 @@ __device__ __forceinline__ void group_sum(T &v) {
 // G = 8 where the GPU is idle and the chain is the time (5K particles: 1393 us
 // for 20 steps with G = 1, 858 with 4, 732 with 8, 793 with 16, 914 with 32).
 inline int lanes_per_query(long long n) {
-  const long long wave = (long long)sm_count() * kPairBlock * 4;
+  const long long wave = (long long)sm_count() * kPairBlock * kPair64Blocks;
   if (n < wave / 8) return 8;
   return n < wave / 2 || (n > wave && n < 4 * wave) ? 4 : 1;
 }

@@ -209,6 +209,7 @@ struct DevGrid {
   double ct;        // traversal cell size
   double hmax;      // max h after the h reset
   double r_search;  // interaction radius the pair kernels need
+  int fix_s;        // unit 2^-fix_s of the FP64 form's integer positions (fp64_ops.cuh)
   float pad_e;      // bound on |x_hi - x| + |x_j,hi - x_j| over the domain (prefilter padding)
   int valid;
 };
@@ -251,6 +252,7 @@ struct RecParams {
   int write_state;   // write p, c, h to the caller's arrays
   int from_state;    // p and h from the caller's arrays (second summation-density pass)
   int reduce_h;      // min h over fluid for the step's TimeStep
+  int fix;           // FP64 form: write the integer positions (lanes_per_query)
 };
 
 struct PairParams {
@@ -330,6 +332,7 @@ __device__ __forceinline__ void seg_add_u32(unsigned int v, int b, F &&commit) {
 //   rec1  float4 (x_lo, y_lo, rho, p / rho^2)    mixed form: x = x_hi + x_lo
 //   rec2  float4 (vx_hi, vy_hi, vx_lo, vy_lo)    mixed form
 //   rec64a double4 (x, y, vx, vy)                FP64 form
+//   rec1   longlong2 (x, y) as 64-bit integers   FP64 form (fp64_ops.cuh)
 //   rec64b double4 (m, rho, p / rho^2, h signed)
 struct WsPtrs {
   DevCtrl *ctrl;
@@ -860,7 +863,7 @@ inline StepArgs step_args(const sph_particles_t *pa) {
 enum IntStage { kStageNone = 0, kStagePredict = 1, kStageCorrectPredict = 2 };
 void launch_bounds(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, const sph_wcsph_t &wc, int stage,
                    bool h_reset, const double *dt_prev, const double *dt_cur, cudaStream_t st);
-RecParams rec_params(const sph_config_t &cfg, const sph_wcsph_t &wc, bool write_state, bool p_from_state,
+RecParams rec_params(long long n, const sph_config_t &cfg, const sph_wcsph_t &wc, bool write_state, bool p_from_state,
                      bool reduce_h);
 // neighbour build after launch_bounds; with rp the records pass is fused in
 void launch_build(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, const sph_wcsph_t &wc,

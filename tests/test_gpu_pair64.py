@@ -85,3 +85,18 @@ def test_narrow_tiles(max_cells):
         pa["v" + k][f] = rng.normal(0, 0.1, f.sum())
     _evaluate(pa, 0.5, 0.02, 0.026, CUBIC, True, max_cells)
     _evaluate(pa, 0.5, 0.02, 0.0, WEND, False, max_cells, beta=0.02)
+
+
+@pytest.mark.parametrize("kernel", [CUBIC, GAUSS, WEND])
+@pytest.mark.parametrize("offset, scale", [(0.0, 1.0), (-0.6, 1.0), (-37.125, 1.0), (1e3, 1.0), (1e5, 1.0),
+                                           (0.0, 1e-4), (0.0, 3e3)])
+def test_integer_differences(kernel, offset, scale):
+    """The integer positions (at 4 lanes): coordinates around zero, negative,
+    far from the origin up to where the FP64 differences take over (1e5 is 4
+    million interaction radii), and small and large units."""
+    from sph import scenarios as S
+    dx = 0.01 * scale
+    pa = S.jittered_lattice(121, 131, dx, seed=kernel)
+    pa["x"] += offset * scale
+    pa["y"] -= 0.5 * offset * scale
+    _evaluate(pa, 1.3 * scale, dx, 1.3 * dx, kernel, False)
