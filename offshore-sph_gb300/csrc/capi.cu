@@ -434,7 +434,7 @@ static void compute_body(const StepArgs &a, const WsPtrs &w, const sph_wcsph_t &
     launch_sumdens(a, w, cfg, wc, st);
     launch_records(a, w, cfg, wc, false, true, false, st);
   }
-  launch_pair(a, w, cfg, wc, dt_out, dt_hist, st, wall);
+  launch_pair(a, w, cfg, wc, dt_out, dt_hist, st, wall, write_state);
 }
 
 int sph_compute(sph_particles_t *pa, const sph_wcsph_t *w, const sph_config_t *cfg, const sph_workspace_t *ws,
@@ -641,7 +641,7 @@ int sph_run_profiled(sph_particles_t *pa, const sph_wcsph_t *w, const sph_config
       launch_records(a, wp, *cfg, *w, false, true, false, st);
     }
     lap(SPH_STAGE_RECORDS);
-    launch_pair(a, wp, *cfg, *w, fixed ? nullptr : nxt, nullptr, st);
+    launch_pair(a, wp, *cfg, *w, fixed ? nullptr : nxt, nullptr, st, nullptr, step_writes_state(*w, *cfg, s, nsteps));
     lap(SPH_STAGE_PAIR);
   }
   launch_correct(a, *cfg, ring + 3 * ((nsteps - 1) & 1), cfg->dt_fixed, st);

@@ -935,12 +935,13 @@ __global__ void __launch_bounds__(kBlock) k_cellsort(const int *__restrict__ per
       const unsigned int tbit = 1u << (tl & 31);
       const bool wall = (tflag[tl >> 5] & tbit) != 0u;
       if (wall) atomicAnd(&tflag[tl >> 5], ~tbit);
+      const int e2 = 2 * tl + (wall ? 1 : 0);  // the entry says so as well
       const unsigned int te = __ldg(&cstart[(tl + 1) << ts2]);
       if (te - (unsigned)k >= (1u << ts2)) {
-        if (wall) tiles_h[atomicAdd(&ctrl->tl_heavy, 1u)] = tl;
-        else tiles[atomicAdd(&ctrl->tl_count, 1u)] = tl;
+        if (wall) tiles_h[atomicAdd(&ctrl->tl_heavy, 1u)] = e2;
+        else tiles[atomicAdd(&ctrl->tl_count, 1u)] = e2;
       } else {
-        tiles[tiles_cap - 1 - atomicAdd(&ctrl->tl_back, 1u)] = tl;
+        tiles[tiles_cap - 1 - atomicAdd(&ctrl->tl_back, 1u)] = e2;
       }
     }
     const int v = perm_tmp[k];
@@ -1144,6 +1145,8 @@ __global__ void k_bt_grid(BatchPtrs B, DevCtrl *ctrl) {
     B.coff[B.n_inst] = total;
     B.scan->ncells = total - 1;  // the scan kernels cover ids 0 .. run - 1
     ctrl->tl_count = 0;
+    ctrl->tl_back = 0;
+    ctrl->build_epoch++;
   }
 }
 
@@ -1197,8 +1200,10 @@ __global__ void __launch_bounds__(kBlock) k_bt_cellsort(const int *__restrict__ 
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long eh = kEncMinId;
   unsigned int nf = 0;
-  int b = -1;
+  int b = -1, tl = -1;
   const int lane = threadIdx.x & 31;
+  int tcell = -1 - lane;  // the first cell of a fluid particle's tile; other lanes match no other
+  unsigned int tsize = 0;
   const bool act = k < n;
   const int key = act ? keys_sorted[k] : -1 - lane;  // inactive lanes match no other lane
   const int v = act ? perm_tmp[k] : 0;
@@ -1213,9 +1218,24 @@ __global__ void __launch_bounds__(kBlock) k_bt_cellsort(const int *__restrict__ 
     const int c0 = B.coff[b], lk = key - c0;
     const DevGrid &g = B.grids[b];
     const int ts2 = 2 * g.ts;
-    if (lk < g.ncells && (unsigned)k == __ldg(&cstart[c0 + ((lk >> ts2) << ts2)]))
-      B.tiles[atomicAdd(&ctrl->tl_count, 1u)] = make_int2(b, lk >> ts2);
+    if (lk < g.ncells && is_fluid(a.label[v])) {
+      tl = lk >> ts2;
+      tcell = c0 + (tl << ts2);
+      tsize = 1u << ts2;
+    }
     record_mixed(a, slot, v, B.ip[b].rp, rec0, rec1, rec2, eh, nf);
+  }
+  // A tile with fluid is listed once, by the first warp that stamps it with
+  // this build's number: the small tanks hold many tiles of wall particles
+  // alone, which have no query.
+  const unsigned int tpeers = __match_any_sync(0xffffffffu, tcell);
+  if (tl >= 0 && lane == __ffs(tpeers) - 1) {
+    const unsigned int epoch = ctrl->build_epoch;
+    if (atomicExch(&B.stamp[tcell], epoch) != epoch) {
+      const int2 e = make_int2(b, tl);
+      if (cstart[tcell + tsize] - cstart[tcell] >= tsize) B.tiles[atomicAdd(&ctrl->tl_count, 1u)] = e;
+      else B.tiles[B.tiles_cap - 1 - atomicAdd(&ctrl->tl_back, 1u)] = e;
+    }
   }
   InstSlots *sl = B.sl;
   seg_min_u64(eh, b, [&](int q, unsigned long long m) { atomicMin(&sl[q].pd_hmin, m); });

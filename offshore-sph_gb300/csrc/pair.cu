@@ -36,93 +36,51 @@ struct MixedAcc {
   float fd = 0.f, fax = 0.f, fay = 0.f, fbx = 0.f, fby = 0.f, fsx = 0.f, fsy = 0.f;
 };
 
-struct MixedConsts {
-  float KC, r02f, co, alpha, beta, eps, D;
-  float avc;  // alpha c_ij with c_ij = co / 2 (Momentum.py's averaged c, the neighbour's c being 0)
-};
-
-template <int KERNEL>
-__device__ __forceinline__ MixedConsts mixed_consts(const PairParams &pp) {
-  MixedConsts c;
-  c.KC = (float)(Support<KERNEL>::q * Support<KERNEL>::q);  // (support / h)^2
-  const float r0f = (float)pp.r0;
-  c.r02f = r0f * r0f;
-  c.co = (float)pp.co;
-  c.alpha = (float)pp.alpha;
-  c.beta = (float)pp.beta;
-  c.eps = (float)pp.eps;
-  c.D = (float)pp.D;
-  c.avc = c.alpha * 0.5f * c.co;
-  return c;
+// two FP32 operations in one instruction, each rounded as its scalar form
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.ftz.f32x2 z, x, y;\n"
+      " mov.b64 {%0, %1}, z;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
 }
-
-// Uniform fluid h (the run has a fixed h, Solver(h=...)) and beta = 0 (the
-// reference's WCSPH default): every fluid record carries the same FP32 h, so
-// for a fluid query i and a fluid neighbour j, h_ij = 0.5 (h_i + h_j) = h_i
-// exactly, and the averaged h of the viscosity term is h_i as well.  The
-// kernel, gradient and viscosity constants are then per query, computed once,
-// and with beta = 0 the viscosity
-//   Pi_ij = mu (beta mu - alpha c_ij) / rho_ij,  mu = h v.r / (r^2 + 0.01 h^2)
-// is (-2 alpha c_ij h) v.r / ((r^2 + 0.01 h^2)(rho_i + rho_j)): one
-// reciprocal per pair.
-struct UniformQ {
-  float lim;     // (support h)^2
-  float inv_h;   // 1 / h
-  float al;      // the kernel's normalisation at h
-  float g0, g1, g2;  // kernel-gradient polynomial coefficients with al / h folded in
-  float hb2;     // 0.01 h^2 (viscosity denominator)
-  float pic;     // -2 alpha c_ij h (viscosity numerator)
-};
-
-template <int KERNEL>
-__device__ __forceinline__ UniformQ uniform_q(const MixedConsts &c, float h) {
-  UniformQ u;
-  u.lim = c.KC * (h * h);
-  u.inv_h = __fdividef(1.0f, h);
-  const float fac = KERNEL == SPH_KERNEL_CUBIC ? (float)kCubicFac
-                                               : (KERNEL == SPH_KERNEL_WENDLAND ? (float)kWendFac : (float)kInvPi);
-  u.al = fac * u.inv_h * u.inv_h;
-  const float alh = u.al * u.inv_h;
-  if (KERNEL == SPH_KERNEL_CUBIC) {
-    // dW/dr / r = al/h (-0.75 (2 - q)^2) / r (q > 1), al/h q (2.25 q - 3) / r (q <= 1)
-    u.g0 = -0.75f * alh;
-    u.g1 = 2.25f * alh;
-    u.g2 = -3.0f * alh;
-  } else if (KERNEL == SPH_KERNEL_WENDLAND) {
-    // dW/dr / r = al/h (1 - q/2)^5 q (-14/3 - 35/3 q) / r
-    u.g0 = (-14.0f / 3.0f) * alh;
-    u.g1 = (-35.0f / 3.0f) * alh;
-    u.g2 = 0.f;
-  } else {
-    // dW/dr / r = -2 al / h^2 exp(-q^2)
-    u.g0 = -2.0f * alh * u.inv_h;
-    u.g1 = u.g2 = 0.f;
-  }
-  u.hb2 = 0.01f * (h * h);
-  u.pic = -2.0f * c.avc * h;
-  return u;
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n sub.rn.ftz.f32x2 z, x, y;\n"
+      " mov.b64 {%0, %1}, z;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
+// differences of the double-float positions and velocities
+__device__ __forceinline__ float2 diff_pos(float4 Qi, float4 Ri, float4 qj, float4 rj) {
+  return add2(sub2(lo2(Qi), lo2(qj)), sub2(lo2(Ri), lo2(rj)));
+}
+__device__ __forceinline__ float2 diff_vel(float4 Vi, float4 vj) {
+  return add2(sub2(lo2(Vi), lo2(vj)), sub2(hi2(Vi), hi2(vj)));
 }
 
 // One FLUID neighbour j of fluid query i under a uniform fluid h and beta = 0
 // (see UniformQ): the same equations as mixed_pair's fluid branch with the
 // per-pair h arithmetic taken out.
 template <int KERNEL, bool XSPH, bool SUMDENS>
-__device__ __forceinline__ void mixed_fluid_uh(MixedAcc &acc, const MixedConsts &c, const UniformQ &u, float hq,
-                                               float4 Qi, float4 Ri, float4 Vi, float4 qj, float4 rj,
-                                               const float4 *vjp) {
-  const float dx = (Qi.x - qj.x) + (Ri.x - rj.x);
-  const float dy = (Qi.y - qj.y) + (Ri.y - rj.y);
+__device__ __forceinline__ void mixed_fluid_uh(MixedAcc &acc, const MixedConsts &c, const UniformQ &u, float4 Qi,
+                                               float4 Ri, float4 Vi, float4 qj, float4 rj, const float4 *vjp) {
+  const float2 d = diff_pos(Qi, Ri, qj, rj);
+  const float dx = d.x, dy = d.y;
   const float d2 = dx * dx + dy * dy;
   if (d2 > u.lim) return;
-  const float4 vj = *vjp;
+  const float2 v = diff_vel(Vi, *vjp);
+  const float vxij = v.x, vyij = v.y;
   // 1/r, and 0 below r = 1e-10 (d2 = 1e-20), where the kernel gradient of
   // the 2h kernels is taken as 0: the guard on the gradient folds into it
   const bool g2h = KERNEL == SPH_KERNEL_CUBIC || KERNEL == SPH_KERNEL_WENDLAND;
   const float inv_r = d2 >= (g2h ? 1e-20f : 0.f) && d2 > 0.f ? rsqrtf(d2) : 0.f;
   const float r = d2 * inv_r;
   const float q = r * u.inv_h;
-  const float vxij = (Vi.x - vj.x) + (Vi.z - vj.z);
-  const float vyij = (Vi.y - vj.y) + (Vi.w - vj.w);
   float w = 0.f, coef;
   if (KERNEL == SPH_KERNEL_CUBIC) {
     const float t2 = fmaxf(2.0f - q, 0.f);
@@ -138,7 +96,7 @@ __device__ __forceinline__ void mixed_fluid_uh(MixedAcc &acc, const MixedConsts 
   } else {
     const float e = __expf(-q * q);
     if (XSPH) w = u.al * e;
-    coef = r * hq > 1e-12f ? u.g0 * e : 0.f;
+    coef = r * u.h > 1e-12f ? u.g0 * e : 0.f;
   }
   const float dwx = coef * dx, dwy = coef * dy;
   const float mj = qj.w;
@@ -156,6 +114,21 @@ __device__ __forceinline__ void mixed_fluid_uh(MixedAcc &acc, const MixedConsts 
   }
 }
 
+// One boundary neighbour j without XSPH: the Lennard-Jones force alone
+// (BoundaryForce.py:6-42), at r <= min(r0, 3 h_ij).
+__device__ __forceinline__ void mixed_boundary(MixedAcc &acc, const MixedConsts &c, float4 Qi, float4 Ri, float4 qj,
+                                               float4 rj) {
+  const float2 d = diff_pos(Qi, Ri, qj, rj);
+  const float d2 = d.x * d.x + d.y * d.y;
+  const float hij = 0.5f * (Qi.z + fabsf(qj.z));
+  if (d2 > fminf(c.r02f, 9.0f * (hij * hij)) || !(d2 > 1e-24f)) return;
+  const float ir2 = __fdividef(1.0f, d2);
+  const float f2 = c.r02f * ir2;
+  const float fac = c.D * (f2 * f2 - f2) * ir2;
+  acc.fbx = fmaf(fac, d.x, acc.fbx);
+  acc.fby = fmaf(fac, d.y, acc.fby);
+}
+
 // One candidate j of query i: the exact support test, then continuity,
 // momentum with artificial viscosity, the Lennard-Jones boundary force and
 // XSPH.  Qi/qj: x_hi, y_hi, h (sign bit: non-fluid), m; Ri/rj: x_lo, y_lo,
@@ -164,23 +137,26 @@ __device__ __forceinline__ void mixed_fluid_uh(MixedAcc &acc, const MixedConsts 
 template <int KERNEL, bool XSPH, bool SUMDENS>
 __device__ __forceinline__ void mixed_pair(MixedAcc &acc, const MixedConsts &c, float4 Qi, float4 Ri, float4 Vi,
                                            float4 qj, float4 rj, const float4 *vjp) {
+  const bool jf = !signbit(qj.z);
+  if (!XSPH && !jf) {
+    mixed_boundary(acc, c, Qi, Ri, qj, rj);
+    return;
+  }
   const float hif = Qi.z;
-  const float dx = (Qi.x - qj.x) + (Ri.x - rj.x);
-  const float dy = (Qi.y - qj.y) + (Ri.y - rj.y);
+  const float2 d = diff_pos(Qi, Ri, qj, rj);
+  const float dx = d.x, dy = d.y;
   const float d2 = dx * dx + dy * dy;
   const float hij = 0.5f * (hif + fabsf(qj.z));
   const float h2 = hij * hij;
-  const bool jf = !signbit(qj.z);
   float lim = c.KC * h2;
   if (!jf) lim = fmaxf(lim, fminf(c.r02f, 9.0f * h2));
   if (d2 > lim) return;
-  const float4 vj = *vjp;
+  const float2 v = diff_vel(Vi, *vjp);
+  const float vxij = v.x, vyij = v.y;
   const float inv_h = __fdividef(1.0f, hij);
   const float inv_r = d2 > 0.f ? rsqrtf(d2) : 0.f;
   const float r = d2 * inv_r;
   const float q = r * inv_h;
-  const float vxij = (Vi.x - vj.x) + (Vi.z - vj.z);
-  const float vyij = (Vi.y - vj.y) + (Vi.w - vj.w);
   float w, coef;
   if (KERNEL == SPH_KERNEL_CUBIC) {
     const float al = (float)kCubicFac * inv_h * inv_h;
@@ -234,7 +210,7 @@ template <int KERNEL, bool XSPH, bool SUMDENS, bool UH>
 __device__ __forceinline__ void mixed_entry(MixedAcc &acc, const MixedConsts &c, const UniformQ &u, float4 Qi,
                                             float4 Ri, float4 Vi, float4 qj, float4 rj, const float4 *vjp) {
   if (UH && !signbit(qj.z))
-    mixed_fluid_uh<KERNEL, XSPH, SUMDENS>(acc, c, u, Qi.z, Qi, Ri, Vi, qj, rj, vjp);
+    mixed_fluid_uh<KERNEL, XSPH, SUMDENS>(acc, c, u, Qi, Ri, Vi, qj, rj, vjp);
   else
     mixed_pair<KERNEL, XSPH, SUMDENS>(acc, c, Qi, Ri, Vi, qj, rj, vjp);
 }
@@ -242,7 +218,8 @@ __device__ __forceinline__ void mixed_entry(MixedAcc &acc, const MixedConsts &c,
 // Writes the derivatives of particle i (gravity on y) and returns its encoded
 // a^2 for the TimeStep reduction.
 template <bool XSPH, bool SUMDENS>
-__device__ __forceinline__ unsigned long long mixed_store(const MixedAcc &acc, const StepArgs &a, int i) {
+__device__ __forceinline__ unsigned long long mixed_store(const MixedAcc &acc, const StepArgs &a, int i,
+                                                          int write_xsph) {
   const float axs = acc.fax + acc.fbx, ays = acc.fay + acc.fby;
   a.ax[i] = f2d(axs);
   a.ay[i] = f2d(ays) - 9.81;
@@ -250,7 +227,7 @@ __device__ __forceinline__ unsigned long long mixed_store(const MixedAcc &acc, c
   if (XSPH) {
     a.xsphx[i] = a.vx[i] + f2d(acc.fsx);
     a.xsphy[i] = a.vy[i] + f2d(acc.fsy);
-  } else {
+  } else if (write_xsph) {
     a.xsphx[i] = 0.0;
     a.xsphy[i] = 0.0;
   }
@@ -284,8 +261,8 @@ __device__ __forceinline__ unsigned long long pair_query(const StepArgs &a, cons
       const int W = g.mode == 0 ? 1 : (slow ? g.wide : g.wt);
       const float4 Ri = P.rec1[k], Vi = P.rec2[k];  // x_lo, y_lo, rho, p / rho^2; velocities
       MixedAcc acc;
-      const MixedConsts mc = mixed_consts<KERNEL>(pp);
-      const UniformQ uq = uniform_q<KERNEL>(mc, hif);
+      const MixedConsts &mc = pp.mc;
+      const UniformQ &uq = pp.u;
 
       // ---- phase 2: pair physics over the list
       auto physics = [&](int cnt) {
@@ -306,7 +283,10 @@ __device__ __forceinline__ unsigned long long pair_query(const StepArgs &a, cons
         const float d2 = dx * dx + dy * dy;
         const float hij = 0.5f * (hif + fabsf(qj.z));
         float reach = SK * hij;
-        if (signbit(qj.z)) reach = fmaxf(reach, fminf(r0f, 3.0f * hij) * 1.000002f);
+        if (signbit(qj.z)) {
+          const float lj = fminf(r0f, 3.0f * hij) * 1.000002f;
+          reach = XSPH ? fmaxf(reach, lj) : lj;
+        }
         const float rp = reach + pad;
         if (d2 <= rp * rp) {
           lists[nl][tid] = j;
@@ -322,7 +302,7 @@ __device__ __forceinline__ unsigned long long pair_query(const StepArgs &a, cons
       // slow queries, whose set size is counted exactly
       const bool any = !slow || exact_count(a, P.perm, g, qref, qkey, W, g.mode == 1, P.meta, cst, a.x[i], a.y[i],
                                             a.h[i]) > 0;
-      if (any) ea = mixed_store<XSPH, SUMDENS>(acc, a, i);
+      if (any) ea = mixed_store<XSPH, SUMDENS>(acc, a, i, pp.write_xsph);
       else ea = enc_d(accel2(a.ax[i], a.ay[i]));  // keeps its previous values (SolverTools.py:150-153)
     }
   }
@@ -585,6 +565,7 @@ struct TileGeom {
   int cell0;  // global id of the grid's first cell (batched form; 0 otherwise)
   long long ncx;
   float r0f, pad, hmaxf;
+  float rb2;  // squared, padded Lennard-Jones reach
 };
 
 __device__ __forceinline__ TileGeom tile_geom(const DevGrid &g, double r0, int cell0) {
@@ -602,6 +583,8 @@ __device__ __forceinline__ TileGeom tile_geom(const DevGrid &g, double r0, int c
   tg.r0f = (float)r0;
   tg.pad = g.pad_e;
   tg.hmaxf = g.hmaxf;
+  const float rb = fminf(tg.r0f, 3.0f * tg.hmaxf) * 1.000002f + tg.pad;
+  tg.rb2 = rb * rb;
   return tg;
 }
 
@@ -613,7 +596,7 @@ struct TileShared {
   unsigned int hoff[kHaloCellsMax + 1];  // shared-memory offset of each halo cell, then the total
   unsigned int hgs[kHaloCellsMax];       // its first sorted slot
   unsigned short qmap[kHaloCap];         // halo cell of each query of the tile
-  int s_tile[2];                         // this and the next claimed work unit (-1: none left)
+  long long s_tile[2];                   // this and the next claimed work unit (-1: none left)
   int s_inst[2];                         // their instances (batched form)
   unsigned long long red[kTileThreads / 32];
 };
@@ -632,12 +615,12 @@ struct TileShared {
 // UH: every fluid particle has the same h (UniformQ).
 // part: 0 the whole tile; 1 and 2 its first and second half of cell rows;
 // 3 to 6 its four quarters (the kernel's last tiles are split so that its
-// final round of work is short).
+// final round of work is short).  wall: it holds boundary particles.
 template <int KERNEL, bool XSPH, bool SUMDENS, bool UH, int TSC, int WC>
 __device__ __forceinline__ unsigned long long tile_process(const StepArgs &a, const PairPtrs &P, const TileGeom &tg,
-                                                           const MixedConsts &mc, int t, int part,
+                                                           const PairParams &pp, int t, int part, bool wall,
                                                            TileShared<KERNEL> &sm, DevCtrl *ctrl, int2 *fb,
-                                                           unsigned int fb_cap, bool skip_dry) {
+                                                           unsigned int fb_cap) {
   constexpr int kListCap = ListCap<KERNEL>::value;
   const int tid = threadIdx.x;
   const int ts = TSC ? TSC : tg.ts;
@@ -654,18 +637,7 @@ __device__ __forceinline__ unsigned long long tile_process(const StepArgs &a, co
   const unsigned int tb = (unsigned int)t << (2 * ts);  // the tile's first cell (row-major inside)
   const unsigned int qs = __ldg(&cst[tb + row0 * T]), qe = __ldg(&cst[tb + (row0 + rows) * T]);
   const int ox = (t % ntlx) * T - W, oy = (t / ntlx) * T + row0 - W;
-  // 1. halo table: counts and first slots.  With skip_dry (the batched form,
-  // whose small tanks hold many tiles of wall particles alone), alongside,
-  // for a sparse unit (less than one particle per cell), whether its own
-  // slots hold a fluid particle (the sign bit of a record's h marks the
-  // others): a unit of boundary particles alone has no query and stages
-  // nothing.  A sparse unit has fewer slots than the block has threads: one
-  // load per thread, issued before the table's loads and used only at the
-  // barrier.  (On the single-scene dam break the test cost more than the
-  // few dry tiles it saves.)
-  const bool dense = !skip_dry || qe - qs >= (unsigned int)(T * rows);
-  float hq0 = -1.f;  // sign bit set: no fluid
-  if (!dense && qs + tid < qe) hq0 = __ldg(&P.rec0[qs + tid].z);
+  // 1. halo table: counts and first slots
   for (int c = tid; c < HC; c += kTileThreads) {
     const int x = ox + c % HW, y = oy + c / HW;
     unsigned int gs = 0, cnt = 0;
@@ -677,7 +649,7 @@ __device__ __forceinline__ unsigned long long tile_process(const StepArgs &a, co
     hgs[c] = gs;
     hoff[c] = cnt;
   }
-  if (!__syncthreads_or(dense || !signbit(hq0))) return ea;
+  __syncthreads();
   if (tid < 32) {  // 2. exclusive scan of the counts, kHaloScanPer cells per lane
     const int c0 = tid * kHaloScanPer;
     unsigned int v[kHaloScanPer], sum = 0;
@@ -764,8 +736,18 @@ __device__ __forceinline__ unsigned long long tile_process(const StepArgs &a, co
   cp_async_wait_all();
   __syncthreads();
   // 3. queries.  Candidate radius: the padded reach of the largest pair h
-  // (every |h| <= hmaxf), so that one compare per candidate suffices
-  const float SK = (float)Support<KERNEL>::q * 1.000002f;  // support / h, padded
+  // (every |h| <= hmaxf), so that one compare per candidate suffices; next to
+  // a wall, without XSPH, boundary candidates have the Lennard-Jones reach for
+  // theirs (they are several times denser than the fluid, and inside the kernel
+  // support most of them do nothing)
+  const MixedConsts &mc = pp.mc;
+  const UniformQ uq = pp.u;  // in registers: read per pair
+  auto reach2 = [&](float h) {
+    const float hq = 0.5f * (h + tg.hmaxf);
+    const float rq = fmaxf((float)Support<KERNEL>::q * 1.000002f * hq, fminf(tg.r0f, 3.0f * hq) * 1.000002f) + tg.pad;
+    return rq * rq;
+  };
+  const float rq2_uh = UH ? reach2(uq.h) : 0.f;
   const unsigned int nq = qe - qs;
   for (unsigned int q = tid; q < nq; q += kTileThreads) {
     const int hc = sm.qmap[q];
@@ -782,7 +764,6 @@ __device__ __forceinline__ unsigned long long tile_process(const StepArgs &a, co
     }
     const float4 Ri = h1[sq], Vi = h2[sq];
     const int i = P.perm[k];
-    const UniformQ uq = uniform_q<KERNEL>(mc, hif);
     MixedAcc acc;
     auto physics = [&](int cnt) {
 #pragma unroll kTileUnrollPairs
@@ -791,42 +772,53 @@ __device__ __forceinline__ unsigned long long tile_process(const StepArgs &a, co
         mixed_entry<KERNEL, XSPH, SUMDENS, UH>(acc, mc, uq, Qi, Ri, Vi, h0[j], h1[j], h2 + j);
       }
     };
-    const float hq = 0.5f * (hif + tg.hmaxf);
-    const float rq = fmaxf(SK * hq, fminf(tg.r0f, 3.0f * hq) * 1.000002f) + tg.pad;
-    const float rq2 = rq * rq;
+    const float rq2 = UH ? rq2_uh : reach2(hif);
     int nl = 0;
-    // the stencil rows' slot ranges, the query's own row as the two ranges
-    // either side of its own slot (the particle itself is no candidate)
-    for (int r = -W, seg = 0; r <= W; seg = 0, r++) {
-      const unsigned int *row = hoff + (hy + r) * HW + hx;
-      unsigned int j = row[-W];
-      const unsigned int e = row[W + 1];
-      unsigned int se = r == 0 ? sq : e;
-      for (;;) {
-        while (j < se) {
-          if (nl == kListCap) {
-            physics(nl);
-            nl = 0;
-          }
-          // a chunk that cannot overflow the list: every candidate is
-          // written, and kept (counted) when inside the radius
-          const unsigned int ce = min(se, j + (unsigned int)(kListCap - nl));
+    auto walk = [&](auto near_wall) {
+      constexpr bool kWall = decltype(near_wall)::value;
+      // the stencil rows' slot ranges, the query's own row as the two ranges
+      // either side of its own slot (the particle itself is no candidate)
+      for (int r = -W, seg = 0; r <= W; seg = 0, r++) {
+        const unsigned int *row = hoff + (hy + r) * HW + hx;
+        unsigned int j = row[-W];
+        const unsigned int e = row[W + 1];
+        unsigned int se = r == 0 ? sq : e;
+        for (;;) {
+          while (j < se) {
+            if (nl == kListCap) {
+              physics(nl);
+              nl = 0;
+            }
+            // a chunk that cannot overflow the list: every candidate is
+            // written, and kept (counted) when inside the radius
+            const unsigned int ce = min(se, j + (unsigned int)(kListCap - nl));
 #pragma unroll kTileUnrollCands
-          for (; j < ce; j++) {
-            const float2 p = *reinterpret_cast<const float2 *>(h0 + j);
-            const float dx = Qi.x - p.x, dy = Qi.y - p.y;
-            sm.lists[nl][tid] = (unsigned short)j;
-            nl += fmaf(dx, dx, dy * dy) <= rq2 ? 1 : 0;
+            for (; j < ce; j++) {
+              float2 p;
+              float lim = rq2;
+              if (kWall) {
+                const float4 p4 = h0[j];
+                p = lo2(p4);
+                lim = signbit(p4.z) ? tg.rb2 : rq2;
+              } else {
+                p = *reinterpret_cast<const float2 *>(h0 + j);
+              }
+              const float2 d = sub2(lo2(Qi), p);
+              sm.lists[nl][tid] = (unsigned short)j;
+              nl += fmaf(d.x, d.x, d.y * d.y) <= lim ? 1 : 0;
+            }
           }
+          if (r != 0 || seg) break;
+          seg = 1;
+          j = sq + 1;
+          se = e;
         }
-        if (r != 0 || seg) break;
-        seg = 1;
-        j = sq + 1;
-        se = e;
       }
-    }
+    };
+    if (wall && !XSPH) walk(std::true_type());
+    else walk(std::false_type());
     physics(nl);
-    const unsigned long long qa = mixed_store<XSPH, SUMDENS>(acc, a, i);
+    const unsigned long long qa = mixed_store<XSPH, SUMDENS>(acc, a, i, pp.write_xsph);
     ea = qa > ea ? qa : ea;
   }
   __syncthreads();
@@ -849,14 +841,14 @@ __device__ __forceinline__ unsigned long long block_max_u64(unsigned long long v
 // the tile of a single-scene grid with the shape the grid has
 template <int KERNEL, bool XSPH, bool SUMDENS, bool UH>
 __device__ __forceinline__ unsigned long long tile_any(const StepArgs &a, const PairPtrs &P, const TileGeom &tg,
-                                                       const MixedConsts &mc, int t, int part,
+                                                       const PairParams &pp, int t, int part, bool wall,
                                                        TileShared<KERNEL> &sm, DevCtrl *ctrl, int2 *fb,
-                                                       unsigned int fb_cap, bool skip_dry) {
+                                                       unsigned int fb_cap) {
   if (tg.ts == 4 && tg.W == 2)
-    return tile_process<KERNEL, XSPH, SUMDENS, UH, 4, 2>(a, P, tg, mc, t, part, sm, ctrl, fb, fb_cap, skip_dry);
+    return tile_process<KERNEL, XSPH, SUMDENS, UH, 4, 2>(a, P, tg, pp, t, part, wall, sm, ctrl, fb, fb_cap);
   if (tg.ts == 3 && tg.W == 2)
-    return tile_process<KERNEL, XSPH, SUMDENS, UH, 3, 2>(a, P, tg, mc, t, part, sm, ctrl, fb, fb_cap, skip_dry);
-  return tile_process<KERNEL, XSPH, SUMDENS, UH, 0, 0>(a, P, tg, mc, t, part, sm, ctrl, fb, fb_cap, skip_dry);
+    return tile_process<KERNEL, XSPH, SUMDENS, UH, 3, 2>(a, P, tg, pp, t, part, wall, sm, ctrl, fb, fb_cap);
+  return tile_process<KERNEL, XSPH, SUMDENS, UH, 0, 0>(a, P, tg, pp, t, part, wall, sm, ctrl, fb, fb_cap);
 }
 
 template <int KERNEL, bool XSPH, bool SUMDENS, bool UH>
@@ -872,7 +864,6 @@ __global__ void __launch_bounds__(kTileThreads, TileBlocks<KERNEL>::value)
   const DevGrid *gp = P.grid;
   const TileGeom tg = tile_geom(*gp, pp.r0, 0);
   const bool filter = gp->mode == 1 && (gp->need_filter || ctrl->alias_count > 0);
-  const MixedConsts mc = mixed_consts<KERNEL>(pp);
   unsigned long long ea = kEncMaxId;
 
   if (filter || tg.HC > kHaloCellsMax) {
@@ -888,8 +879,9 @@ __global__ void __launch_bounds__(kTileThreads, TileBlocks<KERNEL>::value)
     // list), then the sparse ones (listed from its back).  Of that order, the
     // last `sq` tiles come as four quarter-tile units each and the `sh`
     // before them as two half-tile units each, so that the kernel's final
-    // rounds of work are short.  A unit is encoded as 8 tile + part (part 0:
-    // whole tile; 1, 2: halves; 3 to 6: quarters), -1 when none is left.
+    // rounds of work are short.  A unit is encoded as 8 entry + part (part 0:
+    // whole tile; 1, 2: halves; 3 to 6: quarters), -1 when none is left; an
+    // entry is 2 tile + 1 when the tile holds boundary particles.
     const unsigned int nh = ctrl->tl_heavy, ntl = nh + ctrl->tl_count, nall = ntl + ctrl->tl_back;
     const unsigned int sq = (kSplitTail && tg.ts >= 2) ? min(nall, gridDim.x / 4u) : 0u;
     const unsigned int sh = (kSplitTail && tg.ts >= 1) ? min(nall - sq, gridDim.x) : 0u;
@@ -897,12 +889,12 @@ __global__ void __launch_bounds__(kTileThreads, TileBlocks<KERNEL>::value)
     auto tile_at = [&](unsigned int p) {
       return p < nh ? tiles_h[p] : (p < ntl ? tiles[p - nh] : tiles[tiles_cap - 1 - (p - ntl)]);
     };
-    auto claim = [&](unsigned int c) {
-      if (c < nw) return 8 * tile_at(c);
+    auto claim = [&](unsigned int c) -> long long {
+      if (c < nw) return 8ll * tile_at(c);
       c -= nw;
-      if (c < 2 * sh) return 8 * tile_at(nw + (c >> 1)) + 1 + (int)(c & 1u);
+      if (c < 2 * sh) return 8ll * tile_at(nw + (c >> 1)) + 1 + (int)(c & 1u);
       c -= 2 * sh;
-      return c < 4 * sq ? 8 * tile_at(nw + sh + (c >> 2)) + 3 + (int)(c & 3u) : -1;
+      return c < 4 * sq ? 8ll * tile_at(nw + sh + (c >> 2)) + 3 + (int)(c & 3u) : -1;
     };
     if (tid == 0) {
       if (blockIdx.x == 0) {  // the dump cell (reference-OOB particles) is in no tile
@@ -913,12 +905,12 @@ __global__ void __launch_bounds__(kTileThreads, TileBlocks<KERNEL>::value)
     }
     __syncthreads();
     for (int it = 0;; it++) {
-      const int u = sm.s_tile[it & 1];
+      const long long u = sm.s_tile[it & 1];
       if (u < 0) break;
       if (tid == 0)  // claim the next unit while this one runs
         sm.s_tile[(it + 1) & 1] = claim(atomicAdd(&ctrl->tile_next, 1u));
       const unsigned long long q =
-          tile_any<KERNEL, XSPH, SUMDENS, UH>(a, P, tg, mc, u >> 3, u & 7, sm, ctrl, fb, fb_cap, false);
+          tile_any<KERNEL, XSPH, SUMDENS, UH>(a, P, tg, pp, (int)(u >> 4), (int)u & 7, (u & 8) != 0, sm, ctrl, fb, fb_cap);
       ea = q > ea ? q : ea;
     }
   }
@@ -952,28 +944,56 @@ __global__ void __launch_bounds__(kTileThreads, TileBlocks<KERNEL>::value)
   TileShared<KERNEL> &sm = *reinterpret_cast<TileShared<KERNEL> *>(smem_raw);
   const int tid = threadIdx.x;
   DevCtrl *ctrl = P.ctrl;
-  const unsigned int ntl = ctrl->tl_count;
+  // Work units as in k_pair_tiles: dense tiles from the front of the list,
+  // sparse ones from its back, the last of them in quarters and halves (a tile
+  // too small to split comes whole with its first part).
+  const unsigned int ntl = ctrl->tl_count, nall = ntl + ctrl->tl_back;
+  const unsigned int sq = min(nall, gridDim.x / 4u), sh = min(nall - sq, gridDim.x);
+  const unsigned int nw = nall - sq - sh;  // whole-tile units
+  auto claim = [&](int slot) {
+    unsigned int c = atomicAdd(&ctrl->tile_next, 1u), p = nall, part = 0, first = 1, split = 0;
+    if (c < nw) {
+      p = c;
+    } else if (c - nw < 2 * sh) {
+      c -= nw;
+      p = nw + (c >> 1);
+      part = 1 + (c & 1u);
+      first = !(c & 1u);
+      split = 1;
+    } else if (c - nw - 2 * sh < 4 * sq) {
+      c -= nw + 2 * sh;
+      p = nw + sh + (c >> 2);
+      part = 3 + (c & 3u);
+      first = !(c & 3u);
+      split = 2;
+    }
+    int2 e = make_int2(-1, -1);
+    if (p < nall) {
+      e = p < ntl ? B.tiles[p] : B.tiles[B.tiles_cap - 1 - (p - ntl)];
+      if (B.grids[e.x].ts < (int)split) part = first ? 0 : 7;  // 7: nothing to do
+    }
+    sm.s_inst[slot] = e.x;
+    sm.s_tile[slot] = p < nall ? 8 * e.y + (int)part : -1;
+  };
   if (tid == 0) {
-    if (blockIdx.x == 0)  // every instance's dump cell (reference-OOB particles) is in no tile
-      for (int b = 0; b < B.n_inst; b++) {
-        const int c = B.coff[b] + B.grids[b].ncells;
-        const unsigned int d0 = __ldg(&P.cstart[c]), d1 = __ldg(&P.cstart[c + 1]);
-        for (unsigned int s = d0; s < d1; s += kPairBlock) fb_push(ctrl, fb, fb_cap, s, min((unsigned)kPairBlock, d1 - s));
-      }
-    const unsigned int c = atomicAdd(&ctrl->tile_next, 1u);
-    const int2 e = c < ntl ? B.tiles[c] : make_int2(-1, -1);
-    sm.s_inst[0] = e.x;
-    sm.s_tile[0] = e.y;
+    // every instance's dump cell (reference-OOB particles) is in no tile.  (One
+    // block walking all instances took longer than the tiles.)
+    for (int b = blockIdx.x; b < B.n_inst; b += gridDim.x) {
+      const int c = B.coff[b] + B.grids[b].ncells;
+      const unsigned int d0 = __ldg(&P.cstart[c]), d1 = __ldg(&P.cstart[c + 1]);
+      for (unsigned int s = d0; s < d1; s += kPairBlock) fb_push(ctrl, fb, fb_cap, s, min((unsigned)kPairBlock, d1 - s));
+    }
+    claim(0);
   }
   __syncthreads();
   for (int it = 0;; it++) {
-    const int t = sm.s_tile[it & 1], b = sm.s_inst[it & 1];
-    if (t < 0) break;
-    if (tid == 0) {  // claim the next tile while this one runs
-      const unsigned int c = atomicAdd(&ctrl->tile_next, 1u);
-      const int2 e = c < ntl ? B.tiles[c] : make_int2(-1, -1);
-      sm.s_inst[(it + 1) & 1] = e.x;
-      sm.s_tile[(it + 1) & 1] = e.y;
+    const int u = (int)sm.s_tile[it & 1], b = sm.s_inst[it & 1];
+    if (u < 0) break;
+    if (tid == 0) claim((it + 1) & 1);  // the next unit while this one runs
+    const int t = u >> 3;
+    if ((u & 7) == 7) {
+      __syncthreads();
+      continue;
     }
     const DevGrid &g = B.grids[b];
     const PairParams &pp = B.ip[b].pp;
@@ -982,16 +1002,18 @@ __global__ void __launch_bounds__(kTileThreads, TileBlocks<KERNEL>::value)
     if (filter || tg.HC > kHaloCellsMax) {  // this instance's tiles go to the global path
       if (tid == 0) {
         const unsigned int *cst = P.cstart + tg.cell0;
-        const unsigned int qs = __ldg(&cst[t << (2 * tg.ts)]), qe = __ldg(&cst[(t + 1) << (2 * tg.ts)]);
+        // the unit's rows of the tile (all of them, a half, a quarter)
+        const int part = u & 7, T = 1 << tg.ts, rows = part == 0 ? T : (part <= 2 ? T >> 1 : T >> 2);
+        const int c0 = (t << (2 * tg.ts)) + (part == 0 ? 0 : (part <= 2 ? part - 1 : part - 3) * rows * T);
+        const unsigned int qs = __ldg(&cst[c0]), qe = __ldg(&cst[c0 + rows * T]);
         for (unsigned int s = qs; s < qe; s += kPairBlock) fb_push(ctrl, fb, fb_cap, s, min((unsigned)kPairBlock, qe - s));
       }
       __syncthreads();
       continue;
     }
-    const MixedConsts mc = mixed_consts<KERNEL>(pp);
     const unsigned long long ea =
-        pp.beta == 0.0 ? tile_any<KERNEL, XSPH, SUMDENS, true>(a, P, tg, mc, t, 0, sm, ctrl, fb, fb_cap, true)
-                       : tile_any<KERNEL, XSPH, SUMDENS, false>(a, P, tg, mc, t, 0, sm, ctrl, fb, fb_cap, true);
+        pp.beta == 0.0 ? tile_any<KERNEL, XSPH, SUMDENS, true>(a, P, tg, pp, t, u & 7, true, sm, ctrl, fb, fb_cap)
+                       : tile_any<KERNEL, XSPH, SUMDENS, false>(a, P, tg, pp, t, u & 7, true, sm, ctrl, fb, fb_cap);
     const unsigned long long ba = block_max_u64<kTileThreads>(ea, sm.red);
     if (tid == 0 && ba != kEncMaxId) atomicMax(&B.sl[b].pd_a2max, ba);
   }
@@ -1355,8 +1377,9 @@ static void pair_dispatch(const StepArgs &a, const WsPtrs &w, const sph_config_t
 }
 
 void launch_pair(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, const sph_wcsph_t &wc,
-                 double *dt_out, double *dt_hist, cudaStream_t st, const WallLoad *wall) {
+                 double *dt_out, double *dt_hist, cudaStream_t st, const WallLoad *wall, bool write_state) {
   PairParams pp = pair_params(a, cfg, wc, dt_out != nullptr || dt_hist != nullptr);
+  pp.write_xsph = write_state ? 1 : 0;
   if (wall) {
     pp.wall_x = wall->wall_x;
     pp.fr = wall->fr;

@@ -288,8 +288,10 @@ __global__ void __launch_bounds__(kPairBlock, G == 8 ? 4 : kPair64Blocks)
       if (!slow || exact_count(a, P.perm, g, qref, qkey, W, g.mode == 1, P.meta, P.cstart, q.x, q.y, q.h) > 0) {
         const double axf = s.ax, ayf = s.ay - 9.81;
         a.drho[i] = c.sumdens ? 0.0 : s.dd;
-        a.xsphx[i] = c.xsph ? q.vx + s.sx : 0.0;
-        a.xsphy[i] = c.xsph ? q.vy + s.sy : 0.0;
+        if (c.xsph || pp.write_xsph) {
+          a.xsphx[i] = c.xsph ? q.vx + s.sx : 0.0;
+          a.xsphy[i] = c.xsph ? q.vy + s.sy : 0.0;
+        }
         ea = enc_d(accel2(axf, ayf));
         a.ax[i] = axf;
         a.ay[i] = ayf;

@@ -36,8 +36,49 @@ inline PairPtrs pair_ptrs(const WsPtrs &w) {
   return P;
 }
 
+// The FP32 constants of pp (alpha, beta, ... set) for a kernel and a fixed h
+// (h <= 0: none, the uniform-h constants are not used).
+inline void mixed_constants(PairParams &pp, int kernel, double h_fixed) {
+  MixedConsts &c = pp.mc;
+  const float support = kernel == SPH_KERNEL_GAUSSIAN ? 3.f : 2.f;
+  c.KC = support * support;  // (support / h)^2
+  const float r0f = (float)pp.r0;
+  c.r02f = r0f * r0f;
+  c.co = (float)pp.co;
+  c.alpha = (float)pp.alpha;
+  c.beta = (float)pp.beta;
+  c.eps = (float)pp.eps;
+  c.D = (float)pp.D;
+  UniformQ &u = pp.u;
+  const float h = h_fixed > 0.0 ? (float)h_fixed : 1.f;
+  u.h = h;
+  u.lim = c.KC * (h * h);
+  u.inv_h = 1.0f / h;
+  u.al = (float)(kernel == SPH_KERNEL_CUBIC ? kCubicFac : (kernel == SPH_KERNEL_WENDLAND ? kWendFac : kInvPi)) * u.inv_h *
+         u.inv_h;
+  const float alh = u.al * u.inv_h;
+  if (kernel == SPH_KERNEL_CUBIC) {
+    // dW/dr / r = al/h (-0.75 (2 - q)^2) / r (q > 1), al/h q (2.25 q - 3) / r (q <= 1)
+    u.g0 = -0.75f * alh;
+    u.g1 = 2.25f * alh;
+    u.g2 = -3.0f * alh;
+  } else if (kernel == SPH_KERNEL_WENDLAND) {
+    // dW/dr / r = al/h (1 - q/2)^5 q (-14/3 - 35/3 q) / r
+    u.g0 = (-14.0f / 3.0f) * alh;
+    u.g1 = (-35.0f / 3.0f) * alh;
+    u.g2 = 0.f;
+  } else {
+    // dW/dr / r = -2 al / h^2 exp(-q^2)
+    u.g0 = -2.0f * alh * u.inv_h;
+    u.g1 = u.g2 = 0.f;
+  }
+  u.hb2 = 0.01f * (h * h);
+  u.pic = -2.0f * (c.alpha * 0.5f * c.co) * h;
+}
+
 inline PairParams pair_params(const StepArgs &a, const sph_config_t &cfg, const sph_wcsph_t &wc, bool do_dt) {
   PairParams pp;
+  pp.write_xsph = 1;
   pp.wall_x = 0.0;
   pp.fr = nullptr;
   pp.alpha = wc.alpha; pp.beta = wc.beta; pp.co = wc.co; pp.eps = wc.epsilon;
@@ -46,6 +87,7 @@ inline PairParams pair_params(const StepArgs &a, const sph_config_t &cfg, const 
   pp.cfl_c = cfg.cfl_c; pp.cfl_f = cfg.cfl_f;
   pp.do_dt = do_dt ? 1 : 0;
   pp.n = a.n;
+  mixed_constants(pp, cfg.kernel, cfg.h_fixed);
   return pp;
 }
 

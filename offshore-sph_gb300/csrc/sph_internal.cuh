@@ -174,6 +174,7 @@ struct DevCtrl {
   // tiles holding a boundary particle in their own list, tl_count other dense
   // ones from the front of the tile list, tl_back sparse ones from its back
   unsigned int tl_count, tl_back, tl_heavy;
+  unsigned int build_epoch;  // builds of the batched form
   unsigned int bounds_done;  // finished blocks of the bounds pass (its last block sets the grid)
   double dt_ring[2][3];  // {dt, dt_c, dt_f} of the step with that parity
   GridKey grid_key;      // inputs of the grid in use
@@ -255,7 +256,34 @@ struct RecParams {
   int fix;           // FP64 form: write the integer positions (lanes_per_query)
 };
 
+// FP32 constants of the mixed form's pair physics (formed on the host).
+struct MixedConsts {
+  float KC, r02f, co, alpha, beta, eps, D;
+};
+
+// Uniform fluid h (the run has a fixed h, Solver(h=...)) and beta = 0 (the
+// reference's WCSPH default): every fluid record carries the same FP32 h, so
+// for a fluid query i and a fluid neighbour j, h_ij = 0.5 (h_i + h_j) = h_i
+// exactly, and the averaged h of the viscosity term is h_i as well.  The
+// kernel, gradient and viscosity constants are then per query, computed once,
+// and with beta = 0 the viscosity
+//   Pi_ij = mu (beta mu - alpha c_ij) / rho_ij,  mu = h v.r / (r^2 + 0.01 h^2)
+// is (-2 alpha c_ij h) v.r / ((r^2 + 0.01 h^2)(rho_i + rho_j)): one
+// reciprocal per pair.
+struct UniformQ {
+  float h;
+  float lim;     // (support h)^2
+  float inv_h;   // 1 / h
+  float al;      // the kernel's normalisation at h
+  float g0, g1, g2;  // kernel-gradient polynomial coefficients with al / h folded in
+  float hb2;     // 0.01 h^2 (viscosity denominator)
+  float pic;     // -2 alpha c_ij h (viscosity numerator)
+};
+
 struct PairParams {
+  MixedConsts mc;
+  UniformQ u;
+  int write_xsph;  // write the XSPH velocity of a run without XSPH (zeros)
   double alpha, beta, co, eps, r0, D, p1, p2;
   int lj_42;  // p1 == 4 and p2 == 2
   double cfl_c, cfl_f;
@@ -290,7 +318,9 @@ struct BatchPtrs {
   DevGrid *grids;    // per instance
   int *coff;         // first global cell id of each instance, then the total
   int *inst;         // instance of each particle (caller order)
-  int2 *tiles;       // (instance, tile) of the non-empty tiles of the build
+  int2 *tiles;       // (instance, tile) of the build's tiles with fluid: dense ones from the front, sparse from the back
+  unsigned int tiles_cap;
+  unsigned int *stamp;  // by a tile's first cell: the build that listed it
   DevGrid *scan;     // ncells = total cells - 1, for the scan kernels
   int n_inst;
 };
@@ -881,7 +911,7 @@ struct WallLoad {
 };
 void launch_pair(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, const sph_wcsph_t &wc,
                  double *dt_out, double *dt_hist, cudaStream_t st,
-                 const WallLoad *wall = nullptr);
+                 const WallLoad *wall = nullptr, bool write_state = true);
 void launch_pair64(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, const sph_wcsph_t &wc,
                    const PairParams &pp, double *dt_out, double *dt_hist, cudaStream_t st);
 void launch_sum_fixed(const double *v, long long n, double *out, cudaStream_t st);
