@@ -129,6 +129,89 @@ inline Fix64 fix64(double x) {
   return {(unsigned long long)ldexp(f, 63), e - 1};
 }
 
+// exp(-z) for 0 <= z < 11: table lookup and a short polynomial (P. T. P. Tang,
+// Table-driven implementation of the exponential function in IEEE
+// floating-point arithmetic, ACM TOMS 15, 1989), in 64-bit fixed point: z / ln 2
+// = n / 2048 + t, |t| <= 1/4096, x = |t| ln 2,
+// exp(-z) = 2^(-n / 2048) (1 -+ (x + x^3 / 6) + x^2 / 2 + x^4 / 24), the sum's
+// error below 2^-57.
+constexpr int kExpN = 2048;
+struct ExpTable {
+  unsigned long long v[kExpN];  // 2^(-i / 2048) in units of 2^-62
+};
+struct DD {
+  double hi, lo;
+};
+constexpr DD dd_two_prod(double a, double b) {  // Dekker's product
+  const double p = a * b;
+  const double c1 = 134217729.0 * a, c2 = 134217729.0 * b;
+  const double ah = c1 - (c1 - a), bh = c2 - (c2 - b);
+  const double al = a - ah, bl = b - bh;
+  return {p, ((ah * bh - p) + ah * bl + al * bh) + al * bl};
+}
+constexpr DD dd_mul(DD a, DD b) {
+  const DD p = dd_two_prod(a.hi, b.hi);
+  const double l = p.lo + (a.hi * b.lo + a.lo * b.hi);
+  const double s = p.hi + l;
+  return {s, l - (s - p.hi)};
+}
+constexpr ExpTable make_exp_table() {
+  // c = 2^(-1/2048) = exp(-ln 2 / 2048) as a double-double Taylor sum
+  const DD x = {-0x1.62e42fefa39efp-1 / kExpN, -0x1.abc9e3b39803fp-56 / kExpN};
+  DD term = {1.0, 0.0}, c = {1.0, 0.0};
+  for (int k = 1; k <= 8; k++) {
+    term = dd_mul(term, x);
+    const DD inv = {1.0 / k, 0.0};
+    // term / k with one correction of the quotient
+    const DD q0 = dd_mul(term, inv);
+    const DD back = dd_mul(q0, DD{(double)k, 0.0});
+    const double fix = ((term.hi - back.hi) + (term.lo - back.lo)) / k;
+    const double qh = q0.hi + (q0.lo + fix);
+    term = DD{qh, (q0.lo + fix) - (qh - q0.hi)};
+    const double s = c.hi + term.hi;
+    const double err = (c.hi - s) + term.hi;
+    const double lo = err + (c.lo + term.lo);
+    const double s2 = s + lo;
+    c = DD{s2, lo - (s2 - s)};
+  }
+  ExpTable t = {};
+  DD v = {1.0, 0.0};
+  for (int i = 0; i < kExpN; i++) {
+    t.v[i] = (unsigned long long)(v.hi * 0x1p62) + (unsigned long long)(long long)(v.lo * 0x1p62);
+    v = dd_mul(v, c);
+  }
+  return t;
+}
+__device__ constexpr ExpTable g_exp_table = make_exp_table();
+
+// exp(-v c / log2(e)), i.e. 2^(-v c), for v c < 16: a squared distance and
+// log2(e) / h^2
+__device__ __forceinline__ double exp2_neg(const Quad64 &v, const Fix64 &c) {
+  const unsigned long long p = mul_hi(((unsigned long long)v.vh << 32) | v.vl, c.m << 1);  // units of 2^-61
+  const unsigned long long u = p >> min(max(3 - 2 * v.k - c.e, 0), 63);                    // v c, units of 2^-58
+  const unsigned int n = (unsigned int)((u + (1ull << 46)) >> 47);
+  const long long t = (long long)(u - ((unsigned long long)n << 47));  // units of 2^-58
+  const unsigned long long T = __ldg(&g_exp_table.v[n & (kExpN - 1)]);
+  // x = |t| ln 2 in units of 2^-75
+  const unsigned long long x = mul_hi((unsigned long long)(t < 0 ? -t : t) << 17, 0xb17217f7d1cf79acull);
+  const unsigned int xh = (unsigned int)(x >> 31);  // units of 2^-44
+  const unsigned long long x2 = (unsigned long long)xh * xh;  // units of 2^-88
+  const unsigned int x2h = (unsigned int)(x2 >> 32);          // units of 2^-56
+  const unsigned int x3 = __umulhi(__umulhi(x2h, xh), 0x2aaaaaabu);   // x^3 / 6, units of 2^-68
+  const unsigned int x4 = __umulhi(__umulhi(x2h, x2h), 0x0aaaaaabu);  // x^4 / 24, units of 2^-80
+  const unsigned long long even = (x2 >> 14) + (x4 >> 5), odd = x + ((unsigned long long)x3 << 7);
+  // t >= 0: 1 - (odd - even); t < 0: 1 + (odd + even)
+  const unsigned long long m = mul_hi(T, t < 0 ? odd + even : odd - even) >> 11;
+  const unsigned long long e = t < 0 ? T + m : T - m;  // just around [2^61, 2^62]
+  const int low = __clz((int)(e >> 32)) - 1;             // 0 to 2
+  return pack64<10>(e << low, 1023 - low - (int)(n >> 11));
+}
+// exp(-z), 0 <= z < 11
+__device__ __forceinline__ double exp_neg(double z) {
+  constexpr Fix64 log2e = {0x5c551d94ae0bf85eull, 0};
+  return exp2_neg(quad64(z), log2e);
+}
+
 // 1 / ((v + c) r), v a pair's squared distance, c > 0, r > 0: sum and product
 // on the integers as well, one rounding in all
 static __device__ __noinline__ double rcp_sum_slow(double d2, double c, double r) { return 1.0 / ((d2 + c) * r); }
@@ -246,77 +329,6 @@ __device__ __forceinline__ bool le_bits(double a, double b) {
   return (unsigned long long)__double_as_longlong(a) <= (unsigned long long)__double_as_longlong(b);
 }
 
-// exp(-z) for 0 <= z < 16: table lookup and a short polynomial (P. T. P. Tang,
-// Table-driven implementation of the exponential function in IEEE
-// floating-point arithmetic, ACM TOMS 15, 1989), with 2048 entries so that a
-// cubic suffices: z = (n ln 2) / 2048 + s, |s| <= 1.7e-4,
-// exp(-z) = 2^(-n / 2048) (1 - s + s^2 / 2 - s^3 / 6) to 4e-17.  The index
-// comes from FP32, so the FP64 pipe sees 6 operations.
-constexpr int kExpN = 2048;
-struct ExpTable {
-  double v[kExpN];
-};
-struct DD {
-  double hi, lo;
-};
-constexpr DD dd_two_prod(double a, double b) {  // Dekker's product
-  const double p = a * b;
-  const double c1 = 134217729.0 * a, c2 = 134217729.0 * b;
-  const double ah = c1 - (c1 - a), bh = c2 - (c2 - b);
-  const double al = a - ah, bl = b - bh;
-  return {p, ((ah * bh - p) + ah * bl + al * bh) + al * bl};
-}
-constexpr DD dd_mul(DD a, DD b) {
-  const DD p = dd_two_prod(a.hi, b.hi);
-  const double l = p.lo + (a.hi * b.lo + a.lo * b.hi);
-  const double s = p.hi + l;
-  return {s, l - (s - p.hi)};
-}
-// ln 2 in three parts: the first with its last 20 bits zero, so that n times
-// it is exact for n < 2^16
-constexpr double kLn2Hi = 0x1.62e42fefp-1, kLn2Lo = 0x1.473de6af278edp-34;
-constexpr ExpTable make_exp_table() {
-  // c = 2^(-1/2048) = exp(-ln 2 / 2048) as a double-double Taylor sum
-  const DD x = {-0x1.62e42fefa39efp-1 / kExpN, -0x1.abc9e3b39803fp-56 / kExpN};
-  DD term = {1.0, 0.0}, c = {1.0, 0.0};
-  for (int k = 1; k <= 8; k++) {
-    term = dd_mul(term, x);
-    const DD inv = {1.0 / k, 0.0};
-    // term / k with one correction of the quotient
-    const DD q0 = dd_mul(term, inv);
-    const DD back = dd_mul(q0, DD{(double)k, 0.0});
-    const double fix = ((term.hi - back.hi) + (term.lo - back.lo)) / k;
-    const double qh = q0.hi + (q0.lo + fix);
-    term = DD{qh, (q0.lo + fix) - (qh - q0.hi)};
-    const double s = c.hi + term.hi;
-    const double err = (c.hi - s) + term.hi;
-    const double lo = err + (c.lo + term.lo);
-    const double s2 = s + lo;
-    c = DD{s2, lo - (s2 - s)};
-  }
-  ExpTable t = {};
-  DD v = {1.0, 0.0};
-  for (int i = 0; i < kExpN; i++) {
-    t.v[i] = v.hi;
-    v = dd_mul(v, c);
-  }
-  return t;
-}
-__device__ constexpr ExpTable g_exp_table = make_exp_table();
-
-__device__ __forceinline__ double exp_neg(double z) {
-  const float nf = fmaf(d2f_trunc(z), (float)(kExpN / 0.693147180559945309417), 12582912.0f);
-  const int n = (int)(__float_as_uint(nf) - 0x4B400000u);
-  const double nd = f2d(nf - 12582912.0f);
-  double s = fma(nd, -kLn2Hi / kExpN, z);
-  s = fma(nd, -kLn2Lo / kExpN, s);
-  const double p = fma(s, -1.0 / 6.0, 0.5);
-  const double t = fma(s * s, p, -s);
-  const double T = __ldg(&g_exp_table.v[n & (kExpN - 1)]);
-  const double b = __hiloint2double(__double2hiint(T) - ((n >> 11) << 20), __double2loint(T));
-  return fma(b, t, b);
-}
-
 // ---------------------------------------------------------------------------
 // Launch constants of the FP64 pair kernels
 // ---------------------------------------------------------------------------
@@ -330,6 +342,7 @@ struct Pair64 {
   double i_r, i_0;             // inner piece: i_r r + i_0.  Wendland: (i_r r + i_0) (1 + o_r r)^5
   double scale;                // FIX: of the gradient factor that is summed (cubic: -al / h^2)
   Fix64 hf, ihf, hb2f;         // h, 1/h, hb2
+  Fix64 l2e;                   // log2(e) / h^2
   double al;                   // normalisation of W
   double hb2, pic;             // viscosity: pic dot / ((d2 + hb2) (rho_i + rho_j))
   double r02;                  // r0^2
@@ -375,7 +388,8 @@ inline Pair64 pair64_consts(const sph_config_t &cfg, const sph_wcsph_t &wc) {
   c.hf = fix64(h);
   c.ihf = fix64(ih);
   c.hb2f = fix64(c.hb2);
-  c.scale = cfg.kernel == SPH_KERNEL_CUBIC ? -c.al * ih2 : 1.0;
+  c.l2e = fix64(1.44269504088896340736 * ih2);
+  c.scale = cfg.kernel == SPH_KERNEL_CUBIC ? -c.al * ih2 : (cfg.kernel == SPH_KERNEL_GAUSSIAN ? c.i_0 : 1.0);
   c.pic = -wc.alpha * wc.co * h;  // -2 alpha c_ij h with c_ij = co / 2
   c.r02 = wc.r0 * wc.r0;
   c.lj_free = cfg.h_fixed > 0.0 && wc.r0 < 1.5 * h * (1.0 - 1e-9);

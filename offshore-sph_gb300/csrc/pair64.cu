@@ -59,8 +59,8 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
     if constexpr (UH) {
       if constexpr (gauss) {
         if (!le_bits(d2, c.lim_lo) && (!le_bits(d2, c.lim_hi) || !near_exact(q.x - A.x, q.y - A.y, hij))) return;
-        const double e = exp_neg(d2 * (ih * ih));
-        coef = le_bits(d2, c.h2) ? 0.0 : c.i_0 * e;
+        const double e = FIX ? exp2_neg(geo.v, c.l2e) : exp_neg(d2 * (ih * ih));
+        coef = le_bits(d2, c.h2) ? 0.0 : (FIX ? e : c.i_0 * e);  // FIX: scaled in the sum
         if (c.xsph) w = c.al * e;
       } else {
         if (!le_bits(d2, c.lim)) return;  // W and its gradient are 0 at q >= 2
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(kPairBlock, G == 8 ? 4 : kPair64Blocks)
     for_neighbours<G, kCap, kPairBlock>(sten, P.cstart, act, lists, near, [&](unsigned int j) {
       pair64<KERNEL, UH, kFix>(s, q, c, pp, kFix ? fix[j] : longlong2(), P.r64a[j], P.r64b[j]);
     });
-    if (UH && kFix && KERNEL == SPH_KERNEL_CUBIC) {
+    if (UH && kFix && KERNEL != SPH_KERNEL_WENDLAND) {
       s.dd *= c.scale;
       s.ax *= c.scale;
       s.ay *= c.scale;
