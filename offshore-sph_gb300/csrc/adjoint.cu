@@ -38,6 +38,10 @@ namespace sph {
 // two-warp blocks: the kernels have few warps per SM, and small blocks spread
 // them evenly
 constexpr int kAdjBlock = 64;
+// resident blocks of the FP64 kernel: the registers' limit that measured
+// fastest (the 20K wall-load case: 9.73 ms at 6, 9.87 at 8, 9.29 at 10, 9.46
+// at 12)
+constexpr int kAdjBlocks = 10;
 
 struct AdjParams {
   double alpha, beta, co, r0, D, p1, p2, gamma, B, inv_rho0;
@@ -111,9 +115,10 @@ struct AdjReach {
 // operations per fluid pair, with the building blocks and launch constants of
 // the forward (pair64.cu).  Listing the pairs first keeps the lanes of a warp
 // together: evaluating each candidate as the walk met it ran 12.5 of 32 lanes
-// on average.  22K particles, one step: 297 us so, 100 us here (ncu).
+// on average.  22K particles, one step: 297 us so, 100 us with the pairs listed, 91
+// with the forward's integer arithmetic (ncu).
 template <int KERNEL, int G>
-__global__ void __launch_bounds__(kAdjBlock, 6) k_pair_adjoint(AdjPtrs P, AdjParams ap, Pair64 c) {
+__global__ void __launch_bounds__(kAdjBlock, kAdjBlocks) k_pair_adjoint(AdjPtrs P, AdjParams ap, Pair64 c) {
   constexpr int kCap = list_words<G>(ListCap<KERNEL>::value);
   constexpr bool gauss = KERNEL == SPH_KERNEL_GAUSSIAN;
   constexpr bool kFix = G < 8;  // integer differences, as in the forward
@@ -486,22 +491,35 @@ __global__ void k_adj_post(const int8_t *__restrict__ label, long long n, double
   drhob[i] = hdt * rhohb[i];
 }
 
-// sum of v[0 .. n) in a fixed order (one block): deterministic
-__global__ void k_sum_fixed(const double *__restrict__ v, long long n, double *out) {
-  __shared__ double red[1024];
-  double s = 0.0;
-  for (long long i = threadIdx.x; i < n; i += blockDim.x) s += v[i];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
+// Sum of v[0 .. n) in a fixed order (one block): each thread four partial sums
+// over its stride, so that four loads are in flight, then shuffles.
+constexpr int kSumThreads = 1024;
+__global__ void __launch_bounds__(kSumThreads) k_sum_fixed(const double *__restrict__ v, long long n, double *out) {
+  step_kernel_entry();
+  __shared__ double red[32];
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  for (long long i = threadIdx.x; i < n; i += 4 * kSumThreads) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const long long j = i + q * kSumThreads;
+      if (j < n) s[q] += v[j];
+    }
   }
-  if (threadIdx.x == 0) *out = red[0];
+  double t = (s[0] + s[1]) + (s[2] + s[3]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    t = red[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (threadIdx.x == 0) *out = t;
+  }
 }
 
 void launch_sum_fixed(const double *v, long long n, double *out, cudaStream_t st) {
-  k_sum_fixed<<<1, 1024, 0, st>>>(v, n, out);
+  launch_pdl(k_sum_fixed, dim3(1), dim3(kSumThreads), 0, st, v, n, out);
 }
 
 void launch_adjoint_step(const StepArgs &s, const StepArgs &h, const WsPtrs &w, const sph_config_t &cfg,

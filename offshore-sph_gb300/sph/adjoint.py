@@ -13,8 +13,9 @@ step's evaluation.  The reference has no such diagnostic; it is the
 horizontal force the fluid exerts on that wall.
 
 The forward pass runs the device step (``sph_run_wall_load``) and keeps a
-checkpoint of the state every ``checkpoint`` steps.  The backward pass
-replays each segment from its checkpoint, keeping a copy of the workspace
+checkpoint of the state every ``checkpoint`` steps, and for the last segment
+also a copy of the workspace after every step.  The backward pass
+replays each earlier segment from its checkpoint, keeping a copy of the workspace
 after every replayed step (its neighbour build and FP64 records), and walks
 the segment in reverse with the hand-written adjoint step
 (``sph_adjoint_step``: the vector-Jacobian product of the fused pair
@@ -134,12 +135,21 @@ class WallLoadLoss(torch.autograd.Function):
         hist = torch.empty(case.nsteps, dtype=torch.float64, device=pos.device)
         ckpts = []
         K = case.checkpoint
+        last = []
         for s0 in range(0, case.nsteps, K):
             ckpts.append(case.snapshot(dp))
-            case._run(dp, wc, min(K, case.nsteps - s0), hist[s0:])
+            if s0 + K < case.nsteps or not any(ctx.needs_input_grad):
+                case._run(dp, wc, min(K, case.nsteps - s0), hist[s0:])
+                continue
+            # the last segment step by step (the same state, bit for bit), its
+            # builds kept: the backward starts on them instead of replaying
+            for s in range(s0, case.nsteps):
+                case._run(dp, wc, 1, hist[s:])
+                last.append(case.ws.buf.clone())
         case.ws.check()
         ctx.case = case
         ctx.ckpts = ckpts
+        ctx.last = last
         ctx.alpha = alpha.item()
         return case.dt * hist.sum()
 
@@ -163,18 +173,19 @@ class WallLoadLoss(torch.autograd.Function):
         side.wait_stream(main)
         # Two sets of K workspace copies: while the adjoint walks segment seg
         # on the main stream (reading set seg % 2), the side stream replays
-        # segment seg - 1 into the other set.  walked[seg]: the main stream
-        # has finished reading segment seg's set.
-        sets = [[torch.empty_like(case.ws.buf) for _ in range(K)] for _ in range(min(2, nseg))]
+        # segment seg - 1 into the other set.  The last segment's copies come
+        # from the forward.  walked[seg]: the main stream has finished reading
+        # segment seg's set.
+        sets = [[torch.empty_like(case.ws.buf) for _ in range(K)] for _ in range(min(2, nseg - 1))]
         walked = [None] * nseg
 
         def replay(seg):
             # after each step the workspace holds that step's neighbour build
             # and FP64 records, which its adjoint reuses; the same step as the
             # forward's without the wall-load output (the state is identical)
-            bufs = sets[seg % 2]
+            bufs = sets[seg % len(sets)]
             with torch.cuda.stream(side):
-                if seg + 2 < nseg:
+                if seg + 2 < nseg - 1:
                     side.wait_event(walked[seg + 2])
                 dp._buf.copy_(case.base._buf)
                 case.restore(dp, ctx.ckpts[seg])
@@ -183,12 +194,13 @@ class WallLoadLoss(torch.autograd.Function):
                     bufs[s].copy_(case.ws.buf)
                 return side.record_event()
 
-        ready = replay(nseg - 1)
+        ready = None
         for seg in reversed(range(nseg)):
-            main.wait_event(ready)
+            if ready is not None:
+                main.wait_event(ready)
             if seg > 0:
                 ready = replay(seg - 1)
-            bufs = sets[seg % 2]
+            bufs = ctx.last if seg == nseg - 1 else sets[seg % len(sets)]
             for s in reversed(range(min(K, case.nsteps - seg * K))):
                 ws_s = L.Workspace(ptr=bufs[s].data_ptr(), bytes=w0.bytes, n_cap=w0.n_cap, max_cells=w0.max_cells)
                 L.check(lib.sph_adjoint_step(core._P(case.base), core._P(half), C.byref(wc), C.byref(case.cfg_adj),
