@@ -150,7 +150,7 @@ __global__ void k_selftest_staging(const float4 *src, unsigned int *result) {
 // nearly consecutive addresses instead of gathering through the caller's
 // order.  The in-cell order still ranks by the caller's index (WsPtrs::orig),
 // so the results are those of stepping on the caller's arrays, bit for bit.
-// At the end the copy is scattered back.
+// At the end the copy returns to the caller's order.
 // ---------------------------------------------------------------------------
 StepArgs shadow_args(const WsPtrs &w, long long n) {
   StepArgs b;
@@ -171,30 +171,57 @@ __device__ __forceinline__ double *const *state_fields(const StepArgs &a, double
   return f;
 }
 
+// Fields of the copy.  m is not changed by a run, so it does not come back.
+// p is written by the records of the first step before anything reads it, and
+// x0 .. rho0 by the first predictor of the integrator that has them (PEC, on
+// the fluid), so these do not go in.
+constexpr int kFieldM = 0, kFieldP = 2, kFieldX0 = 14;
+
+// Both copies are bound by memory traffic on the side in the caller's order,
+// 8 of a 32-byte sector at a time.  That is the loads for both: the way back
+// goes by the inverse order, which k_correct writes, because stores of 8 bytes
+// to scattered sectors cost more than such loads.  1.03M particles in the
+// order of a lattice: in 77 -> 44 us, back 145 (by stores, with m and every
+// field) -> 70 us.
 // copy slot s = caller particle perm[s]; orig[s] remembers it
-__global__ void k_shadow_gather(StepArgs src, StepArgs dst, const int *__restrict__ perm, int *__restrict__ orig) {
+__global__ void __launch_bounds__(kBlock) k_shadow_gather(StepArgs src, StepArgs dst, const int *__restrict__ perm,
+                                                          int *__restrict__ orig) {
+  step_kernel_entry();
   const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= src.n) return;
   const int i = perm[s];
   orig[s] = i;
-  double *fs[kStateFields], *fd[kStateFields];
+  double *fs[kStateFields], *fd[kStateFields], v[kFieldX0];
   state_fields(src, fs);
   state_fields(dst, fd);
 #pragma unroll
-  for (int q = 0; q < kStateFields; q++) fd[q][s] = fs[q][i];
+  for (int q = 0; q < kFieldX0; q++)  // all loads ahead of the stores
+    if (q != kFieldP) v[q] = fs[q][i];
+#pragma unroll
+  for (int q = 0; q < kFieldX0; q++)
+    if (q != kFieldP) fd[q][s] = v[q];
   const_cast<int8_t *>(dst.label)[s] = src.label[i];
 }
 
-// the copy back to the caller's order (labels do not change)
-__global__ void k_shadow_scatter(StepArgs src, StepArgs dst, const int *__restrict__ orig) {
-  const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= src.n) return;
-  const int i = orig[s];
-  double *fs[kStateFields], *fd[kStateFields];
+// the copy back to the caller's order (labels do not change): caller
+// particle i is the copy's inv[i]
+template <bool PEC>
+__global__ void __launch_bounds__(kBlock) k_shadow_return(StepArgs src, StepArgs dst, const int *__restrict__ inv) {
+  step_kernel_entry();
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= src.n) return;
+  const int s = inv[i];
+  constexpr int fields = PEC ? kStateFields : kFieldX0;
+  double *fs[kStateFields], *fd[kStateFields], v[fields];
   state_fields(src, fs);
   state_fields(dst, fd);
+  const bool fl = is_fluid(dst.label[i]);
 #pragma unroll
-  for (int q = 0; q < kStateFields; q++) fd[q][i] = fs[q][s];
+  for (int q = 0; q < fields; q++)
+    if (q != kFieldM) v[q] = fs[q][s];
+#pragma unroll
+  for (int q = 0; q < fields; q++)
+    if (q != kFieldM && (q < kFieldX0 || fl)) fd[q][i] = v[q];
 }
 
 __global__ void k_fill_dt(double *dt_hist, long long nsteps, double dt) {
@@ -475,7 +502,7 @@ int sph_correct(sph_particles_t *pa, const sph_config_t *cfg, const double *dt, 
 }
 
 // Runs of at least this many steps step on the sorted copy of the state
-// (when the workspace has room for it): the gather and scatter cost about a
+// (when the workspace has room for it): the copies in and back cost about a
 // step's worth of memory traffic.
 constexpr int64_t kShadowMinSteps = 4;
 
@@ -488,14 +515,23 @@ static StepArgs run_state(const StepArgs &a, WsPtrs &wp, const sph_config_t &cfg
   launch_bounds(a, wp, cfg, wc, kStageNone, false, nullptr, nullptr, st);
   launch_build(a, wp, cfg, wc, st);
   const StepArgs b = shadow_args(wp, a.n);
-  k_shadow_gather<<<nblocks(a.n), kBlock, 0, st>>>(a, b, wp.perm, wp.shadow_orig);
+  launch_pdl(k_shadow_gather, dim3(nblocks(a.n)), dim3(kBlock), 0, st, a, b, wp.perm, wp.shadow_orig);
   wp.orig = wp.shadow_orig;
   return b;
 }
 
-static void run_finish(const StepArgs &a, const StepArgs &b, const WsPtrs &wp, cudaStream_t st) {
-  if (!wp.orig) return;
-  k_shadow_scatter<<<nblocks(a.n), kBlock, 0, st>>>(b, a, wp.orig);
+// End of a run: the last step's corrector, and the copy back to the caller's
+// arrays a.  The inverse order is in the arrival ranks, which no build reads
+// any more.
+static void run_finish(const StepArgs &a, const StepArgs &b, const WsPtrs &wp, const sph_config_t &cfg,
+                       const double *dt, cudaStream_t st) {
+  int *inv = wp.orig ? (int *)wp.crank : nullptr;
+  launch_correct(b, cfg, dt, cfg.dt_fixed, st, wp.orig, inv);
+  if (!inv) return;
+  if (cfg.integrator == SPH_INTEGRATOR_PEC)
+    launch_pdl(k_shadow_return<true>, dim3(nblocks(a.n)), dim3(kBlock), 0, st, b, a, inv);
+  else
+    launch_pdl(k_shadow_return<false>, dim3(nblocks(a.n)), dim3(kBlock), 0, st, b, a, inv);
 }
 
 // Whether step s of a run of nsteps writes p, c and the fluid h back to the
@@ -538,8 +574,7 @@ int sph_run(sph_particles_t *pa, const sph_wcsph_t *w, const sph_config_t *cfg, 
     compute_body(a, wp, *w, *cfg, fixed ? nullptr : nxt, hist_next, st, nullptr,
                  step_writes_state(*w, *cfg, s, nsteps));
   }
-  launch_correct(a, *cfg, ring + 3 * ((nsteps - 1) & 1), cfg->dt_fixed, st);
-  run_finish(caller, a, wp, st);
+  run_finish(caller, a, wp, *cfg, ring + 3 * ((nsteps - 1) & 1), st);
   return check_launch();
 }
 
@@ -644,8 +679,7 @@ int sph_run_profiled(sph_particles_t *pa, const sph_wcsph_t *w, const sph_config
     launch_pair(a, wp, *cfg, *w, fixed ? nullptr : nxt, nullptr, st, nullptr, step_writes_state(*w, *cfg, s, nsteps));
     lap(SPH_STAGE_PAIR);
   }
-  launch_correct(a, *cfg, ring + 3 * ((nsteps - 1) & 1), cfg->dt_fixed, st);
-  run_finish(caller, a, wp, st);  // the copy back counts with the last corrector
+  run_finish(caller, a, wp, *cfg, ring + 3 * ((nsteps - 1) & 1), st);  // the copy back counts with the last corrector
   lap(SPH_STAGE_CORRECT);
   int rc = (ok && check_launch() == SPH_OK && cudaEventSynchronize(mark.back()) == cudaSuccess) ? SPH_OK : SPH_ERR_CUDA;
   for (size_t k = 1; rc == SPH_OK && k < mark.size(); k++) {

@@ -99,10 +99,15 @@ __device__ __forceinline__ void correct_one(const StepArgs &a, long long i, cons
   (void)hdt;
 }
 
-__global__ void __launch_bounds__(kBlock) k_correct(StepArgs a, IntParams ip) {
+// inv (when given): the inverse of the order orig, for the copy back of a run
+// on the sorted copy
+__global__ void __launch_bounds__(kBlock) k_correct(StepArgs a, IntParams ip, const int *__restrict__ orig,
+                                                    int *__restrict__ inv) {
   step_kernel_entry();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n || !is_fluid(a.label[i])) return;
+  if (i >= a.n) return;
+  if (inv) inv[orig[i]] = (int)i;
+  if (!is_fluid(a.label[i])) return;
   correct_one(a, i, ip);
 }
 
@@ -125,8 +130,8 @@ void launch_predict(const StepArgs &a, const sph_config_t &cfg, const double *dt
 }
 
 void launch_correct(const StepArgs &a, const sph_config_t &cfg, const double *dt, double dt_fixed,
-                    cudaStream_t st) {
-  launch_pdl(k_correct, dim3(nblocks(a.n)), dim3(kBlock), 0, st, a, int_params(cfg, dt, dt_fixed));
+                    cudaStream_t st, const int *orig, int *inv) {
+  launch_pdl(k_correct, dim3(nblocks(a.n)), dim3(kBlock), 0, st, a, int_params(cfg, dt, dt_fixed), orig, inv);
 }
 
 // TimeStep.compute over fluid (src/Equations/TimeStep.py:7-91)

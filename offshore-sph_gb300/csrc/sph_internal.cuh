@@ -944,7 +944,7 @@ void launch_nn_count(const StepArgs &a, const WsPtrs &w, int64_t *counts, const 
 void launch_predict(const StepArgs &a, const sph_config_t &cfg, const double *dt, double dt_fixed,
                     cudaStream_t st);
 void launch_correct(const StepArgs &a, const sph_config_t &cfg, const double *dt, double dt_fixed,
-                    cudaStream_t st);
+                    cudaStream_t st, const int *orig = nullptr, int *inv = nullptr);
 void launch_timestep(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, double *dt3, double *dt_hist,
                      cudaStream_t st);
 void launch_initialize(const StepArgs &a, const sph_wcsph_t &wc, const sph_config_t &cfg, cudaStream_t st);
