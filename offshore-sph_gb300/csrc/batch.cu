@@ -14,7 +14,7 @@ namespace sph {
 
 void launch_bt_bounds(const StepArgs &a, const WsPtrs &w, const BatchPtrs &B, const sph_config_t &cfg, int stage,
                       int prev, int cur, cudaStream_t st);
-void launch_bt_build(const StepArgs &a, const WsPtrs &w, const BatchPtrs &B, cudaStream_t st);
+void launch_bt_build(const StepArgs &a, const WsPtrs &w, const BatchPtrs &B, bool write_state, cudaStream_t st);
 void launch_bt_pair(const StepArgs &a, const WsPtrs &w, const BatchPtrs &B, int kernel, bool xsph, int tile_blocks,
                     cudaStream_t st);
 void launch_bt_timestep(const StepArgs &a, const WsPtrs &w, const BatchPtrs &B, int slot, double *dt_hist,
@@ -142,7 +142,6 @@ int sph_batch_setup(const sph_workspace_t *ws, int64_t n_inst, const int64_t *of
     rp.Pb_f = (float)wc.Pb;
     rp.h_fixed_on = 1;
     rp.Pb_on = wc.Pb != 0.0 ? 1 : 0;
-    rp.write_state = 1;
     rp.from_state = 0;
     rp.reduce_h = 1;
     PairParams &pp = p.pp;
@@ -207,7 +206,9 @@ int sph_batch_run(sph_particles_t *pa, const sph_config_t *cfg, const sph_worksp
   for (int64_t s = 0; s < nsteps; s++) {
     const int prev = (int)((s + 1) & 1), cur = (int)(s & 1), nxt = (int)((s + 1) & 1);
     launch_bt_bounds(a, wp, B, *cfg, s == 0 ? kStagePredict : kStageCorrectPredict, prev, cur, st);
-    launch_bt_build(a, wp, B, st);  // with the records
+    // with the records; p, c and h go to the caller's arrays in the first
+    // step (the bounds pass reads h) and the last, as in sph_run
+    launch_bt_build(a, wp, B, s == 0 || s + 1 == nsteps, st);
     launch_bt_pair(a, wp, B, cfg->kernel, false, tile_blocks, st);
     launch_bt_dt_finish(wp, B, nxt, (dt_hist && s + 1 < nsteps) ? dt_hist + 3 * ni * (s + 1) : nullptr, st);
   }

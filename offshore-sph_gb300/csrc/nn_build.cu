@@ -746,8 +746,8 @@ enum { kHState = 0, kHFixed = 1, kHCompute = 2 };
 template <int HSRC, bool PB>
 __device__ __forceinline__ void record_mixed_t(const StepArgs &a, long long k, int i, const RecParams &rp,
                                                float4 *__restrict__ rec0, float4 *__restrict__ rec1,
-                                               float4 *__restrict__ rec2, unsigned long long &eh,
-                                               unsigned int &nf) {
+                                               float4 *__restrict__ rec2, bool write_state,
+                                               unsigned long long &eh, unsigned int &nf) {
   const int8_t lab = a.label[i];
   const bool fl = is_fluid(lab);
   const double m = a.m[i], rho = a.rho[i];
@@ -790,7 +790,7 @@ __device__ __forceinline__ void record_mixed_t(const StepArgs &a, long long k, i
   split_df(a.vx[i], vxh, vxl);
   split_df(a.vy[i], vyh, vyl);
   rec2[k] = make_float4(vxh, vyh, vxl, vyl);
-  if (rp.write_state) {
+  if (write_state) {
     a.p[i] = pd;
     a.c[i] = rp.co;
     if (fl) a.h[i] = hd;
@@ -807,14 +807,14 @@ __device__ __forceinline__ void record_mixed(const StepArgs &a, long long k, int
                                              float4 *__restrict__ rec0, float4 *__restrict__ rec1,
                                              float4 *__restrict__ rec2, unsigned long long &eh, unsigned int &nf) {
   if (rp.from_state) {
-    if (rp.Pb_on) record_mixed_t<kHState, true>(a, k, i, rp, rec0, rec1, rec2, eh, nf);
-    else record_mixed_t<kHState, false>(a, k, i, rp, rec0, rec1, rec2, eh, nf);
+    if (rp.Pb_on) record_mixed_t<kHState, true>(a, k, i, rp, rec0, rec1, rec2, rp.write_state, eh, nf);
+    else record_mixed_t<kHState, false>(a, k, i, rp, rec0, rec1, rec2, rp.write_state, eh, nf);
   } else if (rp.h_fixed_on) {
-    if (rp.Pb_on) record_mixed_t<kHFixed, true>(a, k, i, rp, rec0, rec1, rec2, eh, nf);
-    else record_mixed_t<kHFixed, false>(a, k, i, rp, rec0, rec1, rec2, eh, nf);
+    if (rp.Pb_on) record_mixed_t<kHFixed, true>(a, k, i, rp, rec0, rec1, rec2, rp.write_state, eh, nf);
+    else record_mixed_t<kHFixed, false>(a, k, i, rp, rec0, rec1, rec2, rp.write_state, eh, nf);
   } else {
-    if (rp.Pb_on) record_mixed_t<kHCompute, true>(a, k, i, rp, rec0, rec1, rec2, eh, nf);
-    else record_mixed_t<kHCompute, false>(a, k, i, rp, rec0, rec1, rec2, eh, nf);
+    if (rp.Pb_on) record_mixed_t<kHCompute, true>(a, k, i, rp, rec0, rec1, rec2, rp.write_state, eh, nf);
+    else record_mixed_t<kHCompute, false>(a, k, i, rp, rec0, rec1, rec2, rp.write_state, eh, nf);
   }
 }
 
@@ -973,7 +973,7 @@ __global__ void __launch_bounds__(kBlock) k_cellsort(const int *__restrict__ per
     const unsigned int slot = s + rank;
     perm[slot] = v;
     meta[slot] = refcell[v];
-    if (REC == kRecMixed) record_mixed_t<HSRC, PB>(a, slot, v, rp, rec0, rec1, rec2, eh, nf);
+    if (REC == kRecMixed) record_mixed_t<HSRC, PB>(a, slot, v, rp, rec0, rec1, rec2, rp.write_state, eh, nf);
     if (REC == kRecFp64) record_fp64(a, slot, v, rp, gp->fix_s, rec0, rec1, r64a, r64b, eh, nf);
   }
   if (REC != kRecNone && rp.reduce_h) reduce_h_block(eh, nf, red, redn, ctrl);
@@ -1209,7 +1209,7 @@ __global__ void __launch_bounds__(kBlock) k_bt_cellsort(const int *__restrict__ 
                                                         DevCtrl *ctrl, int *__restrict__ perm,
                                                         int2 *__restrict__ meta, StepArgs a,
                                                         float4 *__restrict__ rec0, float4 *__restrict__ rec1,
-                                                        float4 *__restrict__ rec2) {
+                                                        float4 *__restrict__ rec2, bool write_state) {
   step_kernel_entry();
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long eh = kEncMinId;
@@ -1237,7 +1237,9 @@ __global__ void __launch_bounds__(kBlock) k_bt_cellsort(const int *__restrict__ 
       tcell = c0 + (tl << ts2);
       tsize = 1u << ts2;
     }
-    record_mixed(a, slot, v, B.ip[b].rp, rec0, rec1, rec2, eh, nf);
+    const RecParams &rp = B.ip[b].rp;  // a fixed h, and the EOS's p
+    if (rp.Pb_on) record_mixed_t<kHFixed, true>(a, slot, v, rp, rec0, rec1, rec2, write_state, eh, nf);
+    else record_mixed_t<kHFixed, false>(a, slot, v, rp, rec0, rec1, rec2, write_state, eh, nf);
   }
   // A tile with fluid is listed once, by the first warp that stamps it with
   // this build's number: the small tanks hold many tiles of wall particles
@@ -1281,7 +1283,7 @@ void launch_bt_bounds(const StepArgs &a, const WsPtrs &w, const BatchPtrs &B, co
 }
 
 // the batched build with the records fused into the in-cell sort
-void launch_bt_build(const StepArgs &a, const WsPtrs &w, const BatchPtrs &B, cudaStream_t st) {
+void launch_bt_build(const StepArgs &a, const WsPtrs &w, const BatchPtrs &B, bool write_state, cudaStream_t st) {
   const unsigned nb = nblocks(a.n);
   launch_pdl(k_bt_grid, dim3(1), dim3(256), 0, st, B, w.ctrl);
   launch_pdl(k_bt_keys, dim3(nb), dim3(kBlock), 0, st, a.x, a.y, a.n, B, w.ctrl, w.keys, w.refcell, w.crank,
@@ -1291,7 +1293,7 @@ void launch_bt_build(const StepArgs &a, const WsPtrs &w, const BatchPtrs &B, cud
   launch_pdl(k_scatter_rank, dim3(nb), dim3(kBlock), 0, st, w.keys, w.crank, a.n, w.counts, w.cstart, w.perm_tmp,
              w.keys_sorted, w.scan_part, w.n_parts);
   launch_pdl(k_bt_cellsort, dim3(nb), dim3(kBlock), 0, st, w.perm_tmp, w.keys_sorted, w.cstart, w.refcell, a.n, B,
-             w.ctrl, w.perm, w.meta, a, w.rec0, w.rec1, w.rec2);
+             w.ctrl, w.perm, w.meta, a, w.rec0, w.rec1, w.rec2, write_state);
 }
 
 }  // namespace sph

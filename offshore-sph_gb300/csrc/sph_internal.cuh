@@ -342,16 +342,12 @@ struct BatchPtrs {
 // the batched form; lanes of one instance are contiguous (instance-major
 // order), b < 0 for lanes without a particle.  commit(b, value) applies the
 // atomic to instance b's slot.  Every lane of the warp must call.
+__device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v);
 template <class F>
 __device__ __forceinline__ void seg_min_u64(unsigned long long v, int b, F &&commit) {
   const int b0 = __shfl_sync(0xffffffffu, b, 0);
   if (__all_sync(0xffffffffu, b == b0)) {
-    unsigned long long m = v;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long t = __shfl_xor_sync(0xffffffffu, m, o);
-      m = t < m ? t : m;
-    }
+    const unsigned long long m = warp_min_u64(v);
     if ((threadIdx.x & 31) == 0 && b0 >= 0 && m != kEncMinId) commit(b0, m);
   } else if (b >= 0 && v != kEncMinId) {
     commit(b, v);
