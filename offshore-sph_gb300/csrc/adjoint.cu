@@ -116,7 +116,7 @@ struct AdjReach {
 // the forward (pair64.cu).  Listing the pairs first keeps the lanes of a warp
 // together: evaluating each candidate as the walk met it ran 12.5 of 32 lanes
 // on average.  22K particles, one step: 297 us so, 100 us with the pairs listed, 91
-// with the forward's integer arithmetic (ncu).
+// with the forward's integer arithmetic, 82 with 10 blocks per SM (ncu).
 template <int KERNEL, int G>
 __global__ void __launch_bounds__(kAdjBlock, kAdjBlocks) k_pair_adjoint(AdjPtrs P, AdjParams ap, Pair64 c) {
   constexpr int kCap = list_words<G>(ListCap<KERNEL>::value);

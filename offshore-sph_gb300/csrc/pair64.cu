@@ -18,10 +18,10 @@
 //     they contribute nothing).
 // A pair of the cubic spline so takes 13 FP64 operations instead of about 90.
 // 1M-fluid dam break, pair stage: 3.67 ms at 90, 1.27 ms at 31 (Halley steps and
-// launch-constant gradient polynomials in FP64), 0.76 ms now; the FP64 pipe
-// is busy 70% of it and 27% of the issue slots are used.  20 steps of 3200
+// launch-constant gradient polynomials in FP64), 0.75 ms now; the FP64 pipe
+// is busy 65% of it and 42% of the issue slots are used.  20 steps of 3200
 // fluid particles, where latency decides (several lanes per query): 2.40 ms,
-// 0.71 and 0.69.
+// 0.71 and 0.66.
 #include <type_traits>
 
 #include "fp64_ops.cuh"

@@ -225,7 +225,8 @@ __device__ __forceinline__ void group_sum(T &v) {
 
 // Lanes per query of the FP64 kernels for n particles.  Sharing a query costs
 // about a quarter more issue time (short groups, the final sums; dam break of
-// 1M fluid particles: 1.27 ms with G = 1, 1.57 ms with G = 4) and divides the
+// 1M fluid particles: 1.27 ms with G = 1, 1.57 ms with G = 4, measured like the
+// figures below before the arithmetic moved to the integer pipe) and divides the
 // length of a thread's chain of dependent FP64 operations.  So G = 1 where the
 // threads fill most of one wave of blocks (54K particles, Wendland: 784 us for
 // 4 steps against 817 with G = 4) or several; G = 4 where the last wave would
