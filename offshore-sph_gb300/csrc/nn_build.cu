@@ -212,12 +212,13 @@ __device__ void grid_from_bounds(DevCtrl *ctrl, DevGrid *g, const GridParams &gp
 // Persistent grid-stride blocks (a few per SM), so that the block
 // reductions end in few atomics on the shared bound slots.  The last block
 // to finish sets the grid of the next build from the reduced bounds.
-#ifndef SPH_BOUNDS_BLOCKS
-#define SPH_BOUNDS_BLOCKS 4
-#endif
-constexpr int kBoundsBlocks = SPH_BOUNDS_BLOCKS;  // resident blocks per SM
+// bounds_blocks: resident blocks per SM, limited by registers.  Without
+// integrator work 5 fit (an evaluation of 1M particles 257.4 us with 4, 256.7 with 5,
+// 260.1 with 6, where registers spill); with it, 4 (20 steps of 1.03M: 4914 us,
+// 5051 with 5, 5319 with 6).
+constexpr int bounds_blocks(int stage) { return stage == kStageNone ? 5 : 4; }
 template <int INTEG, int STAGE, bool DAMPED, bool XSPH>
-__global__ void __launch_bounds__(kBlock, kBoundsBlocks) k_bounds(StepArgs a, DevCtrl *ctrl, BoundsParams bp,
+__global__ void __launch_bounds__(kBlock, bounds_blocks(STAGE)) k_bounds(StepArgs a, DevCtrl *ctrl, BoundsParams bp,
                                                                   DevGrid *g, GridParams gp) {
   step_kernel_entry();
   __shared__ unsigned long long red[kBlock / 32][6];
@@ -333,8 +334,8 @@ void launch_bounds(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, 
   bp.strict = cfg.pec_strict;
   GridParams gp = grid_params(w, cfg, wc);
   gp.n = a.n;
-  const unsigned nb = persist_blocks(a.n, kBoundsBlocks);
   front_dispatch(bp, [&]<int I, int S, bool D, bool X>() {
+    const unsigned nb = persist_blocks(a.n, bounds_blocks(S));
     launch_pdl(k_bounds<I, S, D, X>, dim3(nb), dim3(kBlock), 0, st, a, w.ctrl, bp, w.grid, gp);
   });
 }
