@@ -50,3 +50,34 @@ def test_gradients_at_each_lane_count(ny, kernel):
             assert _rel(g, w) <= 1e-10
     for m, g in zip(mixed, got):
         assert _rel(m, g) <= 2e-6
+
+
+@pytest.mark.parametrize("checkpoint", [1, 2, 5])
+def test_last_segment_kept_from_the_forward(checkpoint):
+    """The last segment's builds come from the forward: a second backward
+    through the same graph, with another forward in between, gives the same
+    gradients, and so does every split into segments (a last one of one step
+    included), bit for bit."""
+    from sph import adjoint
+
+    def loss_and_leaves(case, alpha):
+        a = torch.tensor(alpha, dtype=torch.float64, device="cuda", requires_grad=True)
+        p, v = case.positions().requires_grad_(True), case.velocities().requires_grad_(True)
+        return adjoint.WallLoadLoss.apply(a, p, v, case), (a, p, v)
+
+    def case_of(k):
+        case = _case(37, 0, "fp64")
+        case.nsteps, case.checkpoint = 5, k
+        return case
+    case = case_of(checkpoint)
+    loss, leaves = loss_and_leaves(case, 0.01)
+    first = torch.autograd.grad(loss, leaves, retain_graph=True)
+    loss_and_leaves(case, 0.02)
+    second = torch.autograd.grad(loss, leaves)
+    whole = case_of(5)
+    want_loss, want_leaves = loss_and_leaves(whole, 0.01)
+    want = torch.autograd.grad(want_loss, want_leaves)
+    assert torch.equal(loss, want_loss)
+    for f, s, w in zip(first, second, want):
+        assert torch.equal(f, s) and torch.equal(f, w)
+        assert f.abs().max() > 0
