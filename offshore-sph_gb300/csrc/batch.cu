@@ -60,7 +60,6 @@ static BatchPtrs batch_ptrs(const sph_workspace_t *ws, int n_inst) {
   B.inst = (int *)(b + L.inst);
   B.tiles = (int2 *)(b + L.tiles);
   B.tiles_cap = (unsigned int)(ws->max_cells + n_inst);
-  B.stamp = (unsigned int *)ws_ptrs(ws).tiles_h;  // the single-scene build's list, unused here
   B.scan = (DevGrid *)(b + L.scan);
   B.n_inst = n_inst;
   return B;
@@ -172,8 +171,6 @@ int sph_batch_setup(const sph_workspace_t *ws, int64_t n_inst, const int64_t *of
   cudaStream_t st = (cudaStream_t)stream;
   const BatchPtrs B = batch_ptrs(ws, (int)n_inst);
   if (init_workspace(ws_ptrs(ws), st) != cudaSuccess) return SPH_ERR_CUDA;
-  if (cudaMemsetAsync(B.stamp, 0, (size_t)(ws->max_cells + 1) * sizeof(unsigned int), st) != cudaSuccess)
-    return SPH_ERR_CUDA;
   if (cudaMemcpyAsync(B.ip, ip.data(), ip.size() * sizeof(InstParams), cudaMemcpyHostToDevice, st) != cudaSuccess)
     return SPH_ERR_CUDA;
   k_bt_inst<<<nblocks(N), kBlock, 0, st>>>(B, N);

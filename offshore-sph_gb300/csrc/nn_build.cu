@@ -1161,31 +1161,41 @@ __global__ void k_bt_grid(BatchPtrs B, DevCtrl *ctrl) {
     B.scan->ncells = total - 1;  // the scan kernels cover ids 0 .. run - 1
     ctrl->tl_count = 0;
     ctrl->tl_back = 0;
-    ctrl->build_epoch++;
   }
 }
 
 // k_keys over every instance: cell ids offset by the instance's first cell;
-// arrival ranks and scan-tile totals as in k_keys.
+// arrival ranks and scan-tile totals as in k_keys.  A fluid particle marks its
+// tile (the bit of the tile's first cell): only the tiles with fluid are
+// listed.  The bits return to zero in k_bt_cellsort, as those of the
+// single-scene build do, so nothing of a build is left for the next one on the
+// same workspace, whichever form it has.
 __global__ void __launch_bounds__(kBlock) k_bt_keys(const double *__restrict__ x, const double *__restrict__ y,
                                                     long long n, BatchPtrs B, DevCtrl *ctrl, int *__restrict__ keys,
                                                     int2 *__restrict__ refcell, unsigned int *__restrict__ crank,
                                                     unsigned int *__restrict__ counts,
-                                                    unsigned int *__restrict__ part) {
+                                                    unsigned int *__restrict__ part,
+                                                    const int8_t *__restrict__ label,
+                                                    unsigned int *__restrict__ tflag) {
   step_kernel_entry();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const bool act = i < n;
   bool alias = false, overflow = false;
-  int key = -1 - lane;
+  int key = -1 - lane, tcell = -1;
   if (act) {
-    const int b = B.inst[i];
+    const int b = B.inst[i], c0 = B.coff[b];
+    const DevGrid &g = B.grids[b];
     int2 ref;
-    key = B.coff[b] + cell_key(B.grids[b], x[i], y[i], ref, alias, overflow);
+    const int lk = cell_key(g, x[i], y[i], ref, alias, overflow);
+    key = c0 + lk;
+    if (lk < g.ncells && is_fluid(label[i])) tcell = c0 + ((lk >> (2 * g.ts)) << (2 * g.ts));
     refcell[i] = ref;
     keys[i] = key;
     if (alias) atomicAdd(&B.sl[b].alias_count, 1u);
   }
+  const unsigned int fpeers = __match_any_sync(0xffffffffu, tcell);
+  if (tcell >= 0 && lane == __ffs(fpeers) - 1) atomicOr(&tflag[tcell >> 5], 1u << (tcell & 31));
   const unsigned int below = (1u << lane) - 1u;
   const unsigned int peers = __match_any_sync(0xffffffffu, key);
   const int leader = __ffs(peers) - 1;
@@ -1210,15 +1220,14 @@ __global__ void __launch_bounds__(kBlock) k_bt_cellsort(const int *__restrict__ 
                                                         DevCtrl *ctrl, int *__restrict__ perm,
                                                         int2 *__restrict__ meta, StepArgs a,
                                                         float4 *__restrict__ rec0, float4 *__restrict__ rec1,
-                                                        float4 *__restrict__ rec2, bool write_state) {
+                                                        float4 *__restrict__ rec2, bool write_state,
+                                                        unsigned int *__restrict__ tflag) {
   step_kernel_entry();
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long eh = kEncMinId;
   unsigned int nf = 0;
-  int b = -1, tl = -1;
+  int b = -1;
   const int lane = threadIdx.x & 31;
-  int tcell = -1 - lane;  // the first cell of a fluid particle's tile; other lanes match no other
-  unsigned int tsize = 0;
   const bool act = k < n;
   const int key = act ? keys_sorted[k] : -1 - lane;  // inactive lanes match no other lane
   const int v = act ? perm_tmp[k] : 0;
@@ -1232,27 +1241,21 @@ __global__ void __launch_bounds__(kBlock) k_bt_cellsort(const int *__restrict__ 
     b = B.inst[v];
     const int c0 = B.coff[b], lk = key - c0;
     const DevGrid &g = B.grids[b];
-    const int ts2 = 2 * g.ts;
-    if (lk < g.ncells && is_fluid(a.label[v])) {
-      tl = lk >> ts2;
-      tcell = c0 + (tl << ts2);
-      tsize = 1u << ts2;
+    // the tile's first slot lists it if it holds fluid (k_bt_keys): the small
+    // tanks hold many tiles of wall particles alone, which have no query
+    const int ts2 = 2 * g.ts, tl = lk >> ts2, tcell = c0 + (tl << ts2);
+    if (lk < g.ncells && (unsigned)k == __ldg(&cstart[tcell])) {
+      const unsigned int tbit = 1u << (tcell & 31);
+      if (tflag[tcell >> 5] & tbit) {
+        atomicAnd(&tflag[tcell >> 5], ~tbit);
+        const int2 t = make_int2(b, tl);
+        if (__ldg(&cstart[tcell + (1 << ts2)]) - (unsigned)k >= (1u << ts2)) B.tiles[atomicAdd(&ctrl->tl_count, 1u)] = t;
+        else B.tiles[B.tiles_cap - 1 - atomicAdd(&ctrl->tl_back, 1u)] = t;
+      }
     }
     const RecParams &rp = B.ip[b].rp;  // a fixed h, and the EOS's p
     if (rp.Pb_on) record_mixed_t<kHFixed, true>(a, slot, v, rp, rec0, rec1, rec2, write_state, eh, nf);
     else record_mixed_t<kHFixed, false>(a, slot, v, rp, rec0, rec1, rec2, write_state, eh, nf);
-  }
-  // A tile with fluid is listed once, by the first warp that stamps it with
-  // this build's number: the small tanks hold many tiles of wall particles
-  // alone, which have no query.
-  const unsigned int tpeers = __match_any_sync(0xffffffffu, tcell);
-  if (tl >= 0 && lane == __ffs(tpeers) - 1) {
-    const unsigned int epoch = ctrl->build_epoch;
-    if (atomicExch(&B.stamp[tcell], epoch) != epoch) {
-      const int2 e = make_int2(b, tl);
-      if (cstart[tcell + tsize] - cstart[tcell] >= tsize) B.tiles[atomicAdd(&ctrl->tl_count, 1u)] = e;
-      else B.tiles[B.tiles_cap - 1 - atomicAdd(&ctrl->tl_back, 1u)] = e;
-    }
   }
   InstSlots *sl = B.sl;
   seg_min_u64(eh, b, [&](int q, unsigned long long m) { atomicMin(&sl[q].pd_hmin, m); });
@@ -1288,13 +1291,13 @@ void launch_bt_build(const StepArgs &a, const WsPtrs &w, const BatchPtrs &B, boo
   const unsigned nb = nblocks(a.n);
   launch_pdl(k_bt_grid, dim3(1), dim3(256), 0, st, B, w.ctrl);
   launch_pdl(k_bt_keys, dim3(nb), dim3(kBlock), 0, st, a.x, a.y, a.n, B, w.ctrl, w.keys, w.refcell, w.crank,
-             w.counts, w.scan_part);
+             w.counts, w.scan_part, a.label, w.tflag);
   launch_pdl(k_scan_cells, dim3((unsigned)w.n_parts), dim3(kScanThreads), 0, st, w.counts, B.scan, w.scan_part,
              w.cstart);
   launch_pdl(k_scatter_rank, dim3(nb), dim3(kBlock), 0, st, w.keys, w.crank, a.n, w.counts, w.cstart, w.perm_tmp,
              w.keys_sorted, w.scan_part, w.n_parts);
   launch_pdl(k_bt_cellsort, dim3(nb), dim3(kBlock), 0, st, w.perm_tmp, w.keys_sorted, w.cstart, w.refcell, a.n, B,
-             w.ctrl, w.perm, w.meta, a, w.rec0, w.rec1, w.rec2, write_state);
+             w.ctrl, w.perm, w.meta, a, w.rec0, w.rec1, w.rec2, write_state, w.tflag);
 }
 
 }  // namespace sph

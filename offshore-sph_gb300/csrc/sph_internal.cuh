@@ -187,7 +187,6 @@ struct DevCtrl {
   // tiles holding a boundary particle in their own list, tl_count other dense
   // ones from the front of the tile list, tl_back sparse ones from its back
   unsigned int tl_count, tl_back, tl_heavy;
-  unsigned int build_epoch;  // builds of the batched form
   unsigned int bounds_done;  // finished blocks of the bounds pass (its last block sets the grid)
   double dt_ring[2][3];  // {dt, dt_c, dt_f} of the step with that parity
   GridKey grid_key;      // inputs of the grid in use
@@ -333,7 +332,6 @@ struct BatchPtrs {
   int *inst;         // instance of each particle (caller order)
   int2 *tiles;       // (instance, tile) of the build's tiles with fluid: dense ones from the front, sparse from the back
   unsigned int tiles_cap;
-  unsigned int *stamp;  // by a tile's first cell: the build that listed it
   DevGrid *scan;     // ncells = total cells - 1, for the scan kernels
   int n_inst;
 };
@@ -391,7 +389,9 @@ struct WsPtrs {
   int2 *fb;  // fallback list of the tile pair kernel: (first slot, count <= 128)
   int *tiles;    // non-empty tiles of the current build (dense from the front, sparse from the back)
   int *tiles_h;  // its dense tiles that hold a boundary particle
-  unsigned int *tflag;  // one bit per tile: it holds a boundary particle (zero between builds)
+  // one bit per tile, zero between builds: it holds a boundary particle; batched
+  // form, by the tile's first cell: it holds a fluid particle
+  unsigned int *tflag;
   long long n_cap, max_cells, n_parts, fb_cap;
   // The sorted copy of the state (when the workspace has room): kStateFields
   // arrays of n_cap doubles, the labels, and each copy index's caller index.
