@@ -973,7 +973,7 @@ __global__ void __launch_bounds__(kTileThreads, TileBlocks<KERNEL>::value)
       if (B.grids[e.x].ts < (int)split) part = first ? 0 : 7;  // 7: nothing to do
     }
     sm.s_inst[slot] = e.x;
-    sm.s_tile[slot] = p < nall ? 8 * e.y + (int)part : -1;
+    sm.s_tile[slot] = p < nall ? 8ll * e.y + part : -1ll;
   };
   if (tid == 0) {
     // every instance's dump cell (reference-OOB particles) is in no tile.  (One
@@ -987,11 +987,12 @@ __global__ void __launch_bounds__(kTileThreads, TileBlocks<KERNEL>::value)
   }
   __syncthreads();
   for (int it = 0;; it++) {
-    const int u = (int)sm.s_tile[it & 1], b = sm.s_inst[it & 1];
+    const long long u = sm.s_tile[it & 1];
+    const int b = sm.s_inst[it & 1];
     if (u < 0) break;
     if (tid == 0) claim((it + 1) & 1);  // the next unit while this one runs
-    const int t = u >> 3;
-    if ((u & 7) == 7) {
+    const int t = (int)(u >> 3), part = (int)u & 7;
+    if (part == 7) {
       __syncthreads();
       continue;
     }
@@ -1003,7 +1004,7 @@ __global__ void __launch_bounds__(kTileThreads, TileBlocks<KERNEL>::value)
       if (tid == 0) {
         const unsigned int *cst = P.cstart + tg.cell0;
         // the unit's rows of the tile (all of them, a half, a quarter)
-        const int part = u & 7, T = 1 << tg.ts, rows = part == 0 ? T : (part <= 2 ? T >> 1 : T >> 2);
+        const int T = 1 << tg.ts, rows = part == 0 ? T : (part <= 2 ? T >> 1 : T >> 2);
         const int c0 = (t << (2 * tg.ts)) + (part == 0 ? 0 : (part <= 2 ? part - 1 : part - 3) * rows * T);
         const unsigned int qs = __ldg(&cst[c0]), qe = __ldg(&cst[c0 + rows * T]);
         for (unsigned int s = qs; s < qe; s += kPairBlock) fb_push(ctrl, fb, fb_cap, s, min((unsigned)kPairBlock, qe - s));
@@ -1012,8 +1013,8 @@ __global__ void __launch_bounds__(kTileThreads, TileBlocks<KERNEL>::value)
       continue;
     }
     const unsigned long long ea =
-        pp.beta == 0.0 ? tile_any<KERNEL, XSPH, SUMDENS, true>(a, P, tg, pp, t, u & 7, true, sm, ctrl, fb, fb_cap)
-                       : tile_any<KERNEL, XSPH, SUMDENS, false>(a, P, tg, pp, t, u & 7, true, sm, ctrl, fb, fb_cap);
+        pp.beta == 0.0 ? tile_any<KERNEL, XSPH, SUMDENS, true>(a, P, tg, pp, t, part, true, sm, ctrl, fb, fb_cap)
+                       : tile_any<KERNEL, XSPH, SUMDENS, false>(a, P, tg, pp, t, part, true, sm, ctrl, fb, fb_cap);
     const unsigned long long ba = block_max_u64<kTileThreads>(ea, sm.red);
     if (tid == 0 && ba != kEncMaxId) atomicMax(&B.sl[b].pd_a2max, ba);
   }

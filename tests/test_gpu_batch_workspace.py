@@ -43,3 +43,35 @@ def test_batched_steps_after_another_entry_point(what, count, shift):
         assert torch.equal(alone.dp._buf, touched.dp._buf), step
     alone.check()
     touched.check()
+
+
+def test_more_than_2_to_28_tiles():
+    """One-cell tiles over a domain of more than 2^28 cells: particles in its
+    corners and its middle step as in a single run."""
+    import numpy as np
+    from sph import batch, build, core, state
+    from sph.Common import particle_dtype
+    build.build()
+    dx, ext = 0.02, 500.0
+    gx, gy = np.meshgrid(np.arange(3) * dx, np.arange(3) * dx)
+    at = [(0, 0), (ext, 0), (0, ext), (ext, ext), (ext / 2, ext / 2), (ext / 3, ext)]
+    pa = np.zeros(9 * len(at), dtype=particle_dtype)
+    pa["x"] = np.concatenate([gx.ravel() + x for x, _ in at])
+    pa["y"] = np.concatenate([gy.ravel() + y for _, y in at])
+    rng = np.random.default_rng(2)
+    pa["vx"], pa["vy"] = rng.normal(0, 0.1, len(pa)), rng.normal(0, 0.1, len(pa))
+    pa["m"], pa["rho"] = 1000.0 * dx * dx, 1000.0
+    E = batch.Ensemble([(pa, dict(height=ext + 1.0, dx=dx))], max_cells=400_000_000)
+    E.setup(0)
+    dp = state.DeviceParticles(E.n)
+    dp._buf.copy_(E.dp._buf)
+    dp.label.copy_(E.dp.label)
+    E.run(2)
+    cells = E.instance_cells(0)
+    E.buf = None
+    cfg = core.config_struct(precision="mixed", h_fixed=E.h[0], cfl_c=0.3, cfl_f=0.25)
+    ws = state.DeviceWorkspace(E.n, cells)
+    core.run(dp, E.wc[0], cfg, ws, 2)
+    ws.check()
+    assert torch.equal(E.dp._buf, dp._buf)
+    assert E.dp.drho.abs().min() > 0
