@@ -168,8 +168,10 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjBlocks) k_pair_adjoint(AdjPtrs 
               coef = fma(c.i_r, r, c.i_0);
               dci = c.i_r * ir;
             } else {
-              coef = fma(c.o_ir, ir, fma(c.o_r, r, c.o_0));
-              dci = ir * fma(-c.o_ir * ir, ir, c.o_r);
+              // o_t t^2 / r, t = 2 - r / h; its derivative -o_t (t / r) (2 / r + 1 / h)
+              const double t = fma(c.o_r, r, 2.0), A = c.o_t * ir * t;
+              coef = A * t;
+              dci = (A * ir) * fma(-2.0, ir, c.o_r);
             }
           } else {
             const double in = fma(c.o_r, r, 1.0), in2 = in * in, in4 = in2 * in2;

@@ -231,28 +231,41 @@ __device__ __forceinline__ double rcp_sum_prod(const Quad64 &v, const Fix64 &c, 
   return pack64<10>(rcp_q63((unsigned int)(p >> 32), (unsigned int)p), 2044 - (e - n + er + lead));
 }
 
+// u^2 / 2^64, within 2 units
+__device__ __forceinline__ unsigned long long square_hi(unsigned long long u) {
+  const unsigned int u1 = (unsigned int)(u >> 32), u0 = (unsigned int)u;
+  return (unsigned long long)u1 * u1 + (((unsigned long long)u1 * u0) >> 31);
+}
+
 // g(q) of the cubic spline's gradient factor -(al / h^2) g, q = r / h:
-// 3 - 2.25 q for q <= 1, 3 / q + 0.75 q - 3 = 0.75 (2 - q)^2 / q up to 2, from
-// the pair's squared distance and ih = 1 / h, h; q < 2 + 2^-40.  Fixed point,
-// absolute error below 2^-58.
+// 3 - 2.25 q for q <= 1, 0.75 (2 - q)^2 / q up to 2, from the pair's squared
+// distance and ih = 1 / h, h; q < 2 + 2^-40.  Fixed point.  2 - q is an exact
+// difference of integers and is normalised before it is squared, so that g has
+// the relative accuracy of 2 - q up to the support's edge (multiplied out, as
+// 3 / q + 0.75 q - 3, it cancels there: 2e-8 off at q = 1.9999).
 __device__ __forceinline__ double cubic_g(const Quad64 &v, const Fix64 &ih, const Fix64 &h) {
   const unsigned long long y = rsqrt_q63(v);
   // q = r ih in units of 2^-61: r = s 2^k, s in [1, 2) in units of 2^-61
   const int sq = v.k + ih.e;  // q = (s ih.m) 2^sq, the product in [1, 4)
   const unsigned long long q = mul_hi(sqrt_q61(v, y) << 2, ih.m << 1) >> min(max(1 - sq, 0), 63);
-  constexpr unsigned long long three = 3ull << 61;
-  unsigned long long g;
-  if (q <= 1ull << 61) {
-    g = three - 2 * q - (q >> 2);
+  constexpr unsigned long long one = 1ull << 61;
+  unsigned long long g;  // the result is g 2^(e - 1086)
+  int e;
+  if (q <= one) {
+    g = 3 * one - 2 * q - (q >> 2);
+    e = 1086 - 61;
   } else {
+    if (q >= 2 * one) return 0.0;
     // 1 / q = y h 2^-k in units of 2^-61: y in [0.5, 1], h.m / 2^62 in [1, 2)
     const unsigned long long iq = mul_hi(y, h.m << 1) >> min(max(1 - (h.e - v.k), 0), 63);
-    const unsigned long long t = 3 * iq + (q >> 1) + (q >> 2);
-    g = t > three ? t - three : 0ull;
+    const unsigned long long t = 2 * one - q;
+    const int n = __clzll((long long)t);                             // t = (t << n) 2^(-61 - n)
+    const unsigned long long p = mul_hi(square_hi(t << n), iq << 2);  // t^2 / q in units of 2^(-57 - 2 n)
+    g = p - (p >> 2);
+    e = 1086 - 57 - 2 * n;
   }
-  if (g == 0ull) return 0.0;
   const int n = __clzll((long long)g);
-  return pack64<10>(g << (n - 1), 1086 - n - 61);
+  return pack64<10>(g << (n - 1), e - n);
 }
 
 // ---------------------------------------------------------------------------
@@ -286,11 +299,6 @@ __device__ __forceinline__ double fix_diff(unsigned long long a, int s, bool neg
   if (a == 0ull) return 0.0;
   const int n = __clzll((long long)a);
   return pack64<10>(a << (n - 1), 1086 - n - s, neg ? 0x80000000u : 0u);
-}
-// u^2 / 2^64, within 2 units
-__device__ __forceinline__ unsigned long long square_hi(unsigned long long u) {
-  const unsigned int u1 = (unsigned int)(u >> 32), u0 = (unsigned int)u;
-  return (unsigned long long)u1 * u1 + (((unsigned long long)u1 * u0) >> 31);
 }
 __device__ __forceinline__ PairGeom pair_geom(longlong2 a, longlong2 b, int s) {
   PairGeom p;
@@ -338,7 +346,7 @@ struct Pair64 {
   double h, ih, lim;           // h, 1/h, (support h)^2
   double lim_lo, lim_hi;       // Gaussian: below / above, q <= 3 is decided
   double h2;                   // cubic: d2 <= h^2 is the inner piece.  Gaussian: d2 <= h2 has no gradient
-  double o_ir, o_r, o_0;       // cubic, outer piece: o_ir / r + o_r r + o_0
+  double o_t, o_r;             // cubic, outer piece: (o_t / r) (2 + o_r r)^2
   double i_r, i_0;             // inner piece: i_r r + i_0.  Wendland: (i_r r + i_0) (1 + o_r r)^5
   double scale;                // FIX: of the gradient factor that is summed (cubic: -al / h^2)
   Fix64 hf, ihf, hb2f;         // h, 1/h, hb2
@@ -358,14 +366,13 @@ inline Pair64 pair64_consts(const sph_config_t &cfg, const sph_wcsph_t &wc) {
   c.h = h;
   c.ih = ih;
   c.h2 = h * h;
-  c.o_ir = c.o_r = c.o_0 = c.i_r = c.i_0 = 0.0;
+  c.o_t = c.o_r = c.i_r = c.i_0 = 0.0;
   if (cfg.kernel == SPH_KERNEL_CUBIC) {
     // al / (h r) times -0.75 (2 - q)^2 and -3 q (1 - 0.75 q) (CubicSpline.py:40-70)
     c.al = kCubicFac * ih2;
     c.lim = 4.0 * h * h;
-    c.o_ir = -3.0 * c.al * ih;
-    c.o_0 = 3.0 * c.al * ih2;
-    c.o_r = -0.75 * c.al * ih2 * ih;
+    c.o_t = -0.75 * c.al * ih;
+    c.o_r = -ih;
     c.i_0 = -3.0 * c.al * ih2;
     c.i_r = 2.25 * c.al * ih2 * ih;
   } else if (cfg.kernel == SPH_KERNEL_WENDLAND) {

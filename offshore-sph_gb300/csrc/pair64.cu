@@ -71,7 +71,10 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
           coef = cubic_g(geo.v, c.ihf, c.hf);
         } else if (KERNEL == SPH_KERNEL_CUBIC) {
           if (le_bits(d2, c.h2)) coef = fma(c.i_r, r, c.i_0);
-          else coef = fma(c.o_ir, ir, fma(c.o_r, r, c.o_0));
+          else {
+            const double t = fma(c.o_r, r, 2.0);
+            coef = (c.o_t * ir) * (t * t);
+          }
         } else {
           const double in = fma(c.o_r, r, 1.0), in2 = in * in;
           coef = (in2 * in2) * (in * fma(c.i_r, r, c.i_0));
@@ -83,10 +86,10 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
         if (c.xsph) {
           const double qq = r * ih;
           if (KERNEL == SPH_KERNEL_CUBIC) {
-            const double t = 2.0 - qq;
+            const double t = fma(c.o_r, r, 2.0);
             w = le_bits(d2, c.h2) ? c.al * (1.0 - 1.5 * (qq * qq) * (1.0 - 0.5 * qq)) : c.al * 0.25 * (t * t * t);
           } else {
-            const double in = 1.0 - 0.5 * qq, in2 = in * in;
+            const double in = fma(c.o_r, r, 1.0), in2 = in * in;
             w = c.al * (in2 * in2 * in2 * ((35.0 / 12.0) * qq * qq + 3.0 * qq + 1.0));
           }
         }
@@ -115,13 +118,13 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
             coef = (al * ih2) * fma(2.25, qq, -3.0);
             if (c.xsph) w = al * (1.0 - 1.5 * (qq * qq) * (1.0 - 0.5 * qq));
           } else {
-            const double t = 2.0 - qq, t2 = t * t;
+            const double t = fma(-r, ih, 2.0), t2 = t * t;
             coef = (-0.75 * al) * t2 * (ih * ir);
             if (c.xsph) w = al * 0.25 * (t2 * t);
           }
         } else {
           const double al = kWendFac * ih2;
-          const double in = fma(-0.5, qq, 1.0), in2 = in * in, in5 = in2 * in2 * in;
+          const double in = fma(-r, half_exact(ih), 1.0), in2 = in * in, in5 = in2 * in2 * in;
           coef = (al * ih2) * in5 * fma(-35.0 / 3.0, qq, -14.0 / 3.0);
           if (c.xsph) w = al * (in5 * in) * ((35.0 / 12.0) * qq * qq + 3.0 * qq + 1.0);
         }
