@@ -156,9 +156,8 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjBlocks) k_pair_adjoint(AdjPtrs 
         if constexpr (gauss) {
           if (!le_bits(d2, c.lim_lo) && (!le_bits(d2, c.lim_hi) || !near_exact(Ak.x - Aj.x, Ak.y - Aj.y, hk))) return;
           if (le_bits(d2, c.h2)) return;
-          const double ih2 = c.ih * c.ih;
-          coef = c.i_0 * exp_neg(d2 * ih2);
-          dci = coef * (-2.0 * ih2);
+          coef = c.i_0 * exp2_neg(geo.v, c.l2e);
+          dci = coef * c.g_d;
         } else {
           if (!le_bits(d2, c.lim) || le_bits(d2, 1e-20)) return;
           double r, ir;
@@ -169,12 +168,12 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjBlocks) k_pair_adjoint(AdjPtrs 
               dci = c.i_r * ir;
             } else {
               // o_t t^2 / r, t = 2 - r / h; its derivative -o_t (t / r) (2 / r + 1 / h)
-              const double t = fma(c.o_r, r, 2.0), A = c.o_t * ir * t;
+              const double t = fma(c.o_rl, r, fma(c.o_r, r, 2.0)), A = c.o_t * ir * t;
               coef = A * t;
               dci = (A * ir) * fma(-2.0, ir, c.o_r);
             }
           } else {
-            const double in = fma(c.o_r, r, 1.0), in2 = in * in, in4 = in2 * in2;
+            const double in = fma(c.o_rl, r, fma(c.o_r, r, 1.0)), in2 = in * in, in4 = in2 * in2;
             const double l = fma(c.i_r, r, c.i_0);
             coef = in4 * (in * l);
             dci = ir * in4 * fma(5.0 * c.o_r, l, in * c.i_r);

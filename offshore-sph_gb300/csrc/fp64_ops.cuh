@@ -79,6 +79,35 @@ __device__ __forceinline__ double rcp64(double x) {
   return pack64<10>(rcp_q63(__funnelshift_l(lo, mh, 11), lo << 11), 2045 - (int)e, hi & 0x80000000u);
 }
 
+// 1/x in two parts y + yl, 1/x^2 and 1/x^4 for x > 0, each rounded once
+static __device__ __noinline__ void rcp_powers_slow(double x, double &y, double &yl, double &y2, double &y4) {
+  y = 1.0 / x;
+  yl = fma(-y, x, 1.0) * y;
+  y2 = y * y;
+  y4 = y2 * y2;
+}
+__device__ __forceinline__ void rcp_powers(double x, double &y, double &yl, double &y2, double &y4) {
+  const unsigned int hi = (unsigned int)__double2hiint(x), lo = (unsigned int)__double2loint(x);
+  const int e = (int)(hi >> 20) - 1023;
+  if ((unsigned int)(e + 250) > 500u) {  // a power out of range, or x not positive
+    rcp_powers_slow(x, y, yl, y2, y4);
+    return;
+  }
+  const unsigned int mh = (hi & 0xfffffu) | 0x100000u;
+  const unsigned long long a = rcp_q63(__funnelshift_l(lo, mh, 11), lo << 11);  // (2^62, 2^63]
+  y = pack64<10>(a, 1022 - e);
+  // what that rounded off, -512 to 511 units of 2^(-63 - e): as a float, and its
+  // exponent moved (0 becomes about 2^-190 of y)
+  const unsigned int f = __float_as_uint((float)(((int)(unsigned int)a << 22) >> 22));
+  yl = __hiloint2double((int)((f & 0x80000000u) | (((f & 0x7fffffffu) >> 3) + ((unsigned int)(833 - e) << 20))), 0);
+  const unsigned long long b = mul_hi(a, a);  // units of 2^-62
+  const int n = __clzll((long long)b);        // 1 to 3
+  y2 = pack64<10>(b << (n - 1), 1024 - n - 2 * e);
+  const unsigned long long d = mul_hi(b << n, b << n);  // units of 2^(-60 - 2 n), [2^62, 2^64)
+  const int m = (int)(d >> 63);
+  y4 = pack64<10>(d >> m, 1025 + m - 2 * n - 4 * e);
+}
+
 // A positive number v 4^k, v in [1, 4) in units of 2^-62.
 struct Quad64 {
   unsigned int vh, vl;
@@ -123,10 +152,15 @@ struct Fix64 {
   unsigned long long m;
   int e;
 };
-inline Fix64 fix64(double x) {
+inline Fix64 fix64(double x, double lo = 0.0) {  // x + lo, lo below x's last bit
   int e = 0;
   const double f = frexp(x, &e);  // [0.5, 1)
-  return {(unsigned long long)ldexp(f, 63), e - 1};
+  return {(unsigned long long)ldexp(f, 63) + (unsigned long long)(long long)ldexp(lo, 63 - e), e - 1};
+}
+// (a + al) / (b + bl) to 63 bits: the quotient and its remainder's
+inline Fix64 fix64_quot(double a, double al, double b, double bl) {
+  const double q = a / b;
+  return fix64(q, (fma(-q, b, a) + (al - q * bl)) / b);
 }
 
 // exp(-z) for 0 <= z < 11: table lookup and a short polynomial (P. T. P. Tang,
@@ -346,8 +380,9 @@ struct Pair64 {
   double h, ih, lim;           // h, 1/h, (support h)^2
   double lim_lo, lim_hi;       // Gaussian: below / above, q <= 3 is decided
   double h2;                   // cubic: d2 <= h^2 is the inner piece.  Gaussian: d2 <= h2 has no gradient
-  double o_t, o_r;             // cubic, outer piece: (o_t / r) (2 + o_r r)^2
-  double i_r, i_0;             // inner piece: i_r r + i_0.  Wendland: (i_r r + i_0) (1 + o_r r)^5
+  double o_t, o_r, o_rl;       // cubic, outer piece: (o_t / r) (2 + o_r r)^2, o_r = -1 / h in two parts
+  double i_r, i_0;             // inner piece: i_r r + i_0.  Wendland: (i_r r + i_0) (1 + o_r r)^5, o_r = -1 / (2 h)
+  double g_d;                  // Gaussian: -2 / h^2, the gradient factor's derivative over r
   double scale;                // FIX: of the gradient factor that is summed (cubic: -al / h^2)
   Fix64 hf, ihf, hb2f;         // h, 1/h, hb2
   Fix64 l2e;                   // log2(e) / h^2
@@ -362,41 +397,44 @@ inline Pair64 pair64_consts(const sph_config_t &cfg, const sph_wcsph_t &wc) {
   c.xsph = wc.use_xsph != 0;
   c.sumdens = wc.use_summation_density != 0;
   const double h = cfg.h_fixed > 0.0 ? cfg.h_fixed : 1.0;
-  const double ih = 1.0 / h, ih2 = ih * ih;
+  const double ih = 1.0 / h, hh = h * h;
   c.h = h;
   c.ih = ih;
-  c.h2 = h * h;
-  c.o_t = c.o_r = c.i_r = c.i_0 = 0.0;
+  c.h2 = hh;
+  c.o_t = c.i_r = c.i_0 = 0.0;
+  c.o_r = -ih;
+  c.o_rl = -fma(-ih, h, 1.0) / h;
+  c.g_d = -2.0 / hh;
   if (cfg.kernel == SPH_KERNEL_CUBIC) {
     // al / (h r) times -0.75 (2 - q)^2 and -3 q (1 - 0.75 q) (CubicSpline.py:40-70)
-    c.al = kCubicFac * ih2;
+    c.al = kCubicFac / hh;
     c.lim = 4.0 * h * h;
-    c.o_t = -0.75 * c.al * ih;
-    c.o_r = -ih;
-    c.i_0 = -3.0 * c.al * ih2;
-    c.i_r = 2.25 * c.al * ih2 * ih;
+    c.o_t = -0.75 * c.al / h;
+    c.i_0 = -3.0 * c.al / hh;
+    c.i_r = 2.25 * c.al / (hh * h);
   } else if (cfg.kernel == SPH_KERNEL_WENDLAND) {
     // al / (h r) (1 - q/2)^5 (-14/3) q (1 + 2.5 q) (Wendland.py:36-64)
-    c.al = kWendFac * ih2;
+    c.al = kWendFac / hh;
     c.lim = 4.0 * h * h;
-    c.o_r = -0.5 * ih;
-    c.i_0 = (-14.0 / 3.0) * c.al * ih2;
-    c.i_r = (-35.0 / 3.0) * c.al * ih2 * ih;
+    c.o_r *= 0.5;
+    c.o_rl *= 0.5;
+    c.i_0 = (-14.0 / 3.0) * c.al / hh;
+    c.i_r = (-35.0 / 3.0) * c.al / (hh * h);
   } else {
     // -2 al / h^2 exp(-q^2) (Gaussian.py:37-59)
-    c.al = kInvPi * ih2;
+    c.al = kInvPi / hh;
     c.lim = 9.0 * h * h;
-    c.i_0 = -2.0 * c.al * ih2;
-    c.h2 = 1e-24 * ih2;  // r h <= 1e-12: no gradient
+    c.i_0 = -2.0 * c.al / hh;
+    c.h2 = 1e-24 / hh;  // r h <= 1e-12: no gradient
   }
   c.lim_lo = c.lim * (1.0 - 1e-9);
   c.lim_hi = c.lim * (1.0 + 1e-9);
-  c.hb2 = 0.01 * (h * h);
+  c.hb2 = 0.01 * hh;
   c.hf = fix64(h);
-  c.ihf = fix64(ih);
+  c.ihf = fix64_quot(1.0, 0.0, h, 0.0);
   c.hb2f = fix64(c.hb2);
-  c.l2e = fix64(1.44269504088896340736 * ih2);
-  c.scale = cfg.kernel == SPH_KERNEL_CUBIC ? -c.al * ih2 : (cfg.kernel == SPH_KERNEL_GAUSSIAN ? c.i_0 : 1.0);
+  c.l2e = fix64_quot(0x1.71547652b82fep+0, 0x1.777d0ffda0d24p-56, hh, fma(h, h, -hh));  // log2(e) in two parts
+  c.scale = cfg.kernel == SPH_KERNEL_CUBIC ? -c.al / hh : (cfg.kernel == SPH_KERNEL_GAUSSIAN ? c.i_0 : 1.0);
   c.pic = -wc.alpha * wc.co * h;  // -2 alpha c_ij h with c_ij = co / 2
   c.r02 = wc.r0 * wc.r0;
   c.lj_free = cfg.h_fixed > 0.0 && wc.r0 < 1.5 * h * (1.0 - 1e-9);

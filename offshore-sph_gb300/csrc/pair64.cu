@@ -59,7 +59,7 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
     if constexpr (UH) {
       if constexpr (gauss) {
         if (!le_bits(d2, c.lim_lo) && (!le_bits(d2, c.lim_hi) || !near_exact(q.x - A.x, q.y - A.y, hij))) return;
-        const double e = FIX ? exp2_neg(geo.v, c.l2e) : exp_neg(d2 * (ih * ih));
+        const double e = exp2_neg(geo.v, c.l2e);
         coef = le_bits(d2, c.h2) ? 0.0 : (FIX ? e : c.i_0 * e);  // FIX: scaled in the sum
         if (c.xsph) w = c.al * e;
       } else {
@@ -72,11 +72,11 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
         } else if (KERNEL == SPH_KERNEL_CUBIC) {
           if (le_bits(d2, c.h2)) coef = fma(c.i_r, r, c.i_0);
           else {
-            const double t = fma(c.o_r, r, 2.0);
+            const double t = fma(c.o_rl, r, fma(c.o_r, r, 2.0));
             coef = (c.o_t * ir) * (t * t);
           }
         } else {
-          const double in = fma(c.o_r, r, 1.0), in2 = in * in;
+          const double in = fma(c.o_rl, r, fma(c.o_r, r, 1.0)), in2 = in * in;
           coef = (in2 * in2) * (in * fma(c.i_r, r, c.i_0));
         }
         if (tiny) {
@@ -86,10 +86,10 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
         if (c.xsph) {
           const double qq = r * ih;
           if (KERNEL == SPH_KERNEL_CUBIC) {
-            const double t = fma(c.o_r, r, 2.0);
+            const double t = fma(c.o_rl, r, fma(c.o_r, r, 2.0));
             w = le_bits(d2, c.h2) ? c.al * (1.0 - 1.5 * (qq * qq) * (1.0 - 0.5 * qq)) : c.al * 0.25 * (t * t * t);
           } else {
-            const double in = fma(c.o_r, r, 1.0), in2 = in * in;
+            const double in = fma(c.o_rl, r, fma(c.o_r, r, 1.0)), in2 = in * in;
             w = c.al * (in2 * in2 * in2 * ((35.0 / 12.0) * qq * qq + 3.0 * qq + 1.0));
           }
         }
@@ -97,14 +97,14 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
     } else {
       hij = half_exact(q.h + B.w);  // both positive or zero
       if (!(__double2hiint(hij) > 0)) return;  // q = r / 0
-      ih = rcp64(hij);
-      const double ih2 = ih * ih;
+      double ihl, ih2, ih4;
+      rcp_powers(hij, ih, ihl, ih2, ih4);
       if constexpr (gauss) {
         const double z = d2 * ih2;
         if (!le_bits(z, 9.0 * (1.0 - 1e-9)) && (!le_bits(z, 9.0 * (1.0 + 1e-9)) || !near_exact(q.x - A.x, q.y - A.y, hij))) return;
-        const double e = kInvPi * ih2 * exp_neg(z);
-        coef = le_bits(d2, 1e-24 * ih2) ? 0.0 : -2.0 * e * ih2;
-        w = e;
+        const double e = exp_neg(z);
+        coef = le_bits(d2, 1e-24 * ih2) ? 0.0 : (-2.0 * kInvPi) * ih4 * e;
+        if (c.xsph) w = kInvPi * ih2 * e;
       } else {
         double r, ir;
         sqrt_rsqrt64(geo.v, r, ir);
@@ -112,21 +112,20 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
         if (tiny) r = 0.0;
         const double qq = r * ih;
         if (!le_bits(qq, 2.0)) return;
+        const double t = fma(-r, ihl, fma(-r, ih, 2.0)), t2 = t * t;  // 2 - q
         if (KERNEL == SPH_KERNEL_CUBIC) {
           const double al = kCubicFac * ih2;
           if (le_bits(qq, 1.0)) {
-            coef = (al * ih2) * fma(2.25, qq, -3.0);
+            coef = (kCubicFac * ih4) * fma(2.25, qq, -3.0);
             if (c.xsph) w = al * (1.0 - 1.5 * (qq * qq) * (1.0 - 0.5 * qq));
           } else {
-            const double t = fma(-r, ih, 2.0), t2 = t * t;
-            coef = (-0.75 * al) * t2 * (ih * ir);
+            coef = (-0.75 * kCubicFac) * ih4 * (hij * ir) * t2;
             if (c.xsph) w = al * 0.25 * (t2 * t);
           }
         } else {
-          const double al = kWendFac * ih2;
-          const double in = fma(-r, half_exact(ih), 1.0), in2 = in * in, in5 = in2 * in2 * in;
-          coef = (al * ih2) * in5 * fma(-35.0 / 3.0, qq, -14.0 / 3.0);
-          if (c.xsph) w = al * (in5 * in) * ((35.0 / 12.0) * qq * qq + 3.0 * qq + 1.0);
+          const double t5 = t2 * t2 * t;  // 32 (1 - q / 2)^5
+          coef = (kWendFac / 32 * ih4) * t5 * fma(-35.0 / 3.0, qq, -14.0 / 3.0);
+          if (c.xsph) w = (kWendFac / 64 * ih2) * (t5 * t) * ((35.0 / 12.0) * qq * qq + 3.0 * qq + 1.0);
         }
         if (tiny) coef = 0.0;
       }

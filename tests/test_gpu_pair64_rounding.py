@@ -1,0 +1,86 @@
+"""Rounding of the FP64 pair kernel: the derivatives of isolated pairs are off
+from the exact ones by no more than the reference's arithmetic is (its formulas
+with every operation rounded to 64 bits), in the mean square over the pairs.
+The mean square of N errors is known to 1 / sqrt(N) or so, which the bar
+allows twice.  Errors of the 2 h kernels are weighted by 2 - q, to which the
+powers of 2 - q are conditioned."""
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+CUBIC, GAUSS, WEND = 0, 1, 2
+MASS = 0.4
+
+
+def _pairs(n, h, kernel, seed):
+    """n pairs of particles 12 h apart on a square array, q from 0.3 to the
+    kernel's support, the second half of each pair after the first halves."""
+    from sph.Common import particle_dtype
+    rng = np.random.default_rng(seed)
+    side = int(np.ceil(np.sqrt(n)))
+    k = np.arange(n)
+    q = rng.uniform(0.3, 2.9 if kernel == GAUSS else 1.99, n)
+    ang = rng.uniform(-1.0, 1.0, n)
+    pa = np.zeros(2 * n, dtype=particle_dtype)
+    pa["x"][:n], pa["y"][:n] = 12.0 * h * (k % side) + 0.3, 12.0 * h * (k // side) + 0.3
+    pa["x"][n:], pa["y"][n:] = pa["x"][:n] + q * h * np.cos(ang), pa["y"][:n] + q * h * np.sin(ang)
+    pa["m"] = MASS
+    pa["rho"] = rng.uniform(1010.0, 1050.0, 2 * n)
+    va = ang + rng.uniform(-1.0, 1.0, n)
+    s = rng.uniform(0.1, 1.0, n)
+    pa["vx"][n:], pa["vy"][n:] = s * np.cos(va), s * np.sin(va)
+    return pa
+
+
+def _restated(F, s, n, kernel):
+    """drho of every particle by the reference's formulas, in the type F, from
+    the inputs s and the h that the evaluation had (CubicSpline.py:40-70,
+    Gaussian.py:37-59, Wendland.py:36-64, Continuity.py)."""
+    j = np.r_[n:2 * n, 0:n]
+    x, y, vx, vy, h = (s[k].astype(F) for k in ("x", "y", "vx", "vy", "h"))
+    pi = F("3.14159265358979323846264338327950288") if F is not np.float64 else math.pi
+    dx, dy = x - x[j], y - y[j]
+    r = np.sqrt(dx * dx + dy * dy)
+    hij = F(0.5) * (h + h[j])
+    q = r / hij
+    if kernel == CUBIC:
+        al = F(10) / (F(7) * pi) / (hij * hij)
+        g = np.where(q > 1, F(-0.75) * ((2 - q) * (2 - q)), F(-3) * q * (1 - F(0.75) * q))
+        coef = al * g / (hij * r)
+    elif kernel == WEND:
+        al = F(9) / (F(4) * pi) / (hij * hij)
+        t = 1 - F(0.5) * q
+        coef = al * (t * t * t * t * t) * (F(-14) / F(3)) * q * (1 + F(2.5) * q) / (hij * r)
+    else:
+        al = F(1) / pi / (hij * hij)
+        coef = F(-2) * q * al * np.exp(-q * q) / (r * hij)
+    vxij, vyij = vx - vx[j], vy - vy[j]
+    drho = F(MASS) * (vxij * (coef * dx) + vyij * (coef * dy))
+    return q, drho
+
+
+@pytest.mark.parametrize("kernel", [CUBIC, GAUSS, WEND])
+@pytest.mark.parametrize("fixed", [True, False])
+@pytest.mark.parametrize("n", [3001, 10007, 35003])
+def test_continuity_of_a_pair(kernel, fixed, n):
+    """n pairs take 8, 4 and 1 lanes per query."""
+    from sph import build, core, state
+    build.build()
+    h = 0.0325 if fixed else 1.3 * np.sqrt(MASS / 1030.0)
+    pa = _pairs(n, h, kernel, n + kernel)
+    dp = state.DeviceParticles.from_array(pa)
+    dp.h.fill_(h)
+    wc = core.wcsph_struct(5.0, 0.01, 1000.0)
+    ws = state.DeviceWorkspace(dp.n)
+    core.compute(dp, wc, core.config_struct(kernel=kernel, precision="fp64", h_fixed=h if fixed else 0.0), ws)
+    ws.check()
+    got = dp.soa()
+    q, want = _restated(np.longdouble, got, n, kernel)
+    _, fp64 = _restated(np.float64, got, n, kernel)
+    w = np.minimum(2 - q, 1) if kernel != GAUSS else np.ones_like(q)
+    hij = 0.5 * (got["h"] + np.roll(got["h"], n))
+    ok = q * hij < 1.99 * got["h"].min()  # the reach of the reference's stencil
+    rms = lambda v: np.sqrt(np.mean((((v - want) / want * w)[ok]).astype(np.float64) ** 2))  # noqa: E731
+    assert rms(got["drho"]) <= rms(fp64) * (1 + 2 / np.sqrt(ok.sum())), (rms(got["drho"]), rms(fp64))
