@@ -836,8 +836,14 @@ __device__ __forceinline__ void record_fp64(const StepArgs &a, long long k, int 
   if (fl && !rp.from_state) h = rp.h_fixed_on ? rp.h_fixed : compute_h_call(m, rho);
   const double p = rp.from_state ? a.p[i] : tait_p(rho, lab, rp.gamma, rp.B, rp.inv_rho0, rp.Pb);
   // p / rho^2 of a fluid particle; no kernel reads a boundary particle's,
-  // whose 0 / 0 took the division's slow path
-  const double othr = !fl ? 0.0 : (rho > 0.0 ? p * rcp64(rho * rho) : p / (rho * rho));
+  // whose 0 / 0 took the division's slow path.  The quotient by rcp64 and its
+  // remainder (P. W. Markstein, IBM J. Res. Dev. 34, 1990), rounded as a division
+  // rounds it: 4 FP64 operations, and a division 7 us of a step of 1M particles.
+  double othr = 0.0;
+  if (fl) {
+    const double d = rho * rho, y = rcp64(d), q = p * y;
+    othr = finite_bits(q) && finite_bits(d) ? fma(fma(-q, d, p), y, q) : p / d;
+  }
   const double hs = fl ? h : -h;
   r64a[k] = make_double4_32a(x, y, a.vx[i], a.vy[i]);
   if (rp.fix) reinterpret_cast<longlong2 *>(rec1)[k] = make_longlong2(to_fix(x, fix_s), to_fix(y, fix_s));

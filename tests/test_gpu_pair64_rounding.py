@@ -84,3 +84,35 @@ def test_continuity_of_a_pair(kernel, fixed, n):
     ok = q * hij < 1.99 * got["h"].min()  # the reach of the reference's stencil
     rms = lambda v: np.sqrt(np.mean((((v - want) / want * w)[ok]).astype(np.float64) ** 2))  # noqa: E731
     assert rms(got["drho"]) <= rms(fp64) * (1 + 2 / np.sqrt(ok.sum())), (rms(got["drho"]), rms(fp64))
+
+
+def test_pressure_term():
+    """p / rho^2 has the two roundings of the reference's (WCSPH.py:160-164).
+    Pairs at r = h on one line, h a power of two: the gradient factor is 0.75
+    and the difference h, both exact, and the constants are the same for every
+    pair, so what varies from pair to pair is the rounding of p / rho^2, of the
+    sum, and of two products."""
+    from sph import build, core, state
+    from sph.Common import particle_dtype
+    build.build()
+    n, h = 10007, 0.03125
+    rng = np.random.default_rng(1)
+    k = np.arange(n)
+    pa = np.zeros(2 * n + 1, dtype=particle_dtype)  # and one alone, which keeps the others off the grid's edge
+    pa["x"][:n], pa["y"][:n] = 12 * h * (k % 101), 12 * h * (k // 101)
+    pa["x"][n:-1], pa["y"][n:-1] = pa["x"][:n] + h, pa["y"][:n]
+    pa["x"][-1], pa["y"][-1] = 3.3 * h, 12 * h * (n // 101) + 6.7 * h
+    pa["m"], pa["rho"] = 0.5, rng.uniform(1010.0, 1050.0, 2 * n + 1)
+    dp = state.DeviceParticles.from_array(pa)
+    dp.h.fill_(h)
+    ws = state.DeviceWorkspace(dp.n)
+    core.compute(dp, core.wcsph_struct(5.0, 0.01, 1000.0, alpha=0.0), core.config_struct(h_fixed=h), ws)
+    ws.check()
+    got = {k: v[:-1] for k, v in dp.soa().items()}
+
+    def term(F):
+        o = got["p"].astype(F) / (got["rho"].astype(F) * got["rho"].astype(F))
+        return F(0.375) * (o + np.roll(o, n)) * F(0.1)
+    want = term(np.longdouble)
+    rms = lambda v: np.std((np.abs(v) / want / np.mean(np.abs(v) / want) - 1).astype(np.float64))  # noqa: E731
+    assert rms(got["ax"]) <= rms(term(np.float64)) * (1 + 2 / np.sqrt(2 * n)), (rms(got["ax"]), rms(term(np.float64)))
