@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjBlocks) k_pair_adjoint(AdjPtrs 
     const double ac = ap.alpha * 0.5 * ap.co;
     const longlong2 pk = kFix ? P.fix[kq] : longlong2();
     const int fix_s = g.fix_s;
-    const bool wide = g.pad_e > 0.5f * (float)g.r_search;
+    const bool wide = (kFix && fix_cut(pk)) || g.pad_e > 0.5f * (float)g.r_search;
     const int2 qref = P.meta[kq];
     const bool slow = qref.x >= g.ncx;
     const int W = g.mode == 0 ? 1 : (slow ? g.wide : g.wt);
@@ -145,8 +145,12 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjBlocks) k_pair_adjoint(AdjPtrs 
     for_neighbours<G, kCap, kAdjBlock>(sten, P.cstart, act, lists, near, [&](unsigned int j) {
       const double4_32a Aj = P.r64a[j], Bj = P.r64b[j];
       PairGeom geo;
-      if constexpr (kFix) geo = wide ? pair_geom_wide(Ak.x - Aj.x, Ak.y - Aj.y) : pair_geom(pk, P.fix[j], fix_s);
-      else geo = pair_geom_fp64(Ak.x - Aj.x, Ak.y - Aj.y);
+      if constexpr (kFix) {
+        const longlong2 pj = P.fix[j];
+        geo = wide || fix_cut(pj) ? pair_geom_wide(Ak.x - Aj.x, Ak.y - Aj.y) : pair_geom(pk, pj, fix_s);
+      } else {
+        geo = pair_geom_fp64(Ak.x - Aj.x, Ak.y - Aj.y);
+      }
       const double dx = geo.dx, dy = geo.dy, d2 = geo.d2;
       if (le_bits(d2, 1e-24)) return;  // coincident: no kernel gradient, no boundary force
       if (!signbit(Bj.w)) {

@@ -306,8 +306,9 @@ __device__ __forceinline__ double cubic_g(const Quad64 &v, const Fix64 &ih, cons
 // Positions as 64-bit integers, for pair differences on the integer pipe: a
 // position in units of 2^-s modulo 2^64, with s such that the interaction
 // radius is below 2^62 units (fix_shift), so that the difference of two
-// candidates' integers is that of their positions: exact for coordinates with
-// no bits below 2^-s (|x| > R / 512), within R 2^-61 for the others.
+// candidates' integers is that of their positions, exactly.  The lowest bit is not
+// the position's: it marks a coordinate with bits below 2^(1 - s) (one closer to
+// zero than R / 256, unless it ends in zeros), whose pairs take FP64 differences.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int fix_shift(double R) {
   return 61 - ((int)(((unsigned int)__double2hiint(R) >> 20) & 0x7ffu) - 1023);
@@ -315,12 +316,18 @@ __device__ __forceinline__ int fix_shift(double R) {
 __device__ __forceinline__ long long to_fix(double x, int s) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(x);
   const int e = (int)((u >> 52) & 0x7ffu);
-  unsigned long long m = (u & 0xfffffffffffffull) | (e ? 0x10000000000000ull : 0ull);
+  unsigned long long m = (u & 0xfffffffffffffull) | (e ? 0x10000000000000ull : 0ull), cut = 0ull;
   const int sh = e - 1075 + s;
-  if (sh >= 0) m = sh < 64 ? m << sh : 0ull;
-  else m = sh > -64 ? m >> -sh : 0ull;
-  return (u >> 63) ? -(long long)m : (long long)m;
+  if (sh > 0) {
+    m = sh < 64 ? m << sh : 0ull;
+  } else {
+    const unsigned long long low = sh > -63 ? (2ull << -sh) - 1ull : ~0ull;
+    cut = (m & low) ? 1ull : 0ull;
+    m = sh > -64 ? (m & ~low) >> -sh : 0ull;
+  }
+  return (long long)(((u >> 63) ? 0ull - m : m) | cut);
 }
+__device__ __forceinline__ bool fix_cut(longlong2 a) { return ((a.x | a.y) & 1ll) != 0ll; }
 
 // A pair's geometry: the differences, the squared distance (each rounded once)
 // and the latter's significand for sqrt_rsqrt64.
@@ -361,8 +368,9 @@ __device__ __forceinline__ PairGeom pair_geom_fp64(double dx, double dy) {
   p.v = quad64(p.d2);
   return p;
 }
-// out of line: where the padding of the FP32 test could let differences past
-// the integers' range through (a domain of some millions of radii)
+// out of line: for a coordinate whose integer is not all of it (to_fix), and
+// where the padding of the FP32 test could let differences past the integers'
+// range through (a domain of some millions of radii)
 static __device__ __noinline__ PairGeom pair_geom_wide(double dx, double dy) { return pair_geom_fp64(dx, dy); }
 
 // a <= b for non-negative doubles (false when either is NaN and a is not

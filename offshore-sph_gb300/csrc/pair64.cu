@@ -38,7 +38,7 @@ struct Query64 {
   double x, y, vx, vy, rho, oth, h;
   longlong2 p;  // integer position
   int fix_s;
-  bool wide;    // the integers' differences could wrap
+  bool wide;    // FP64 differences: its integers are cut, or their differences could wrap
 };
 
 // One listed candidate j of query q: the exact support test, then
@@ -50,7 +50,7 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
                                        longlong2 pj, const double4_32a &A, const double4_32a &B) {
   constexpr bool gauss = KERNEL == SPH_KERNEL_GAUSSIAN;
   PairGeom geo;
-  if constexpr (FIX) geo = q.wide ? pair_geom_wide(q.x - A.x, q.y - A.y) : pair_geom(q.p, pj, q.fix_s);
+  if constexpr (FIX) geo = q.wide || fix_cut(pj) ? pair_geom_wide(q.x - A.x, q.y - A.y) : pair_geom(q.p, pj, q.fix_s);
   else geo = pair_geom_fp64(q.x - A.x, q.y - A.y);
   const double dx = geo.dx, dy = geo.dy, d2 = geo.d2;
   const bool fluid = !signbit(B.w);
@@ -139,7 +139,7 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
     if (negative_bits(dot)) {
       if constexpr (UH) {
         const double inv = FIX ? rcp_sum_prod(geo.v, c.hb2f, rs, d2, c.hb2) : rcp64((d2 + c.hb2) * rs);
-        S = fma(c.pic * dot, inv, S);
+        S = fma(c.pic * inv, dot, S);
       } else {
         // mu = h v.r / (r^2 + 0.01 h^2), Pi = mu (beta mu - alpha c_ij) / rho_ij
         const double hb = half_exact(q.h + hij);
@@ -257,7 +257,8 @@ __global__ void __launch_bounds__(kPairBlock, G == 8 ? 4 : kPair64Blocks)
     const int W = g.mode == 0 ? 1 : (slow ? g.wide : g.wt);
     const double4_32a A = P.r64a[kq], B = P.r64b[kq];
     const longlong2 *fix = reinterpret_cast<const longlong2 *>(P.rec1);
-    const Query64 q = {A.x, A.y, A.z, A.w, B.y, B.z, B.w, fix[kq], g.fix_s, g.pad_e > 0.5f * (float)g.r_search};
+    const Query64 q = {A.x, A.y, A.z, A.w, B.y, B.z, B.w, fix[kq], g.fix_s,
+                       (kFix && fix_cut(fix[kq])) || g.pad_e > 0.5f * (float)g.r_search};
     Acc64 s;
     // the FP32 test: the padded reach of the pair's h (kernel support; a
     // boundary neighbour without XSPH: the Lennard-Jones reach min(r0, 3 h_ij))
