@@ -567,7 +567,7 @@ void launch_adjoint_step(const StepArgs &s, const StepArgs &h, const WsPtrs &w, 
   ap.alpha = wc.alpha;
   ap.beta = wc.beta;
   ap.co = wc.co;
-  ap.r0 = wc.r0;
+  ap.r0 = lj_reach(wc);
   ap.D = wc.D;
   ap.p1 = wc.p1;
   ap.p2 = wc.p2;

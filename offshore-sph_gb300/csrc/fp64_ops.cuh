@@ -400,6 +400,9 @@ struct Pair64 {
   int lj_free;                 // r0 < 1.5 h: the Lennard-Jones pairs all have q <= 3
 };
 
+// the Lennard-Jones length: r <= r0 has no pair for a negative or NaN r0
+inline double lj_reach(const sph_wcsph_t &wc) { return wc.r0 > 0.0 ? wc.r0 : 0.0; }
+
 inline Pair64 pair64_consts(const sph_config_t &cfg, const sph_wcsph_t &wc) {
   Pair64 c;
   c.xsph = wc.use_xsph != 0;
@@ -444,7 +447,7 @@ inline Pair64 pair64_consts(const sph_config_t &cfg, const sph_wcsph_t &wc) {
   c.l2e = fix64_quot(0x1.71547652b82fep+0, 0x1.777d0ffda0d24p-56, hh, fma(h, h, -hh));  // log2(e) in two parts
   c.scale = cfg.kernel == SPH_KERNEL_CUBIC ? -c.al / hh : (cfg.kernel == SPH_KERNEL_GAUSSIAN ? c.i_0 : 1.0);
   c.pic = -wc.alpha * wc.co * h;  // -2 alpha c_ij h with c_ij = co / 2
-  c.r02 = wc.r0 * wc.r0;
+  c.r02 = lj_reach(wc) * lj_reach(wc);
   c.lj_free = cfg.h_fixed > 0.0 && wc.r0 < 1.5 * h * (1.0 - 1e-9);
   return c;
 }

@@ -323,7 +323,8 @@ static void pair64_launch(const StepArgs &a, const WsPtrs &w, const PairParams &
 }
 
 void launch_pair64(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, const sph_wcsph_t &wc,
-                   const PairParams &pp, double *dt_out, double *dt_hist, cudaStream_t st) {
+                   PairParams pp, double *dt_out, double *dt_hist, cudaStream_t st) {
+  pp.r0 = lj_reach(wc);
   const Pair64 c = pair64_consts(cfg, wc);
   const bool uh = cfg.h_fixed > 0.0 && wc.beta == 0.0;
   auto go = [&](auto kern) {

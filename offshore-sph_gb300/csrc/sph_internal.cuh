@@ -922,7 +922,7 @@ void launch_pair(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, co
                  double *dt_out, double *dt_hist, cudaStream_t st,
                  const WallLoad *wall = nullptr, bool write_state = true);
 void launch_pair64(const StepArgs &a, const WsPtrs &w, const sph_config_t &cfg, const sph_wcsph_t &wc,
-                   const PairParams &pp, double *dt_out, double *dt_hist, cudaStream_t st);
+                   PairParams pp, double *dt_out, double *dt_hist, cudaStream_t st);
 void launch_sum_fixed(const double *v, long long n, double *out, cudaStream_t st);
 void launch_adjoint_step(const StepArgs &s, const StepArgs &h, const WsPtrs &w, const sph_config_t &cfg,
                          const sph_wcsph_t &wc, const sph_adjoint_t &adj, cudaStream_t st);
