@@ -13,15 +13,16 @@ step's evaluation.  The reference has no such diagnostic; it is the
 horizontal force the fluid exerts on that wall.
 
 The forward pass runs the device step (``sph_run_wall_load``) and keeps a
-checkpoint of the state every ``checkpoint`` steps, and for the last segment
-also a copy of the workspace after every step.  The backward pass
-replays each earlier segment from its checkpoint, keeping a copy of the workspace
+checkpoint of the state every ``checkpoint`` steps.  The backward pass
+replays each segment from its checkpoint, keeping a copy of the workspace
 after every replayed step (its neighbour build and FP64 records), and walks
 the segment in reverse with the hand-written adjoint step
 (``sph_adjoint_step``: the vector-Jacobian product of the fused pair
 evaluation and of PEC), which reuses those builds.  The replay of the
 segment before runs on a second stream while the walk runs, into the other
-of two sets of workspace copies.  ``adjoint_precision``
+of two sets of workspace copies.  The last segment's copies come from the
+forward when they take at most ``KEEP_BYTES`` (``_Kept``), so that the
+backward starts on them instead of replaying.  ``adjoint_precision``
 "mixed" runs that product's pair arithmetic in FP32 (the mixed form); the
 forward, the checkpoints and the replay stay FP64, so the loss and its
 finite differences are the FP64 ones.
@@ -29,6 +30,7 @@ The initial density is an input held fixed (it is not recomputed from
 perturbed positions), as are h and the boundary particles.
 """
 import ctypes as C
+import weakref
 
 import numpy as np
 import torch
@@ -41,6 +43,32 @@ from .state import DeviceParticles, DeviceWorkspace, current_stream
 #: the state of a step: what sph_run leaves and the next step reads
 STATE_FIELDS = ("x", "y", "vx", "vy", "rho", "ax", "ay", "drho")
 _STATE_ROWS = [FLOAT_FIELDS.index(k) for k in STATE_FIELDS]
+
+
+#: Largest size of the workspace copies that a forward keeps for its backward
+#: (20 steps of 100K particles; the replay that they save is about 7% of a
+#: forward and backward of 40 steps: 9.29 ms with it, 8.71 without, for 20K
+#: particles).  A loss of a larger scene holds its checkpoints alone, as 20
+#: copies of a 1M-particle workspace are 8 GB.
+KEEP_BYTES = 1 << 30
+
+
+class _Kept:
+    """Workspace copies of a loss's last segment, held from its forward to its
+    first backward or until the loss is gone.  A case has one such set: a later
+    forward of the case takes an earlier loss's set over, and that loss's
+    backward replays its last segment like the others."""
+
+    def __init__(self, bufs, stream):
+        self.slot = [bufs]
+        self.stream = stream
+
+    def take(self):
+        """The copies, or None when they are gone; they are the caller's now."""
+        try:
+            return self.slot.pop()
+        except IndexError:
+            return None
 
 
 class WallLoadCase:
@@ -78,6 +106,7 @@ class WallLoadCase:
         self._rows = torch.tensor(_STATE_ROWS, dtype=torch.int64, device=device)
         # the backward's replays run here, beside the adjoint walk
         self.replay_stream = torch.cuda.Stream(device=device)
+        self._kept = None  # weak reference to the _Kept of the last forward
 
     def wcsph(self, alpha):
         return core.wcsph_struct(self.height, self.r0, self.rho0, alpha=float(alpha))
@@ -117,6 +146,19 @@ class WallLoadCase:
             self.ws.check()
             return self.dt * hist.sum()
 
+    def _keep(self, n):
+        """Room for the workspace copies of n steps (see _Kept)."""
+        stream = torch.cuda.current_stream(self.ws.buf.device)
+        old = self._kept() if self._kept is not None else None
+        bufs = old.take() if old is not None else None
+        if bufs is None or old.stream != stream:
+            bufs = []
+        del bufs[n:]
+        bufs.extend(torch.empty_like(self.ws.buf) for _ in range(n - len(bufs)))
+        kept = _Kept(bufs, stream)
+        self._kept = weakref.ref(kept)
+        return kept, bufs
+
     def snapshot(self, dp):
         return dp._buf[self._rows, :self.n]
 
@@ -128,28 +170,36 @@ class WallLoadLoss(torch.autograd.Function):
     """loss = WallLoadLoss.apply(alpha, pos, vel, case): alpha a 0-d float64
     tensor, pos and vel (n_fluid, 2) float64 CUDA tensors."""
 
+    @classmethod
+    def apply(cls, alpha, pos, vel, case):
+        # the forward runs with gradients disabled, so it is told here whether
+        # a backward can follow
+        return super().apply(alpha, pos, vel, case, torch.is_grad_enabled())
+
     @staticmethod
-    def forward(ctx, alpha, pos, vel, case):
+    def forward(ctx, alpha, pos, vel, case, grad_mode):
         wc = case.wcsph(alpha.item())
         dp = case._start(pos, vel)
         hist = torch.empty(case.nsteps, dtype=torch.float64, device=pos.device)
         ckpts = []
         K = case.checkpoint
-        last = []
+        ctx.kept = None
         for s0 in range(0, case.nsteps, K):
             ckpts.append(case.snapshot(dp))
-            if s0 + K < case.nsteps or not any(ctx.needs_input_grad):
-                case._run(dp, wc, min(K, case.nsteps - s0), hist[s0:])
+            n = min(K, case.nsteps - s0)
+            if (s0 + K < case.nsteps or not grad_mode or not any(ctx.needs_input_grad) or
+                    n * case.ws.buf.numel() > KEEP_BYTES):
+                case._run(dp, wc, n, hist[s0:])
                 continue
             # the last segment step by step (the same state, bit for bit), its
             # builds kept: the backward starts on them instead of replaying
-            for s in range(s0, case.nsteps):
-                case._run(dp, wc, 1, hist[s:])
-                last.append(case.ws.buf.clone())
+            ctx.kept, bufs = case._keep(n)
+            for s in range(n):
+                case._run(dp, wc, 1, hist[s0 + s:])
+                bufs[s].copy_(case.ws.buf)
         case.ws.check()
         ctx.case = case
         ctx.ckpts = ckpts
-        ctx.last = last
         ctx.alpha = alpha.item()
         return case.dt * hist.sum()
 
@@ -170,22 +220,31 @@ class WallLoadLoss(torch.autograd.Function):
         w0 = case.ws.ws
         nseg = len(ctx.ckpts)
         main, side = torch.cuda.current_stream(dev), case.replay_stream
-        side.wait_stream(main)
         # Two sets of K workspace copies: while the adjoint walks segment seg
         # on the main stream (reading set seg % 2), the side stream replays
-        # segment seg - 1 into the other set.  The last segment's copies come
-        # from the forward.  walked[seg]: the main stream has finished reading
-        # segment seg's set.
-        sets = [[torch.empty_like(case.ws.buf) for _ in range(K)] for _ in range(min(2, nseg - 1))]
+        # segment seg - 1 into the other set.  The last segment's set is the
+        # one the forward kept, when it is still there.  walked[seg]: the main
+        # stream has finished reading segment seg's set.
+        kept = ctx.kept.take() if ctx.kept is not None else None
+        if kept is not None and ctx.kept.stream != main:
+            kept = None
+        sets = [[] for _ in range(min(2, nseg))]
+        if kept is not None:
+            sets[(nseg - 1) % 2] = kept
+        for k, bufs in enumerate(sets):
+            # as long as the longest segment that uses the set
+            need = max(min(K, case.nsteps - seg * K) for seg in range(k, nseg, 2))
+            bufs.extend(torch.empty_like(case.ws.buf) for _ in range(need - len(bufs)))
+        side.wait_stream(main)
         walked = [None] * nseg
 
         def replay(seg):
             # after each step the workspace holds that step's neighbour build
             # and FP64 records, which its adjoint reuses; the same step as the
             # forward's without the wall-load output (the state is identical)
-            bufs = sets[seg % len(sets)]
+            bufs = sets[seg % 2]
             with torch.cuda.stream(side):
-                if seg + 2 < nseg - 1:
+                if seg + 2 < nseg:
                     side.wait_event(walked[seg + 2])
                 dp._buf.copy_(case.base._buf)
                 case.restore(dp, ctx.ckpts[seg])
@@ -194,13 +253,13 @@ class WallLoadLoss(torch.autograd.Function):
                     bufs[s].copy_(case.ws.buf)
                 return side.record_event()
 
-        ready = None
+        ready = replay(nseg - 1) if kept is None and nseg > 0 else None
         for seg in reversed(range(nseg)):
             if ready is not None:
                 main.wait_event(ready)
             if seg > 0:
                 ready = replay(seg - 1)
-            bufs = ctx.last if seg == nseg - 1 else sets[seg % len(sets)]
+            bufs = sets[seg % 2]
             for s in reversed(range(min(K, case.nsteps - seg * K))):
                 ws_s = L.Workspace(ptr=bufs[s].data_ptr(), bytes=w0.bytes, n_cap=w0.n_cap, max_cells=w0.max_cells)
                 L.check(lib.sph_adjoint_step(core._P(case.base), core._P(half), C.byref(wc), C.byref(case.cfg_adj),
@@ -208,12 +267,12 @@ class WallLoadLoss(torch.autograd.Function):
             walked[seg] = main.record_event()
         main.wait_stream(side)
         case.ws.check()
-        del sets
+        del sets, kept
         f = case.fluid
         galpha = A["alphab"].sum().reshape(())
         gpos = torch.stack((A["xb"][f], A["yb"][f]), 1)
         gvel = torch.stack((A["vxb"][f], A["vyb"][f]), 1)
-        return galpha, gpos, gvel, None
+        return galpha, gpos, gvel, None, None
 
 
 def gradients(case, alpha, pos=None, vel=None):
