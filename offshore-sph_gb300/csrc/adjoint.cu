@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjBlocks) k_pair_adjoint(AdjPtrs 
 
 // ---------------------------------------------------------------------------
 // Mixed form of the adjoint pair product: the same vector-Jacobian product as
-// adjoint_query with the pair arithmetic in FP32 (hardware reciprocals and
+// k_pair_adjoint with the pair arithmetic in FP32 (hardware reciprocals and
 // square roots) and the per-particle sums in FP32, over the FP64 records of
 // the forward evaluation and the FP64 adjoint vectors.  Differences of FP64
 // positions and velocities are formed in FP64 and then rounded, so large
@@ -580,7 +580,7 @@ void launch_adjoint_step(const StepArgs &s, const StepArgs &h, const WsPtrs &w, 
   ap.dt = dt;
   ap.n = n;
   const Pair64 c = pair64_consts(cfg, wc);
-  const int lanes = lanes_per_query(n);
+  const int lanes = lanes_per_query(n, cfg.kernel, true, true);
   auto go = [&](auto kern, auto l) {
     constexpr int K = decltype(kern)::value, G = decltype(l)::value;
     const unsigned nbp = nblocks(n * G, kAdjBlock);

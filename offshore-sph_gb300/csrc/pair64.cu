@@ -316,7 +316,7 @@ static void pair64_launch(const StepArgs &a, const WsPtrs &w, const PairParams &
     launch_pdl(k_pair64<KERNEL, UH, G>, dim3(nblocks(a.n * G, kPairBlock)), dim3(kPairBlock), 0, st, a, pair_ptrs(w), pp,
                c, dt_out, dt_hist);
   };
-  const int lanes = lanes_per_query(a.n);
+  const int lanes = lanes_per_query(a.n, KERNEL, UH);
   if (lanes == 8) go(std::integral_constant<int, 8>());
   else if (lanes == 4) go(std::integral_constant<int, 4>());
   else go(std::integral_constant<int, 1>());

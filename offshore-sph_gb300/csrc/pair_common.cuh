@@ -223,20 +223,40 @@ __device__ __forceinline__ void group_sum(T &v) {
   for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
 }
 
-// Lanes per query of the FP64 kernels for n particles.  Sharing a query costs
-// about a quarter more issue time (short groups, the final sums; dam break of
-// 1M fluid particles: 1.27 ms with G = 1, 1.57 ms with G = 4, measured like the
-// figures below before the arithmetic moved to the integer pipe) and divides the
-// length of a thread's chain of dependent FP64 operations.  So G = 1 where the
-// threads fill most of one wave of blocks (54K particles, Wendland: 784 us for
-// 4 steps against 817 with G = 4) or several; G = 4 where the last wave would
-// be nearly empty (99K, Gaussian: 356 us with G = 1, 327 with 4, 355 with 8);
-// G = 8 where the GPU is idle and the chain is the time (5K particles: 1393 us
-// for 20 steps with G = 1, 858 with 4, 732 with 8, 793 with 16, 914 with 32).
-inline int lanes_per_query(long long n) {
+// Lanes per query of the FP64 kernels for n particles, and of the adjoint's.
+// Sharing a query divides the length of a thread's chain of dependent operations
+// and costs issue time (short groups, the final sums): 20 to 50% with the cubic's
+// short pairs, 4 to 20% with the others.  By sizes in waves of one query per
+// thread (97,280 queries on 152 SMs), pair stage in us, lattice, cubic with fixed h
+// | Gaussian | Wendland with computed h | FP64 adjoint, cubic:
+//
+//   waves   G = 1                     G = 4                     G = 8
+//   0.05     57 |  92 |  76 |  77      28 |  32 |  29 |  41      18 |  22 |  25 |  31
+//   0.125    56 |  91 |  76 |  78      31 |  36 |  41 |  47      41 |  55 |  54 |  51
+//   0.49     63 | 108 | 119 | 106      60 |  87 | 107 | 110      97 | 130 | 144 | 133
+//   0.56     63 | 106 | 120 | 119      78 | 112 | 129 | 132     112 | 149 | 162 | 168
+//   1.02    118 | 218 | 227 | 226     125 | 172 | 205 | 229     187 | 249 | 271 | 312
+//   1.25    125 | 239 | 248 | 262     136 | 199 | 242 | 282     231 | 305 | 325 | 390
+//   1.75    141 | 271 | 312 | 324     186 | 271 | 331 | 363
+//   2.25    188 | 363 | 406 | 384     236 | 340 | 414 | 442
+//   3.9     274 | 532 | 661           402 | 566 | 694
+//
+// (the adjoint's sizes are 1.16, 1.46, 1.91 and 2.35 from the row of 1.02 on).  So
+// G = 8 where the GPU is idle and the chain is the time, G = 4 up to half a
+// wave, and from there on G = 1 where the last wave is full enough: always with
+// the cubic and Wendland at a fixed h and in the adjoint; the Gaussian's long
+// pairs are worth sharing while the last wave is at most half full, up to 4 waves,
+// and a computed h's in the first quarter of the second wave (cubic at 1.02
+// waves 214 and 193 us).  The Gaussian's adjoint shares up to 4 waves: its mixed
+// form takes 217 us with one lane and 178 with 4 at 1.0 waves, 318 and 303 at
+// 1.8, 418 and 417 at 2.6, and its FP64 form differs by at most 3%.
+inline int lanes_per_query(long long n, int kernel = SPH_KERNEL_CUBIC, bool uniform_h = true, bool adjoint = false) {
   const long long wave = (long long)sm_count() * kPairBlock * kPair64Blocks;
   if (n < wave / 8) return 8;
-  return n < wave / 2 || (n > wave && n < 4 * wave) ? 4 : 1;
+  if (n < wave / 2) return 4;
+  if (n <= wave || n >= 4 * wave) return 1;
+  if (kernel == SPH_KERNEL_GAUSSIAN) return adjoint || n % wave <= wave / 2 ? 4 : 1;
+  return !uniform_h && n <= wave + wave / 4 ? 4 : 1;
 }
 
 // Exact size of the reference's neighbour set of a query whose own cell is
