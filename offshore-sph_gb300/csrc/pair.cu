@@ -302,8 +302,12 @@ __device__ __forceinline__ unsigned long long pair_query(const StepArgs &a, cons
       // slow queries, whose set size is counted exactly
       const bool any = !slow || exact_count(a, P.perm, g, qref, qkey, W, g.mode == 1, P.meta, cst, a.x[i], a.y[i],
                                             a.h[i]) > 0;
-      if (any) ea = mixed_store<XSPH, SUMDENS>(acc, a, i, pp.write_xsph);
-      else ea = enc_d(accel2(a.ax[i], a.ay[i]));  // keeps its previous values (SolverTools.py:150-153)
+      if (any) {
+        ea = mixed_store<XSPH, SUMDENS>(acc, a, i, pp.write_xsph || slow);
+      } else {
+        ea = enc_d(accel2(a.ax[i], a.ay[i]));  // keeps its previous values (SolverTools.py:150-153)
+        if (!XSPH && pp.write_xsph) P.ctrl->xsph_left = 1u;
+      }
     }
   }
   return ea;
@@ -325,8 +329,15 @@ __global__ void __launch_bounds__(kPairBlock, kListBlocks)
   // A block that starts after the last participant emptied the list reads
   // 0 and leaves too: the list is emptied only once every participant,
   // itself included, has read the count.
-  const unsigned int parts = cnt < gridDim.x ? (cnt > 0u ? cnt : 1u) : gridDim.x;
+  const bool left = !XSPH && !pp.write_xsph && P.ctrl->xsph_left;  // set in other steps only
+  const unsigned int parts = !left && cnt < gridDim.x ? (cnt > 0u ? cnt : 1u) : gridDim.x;
   if (blockIdx.x >= parts) return;
+  if (left)
+    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < pp.n; k += (long long)gridDim.x * blockDim.x)
+      if (!signbit(P.rec0[k].z) && P.rec0[k].z > 0.f && P.meta[k].x < P.grid->ncx) {
+        a.xsphx[P.perm[k]] = 0.0;
+        a.xsphy[P.perm[k]] = 0.0;
+      }
   unsigned long long ea = kEncMaxId;
   if (blockIdx.x < cnt) {
     const DevGrid g = *P.grid;

@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(kPairBlock, G == 8 ? 4 : kPair64Blocks)
       if (!slow || exact_count(a, P.perm, g, qref, qkey, W, g.mode == 1, P.meta, P.cstart, q.x, q.y, q.h) > 0) {
         const double axf = s.ax, ayf = s.ay - 9.81;
         a.drho[i] = c.sumdens ? 0.0 : s.dd;
-        if (c.xsph || pp.write_xsph) {
+        if (c.xsph || pp.write_xsph || slow || P.ctrl->xsph_left) {
           a.xsphx[i] = c.xsph ? q.vx + s.sx : 0.0;
           a.xsphy[i] = c.xsph ? q.vy + s.sy : 0.0;
         }
@@ -302,6 +302,7 @@ __global__ void __launch_bounds__(kPairBlock, G == 8 ? 4 : kPair64Blocks)
       } else {
         ea = enc_d(accel2(a.ax[i], a.ay[i]));  // keeps its previous values (SolverTools.py:150-153)
         if (pp.fr) pp.fr[i] = 0.0;
+        if (!c.xsph && pp.write_xsph) P.ctrl->xsph_left = 1u;
       }
     }
   }

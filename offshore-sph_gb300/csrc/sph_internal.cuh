@@ -188,6 +188,10 @@ struct DevCtrl {
   // ones from the front of the tile list, tl_back sparse ones from its back
   unsigned int tl_count, tl_back, tl_heavy;
   unsigned int bounds_done;  // finished blocks of the bounds pass (its last block sets the grid)
+  // a query had no neighbour in a step that writes the XSPH velocity of a run
+  // without XSPH, and kept what it was: from then on the steps between a run's
+  // first and last write it too (the query may have neighbours in one of them)
+  unsigned int xsph_left;
   double dt_ring[2][3];  // {dt, dt_c, dt_f} of the step with that parity
   GridKey grid_key;      // inputs of the grid in use
 };
