@@ -116,3 +116,76 @@ def test_pressure_term():
     want = term(np.longdouble)
     rms = lambda v: np.std((np.abs(v) / want / np.mean(np.abs(v) / want) - 1).astype(np.float64))  # noqa: E731
     assert rms(got["ax"]) <= rms(term(np.float64)) * (1 + 2 / np.sqrt(2 * n)), (rms(got["ax"]), rms(term(np.float64)))
+
+
+@pytest.mark.parametrize("kernel", [CUBIC, GAUSS, WEND])
+@pytest.mark.parametrize("fixed", [True, False])
+@pytest.mark.parametrize("n", [3001, 10007, 35003])
+def test_xsph_of_a_pair(kernel, fixed, n):
+    """The XSPH velocity of the pairs' first halves, which are at rest
+    (XSPH.py:26-31, the kernels' values)."""
+    from sph import build, core, state
+    build.build()
+    h = 0.0325 if fixed else 1.3 * np.sqrt(MASS / 1030.0)
+    pa = _pairs(n, h, kernel, n + kernel)
+    dp = state.DeviceParticles.from_array(pa)
+    dp.h.fill_(h)
+    ws = state.DeviceWorkspace(dp.n)
+    core.compute(dp, core.wcsph_struct(5.0, 0.01, 1000.0, use_xsph=True),
+                 core.config_struct(kernel=kernel, precision="fp64", h_fixed=h if fixed else 0.0), ws)
+    ws.check()
+    got = dp.soa()
+
+    def velocity(F):
+        x, y, vx, rho, hh = (got[k].astype(F) for k in ("x", "y", "vx", "rho", "h"))
+        pi = F("3.14159265358979323846264338327950288") if F is not np.float64 else math.pi
+        dx, dy = x[:n] - x[n:], y[:n] - y[n:]
+        r = np.sqrt(dx * dx + dy * dy)
+        hij = F(0.5) * (hh[:n] + hh[n:])
+        q = r / hij
+        if kernel == CUBIC:
+            w = F(10) / (F(7) * pi) / (hij * hij) * np.where(
+                q > 1, F(0.25) * ((2 - q) * (2 - q) * (2 - q)), 1 - F(1.5) * (q * q) * (1 - F(0.5) * q))
+        elif kernel == WEND:
+            t = 1 - F(0.5) * q
+            w = F(9) / (F(4) * pi) / (hij * hij) * (t * t * t * t * t * t) * (F(35) / F(12) * q * q + 3 * q + 1)
+        else:
+            w = F(1) / pi / (hij * hij) * np.exp(-q * q)
+        return q, -F(0.5) * F(MASS) * w / (F(0.5) * (rho[:n] + rho[n:])) * (vx[:n] - vx[n:])
+    q, want = velocity(np.longdouble)
+    _, fp64 = velocity(np.float64)
+    weight = np.minimum(2 - q, 1) if kernel != GAUSS else np.ones_like(q)
+    ok = q * got["h"].max() < 1.99 * got["h"].min()
+    rms = lambda v: np.sqrt(np.mean((((v - want) / want * weight)[ok]).astype(np.float64) ** 2))  # noqa: E731
+    assert rms(got["xsphx"][:n]) <= rms(fp64) * (1 + 2 / np.sqrt(ok.sum())), (rms(got["xsphx"][:n]), rms(fp64))
+
+
+@pytest.mark.parametrize("n", [3001, 10007, 35003])
+def test_boundary_force_of_a_pair(n):
+    """The Lennard-Jones force of single boundary particles
+    (BoundaryForce.py:6-42)."""
+    from sph import build, core, state
+    build.build()
+    h, r0 = 0.0325, 0.025
+    pa = _pairs(n, h, CUBIC, n)
+    rng = np.random.default_rng(n)
+    r, ang = r0 * rng.uniform(0.3, 0.9, n), rng.uniform(-1.0, 1.0, n)
+    pa["x"][n:], pa["y"][n:] = pa["x"][:n] + r * np.cos(ang), pa["y"][:n] + r * np.sin(ang)
+    pa["label"][n:], pa["m"][n:], pa["vx"][n:], pa["vy"][n:] = 1, 0.0, 0.0, 0.0
+    dp = state.DeviceParticles.from_array(pa)
+    wc = core.wcsph_struct(5.0, r0, 1000.0)
+    ws = state.DeviceWorkspace(dp.n)
+    core.compute(dp, wc, core.config_struct(h_fixed=h), ws)
+    ws.check()
+    got = dp.soa()
+
+    def force(F):
+        x, y = got["x"].astype(F), got["y"].astype(F)
+        dx, dy = x[:n] - x[n:], y[:n] - y[n:]
+        r = np.sqrt(dx * dx + dy * dy)
+        f = F(wc.r0) / r
+        f2 = f * f
+        return F(wc.D) * (f2 * f2 - f2) * dx / (r * r)
+    want = force(np.longdouble)
+    rms = lambda v: np.sqrt(np.mean(((v - want) / want).astype(np.float64) ** 2))  # noqa: E731
+    assert rms(got["ax"][:n]) <= rms(force(np.float64)) * (1 + 2 / np.sqrt(n)), (rms(got["ax"][:n]), rms(force(np.float64)))
