@@ -391,7 +391,7 @@ struct Pair64 {
   double o_t, o_r, o_rl;       // cubic, outer piece: (o_t / r) (2 + o_r r)^2, o_r = -1 / h in two parts
   double i_r, i_0;             // inner piece: i_r r + i_0.  Wendland: (i_r r + i_0) (1 + o_r r)^5, o_r = -1 / (2 h)
   double g_d;                  // Gaussian: -2 / h^2, the gradient factor's derivative over r
-  double scale;                // FIX: of the gradient factor that is summed (cubic: -al / h^2)
+  double scale;                // of the gradient factor that is summed (cubic -al / h^2, Gaussian i_0, Wendland 1)
   Fix64 hf, ihf, hb2f;         // h, 1/h, hb2
   Fix64 l2e;                   // log2(e) / h^2
   double al;                   // normalisation of W

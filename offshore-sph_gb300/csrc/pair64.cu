@@ -8,20 +8,22 @@
 //   - candidates are filtered in FP32 (padded) and compared on the integer
 //     pipe (positive doubles order like their bits);
 //   - position differences and the squared distance come from 64-bit integer
-//     positions, reciprocals and square roots from 64-bit fixed-point Newton
-//     steps, each rounded once.  The neighbour test q = r / h_ij <= 3
+//     positions (except for coordinates that these cut), reciprocals and square
+//     roots from 64-bit fixed-point Newton steps, each rounded once.  The neighbour test q = r / h_ij <= 3
 //     (NNLinkedList.py:74) is redone with correctly rounded operations where
 //     an estimate could decide it differently;
 //   - with a uniform fluid h (Solver(h=...)) and beta = 0, the cubic's gradient
 //     factor and the viscosity's reciprocal are fixed-point too, and boundary
 //     neighbours beyond the Lennard-Jones reach are not listed (without XSPH
 //     they contribute nothing).
-// A pair of the cubic spline so takes 13 FP64 operations instead of about 90.
+// A pair of the cubic spline so takes 11 FP64 operations instead of about 90.
 // 1M-fluid dam break, pair stage: 3.67 ms at 90, 1.27 ms at 31 (Halley steps and
-// launch-constant gradient polynomials in FP64), 0.75 ms now; the FP64 pipe
-// is busy 65% of it and 42% of the issue slots are used.  20 steps of 3200
+// launch-constant gradient polynomials in FP64), 0.66 ms now; the FP64 pipe
+// is busy 62% of it and 44% of the issue slots are used.  20 steps of 3200
 // fluid particles, where latency decides (several lanes per query): 2.40 ms,
-// 0.71 and 0.66.
+// 0.71 and 0.67.
+// A pair's terms are at least as close to the exact ones as the reference's
+// formulas with every operation rounded to 64 bits.
 #include <type_traits>
 
 #include "fp64_ops.cuh"
@@ -60,21 +62,15 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
       if constexpr (gauss) {
         if (!le_bits(d2, c.lim_lo) && (!le_bits(d2, c.lim_hi) || !near_exact(q.x - A.x, q.y - A.y, hij))) return;
         const double e = exp2_neg(geo.v, c.l2e);
-        coef = le_bits(d2, c.h2) ? 0.0 : (FIX ? e : c.i_0 * e);  // FIX: scaled in the sum
+        coef = le_bits(d2, c.h2) ? 0.0 : e;  // scaled in the sum
         if (c.xsph) w = c.al * e;
       } else {
         if (!le_bits(d2, c.lim)) return;  // W and its gradient are 0 at q >= 2
         const bool tiny = le_bits(d2, 1e-20);  // r < 1e-10: no gradient
         double r = 0.0, ir;
-        if (!(FIX && KERNEL == SPH_KERNEL_CUBIC) || c.xsph) sqrt_rsqrt64(geo.v, r, ir);
-        if (FIX && KERNEL == SPH_KERNEL_CUBIC) {
-          coef = cubic_g(geo.v, c.ihf, c.hf);
-        } else if (KERNEL == SPH_KERNEL_CUBIC) {
-          if (le_bits(d2, c.h2)) coef = fma(c.i_r, r, c.i_0);
-          else {
-            const double t = fma(c.o_rl, r, fma(c.o_r, r, 2.0));
-            coef = (c.o_t * ir) * (t * t);
-          }
+        if (KERNEL != SPH_KERNEL_CUBIC || c.xsph) sqrt_rsqrt64(geo.v, r, ir);
+        if (KERNEL == SPH_KERNEL_CUBIC) {
+          coef = cubic_g(geo.v, c.ihf, c.hf);  // scaled in the sum
         } else {
           const double in = fma(c.o_rl, r, fma(c.o_r, r, 1.0)), in2 = in * in;
           coef = (in2 * in2) * (in * fma(c.i_r, r, c.i_0));
@@ -138,7 +134,7 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
     const double rs = q.rho + B.y;  // 2 rho_ij
     if (negative_bits(dot)) {
       if constexpr (UH) {
-        const double inv = FIX ? rcp_sum_prod(geo.v, c.hb2f, rs, d2, c.hb2) : rcp64((d2 + c.hb2) * rs);
+        const double inv = rcp_sum_prod(geo.v, c.hb2f, rs, d2, c.hb2);
         S = fma(c.pic * inv, dot, S);
       } else {
         // mu = h v.r / (r^2 + 0.01 h^2), Pi = mu (beta mu - alpha c_ij) / rho_ij
@@ -233,8 +229,8 @@ __global__ void __launch_bounds__(kPairBlock, G == 8 ? 4 : kPair64Blocks)
     k_pair64(StepArgs a, PairPtrs P, PairParams pp, Pair64 c, double *dt_out, double *dt_hist) {
   step_kernel_entry();
   // Integer differences save FP64 issue time and lengthen a pair's chain: not
-  // where a query's latency is the time (20 steps of 3200 fluid particles 674
-  // us without, 695 with; 4 steps of 1M: 5117 and 4601)
+  // where a query's latency is the time (20 steps of 3200 fluid particles 672
+  // us without, 690 with; 4 steps of 1M: 3737 and 3515)
   constexpr bool kFix = G < 8;
   constexpr int kCap = list_words<G>(ListCap<KERNEL>::value);
   __shared__ unsigned int lists[kCap * kPairBlock / G];
@@ -270,7 +266,7 @@ __global__ void __launch_bounds__(kPairBlock, G == 8 ? 4 : kPair64Blocks)
     for_neighbours<G, kCap, kPairBlock>(sten, P.cstart, act, lists, near, [&](unsigned int j) {
       pair64<KERNEL, UH, kFix>(s, q, c, pp, kFix ? fix[j] : longlong2(), P.r64a[j], P.r64b[j]);
     });
-    if (UH && kFix && KERNEL != SPH_KERNEL_WENDLAND) {
+    if (UH && KERNEL != SPH_KERNEL_WENDLAND) {
       s.dd *= c.scale;
       s.ax *= c.scale;
       s.ay *= c.scale;
