@@ -39,8 +39,8 @@ namespace sph {
 // them evenly
 constexpr int kAdjBlock = 64;
 // resident blocks of the FP64 kernel: the registers' limit that measured
-// fastest (the 20K wall-load case: 9.73 ms at 6, 9.87 at 8, 9.29 at 10, 9.46
-// at 12)
+// fastest (40 steps of the 20K wall-load case: 9.09 ms at 6, 8.93 at 8, 8.70 at
+// 10, 8.77 at 12)
 constexpr int kAdjBlocks = 10;
 
 struct AdjParams {
@@ -111,12 +111,13 @@ struct AdjReach {
   }
 };
 
-// G lanes per query (for_neighbours).  The FP64 pipe bounds it: about 70 FP64
+// G lanes per query (for_neighbours).  The FP64 pipe bounds it: about 50 FP64
 // operations per fluid pair, with the building blocks and launch constants of
 // the forward (pair64.cu).  Listing the pairs first keeps the lanes of a warp
 // together: evaluating each candidate as the walk met it ran 12.5 of 32 lanes
 // on average.  22K particles, one step: 297 us so, 100 us with the pairs listed, 91
-// with the forward's integer arithmetic, 82 with 10 blocks per SM (ncu).
+// with the forward's integer arithmetic, 82 with 10 blocks per SM, 87 with 2 - q
+// formed before it is squared (ncu).
 template <int KERNEL, int G>
 __global__ void __launch_bounds__(kAdjBlock, kAdjBlocks) k_pair_adjoint(AdjPtrs P, AdjParams ap, Pair64 c) {
   constexpr int kCap = list_words<G>(ListCap<KERNEL>::value);

@@ -213,9 +213,9 @@ __device__ void grid_from_bounds(DevCtrl *ctrl, DevGrid *g, const GridParams &gp
 // reductions end in few atomics on the shared bound slots.  The last block
 // to finish sets the grid of the next build from the reduced bounds.
 // bounds_blocks: resident blocks per SM, limited by registers.  Without
-// integrator work 5 fit (an evaluation of 1M particles 257.4 us with 4, 256.7 with 5,
-// 260.1 with 6, where registers spill); with it, 4 (20 steps of 1.03M: 4914 us,
-// 5051 with 5, 5319 with 6).
+// integrator work 5 fit (an evaluation of 1M particles takes 257 us with 3 to 5,
+// within the runs' noise, and 260 with 6, where registers spill); with it, 4 (20
+// steps of 1.03M: 4914 us, 5051 with 5, 5319 with 6).
 constexpr int bounds_blocks(int stage) { return stage == kStageNone ? 5 : 4; }
 template <int INTEG, int STAGE, bool DAMPED, bool XSPH>
 __global__ void __launch_bounds__(kBlock, bounds_blocks(STAGE)) k_bounds(StepArgs a, DevCtrl *ctrl, BoundsParams bp,
