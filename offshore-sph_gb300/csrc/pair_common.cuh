@@ -225,38 +225,45 @@ __device__ __forceinline__ void group_sum(T &v) {
 
 // Lanes per query of the FP64 kernels for n particles, and of the adjoint's.
 // Sharing a query divides the length of a thread's chain of dependent operations
-// and costs issue time (short groups, the final sums): 20 to 50% with the cubic's
-// short pairs, 4 to 20% with the others.  By sizes in waves of one query per
-// thread (97,280 queries on 152 SMs), pair stage in us, lattice, cubic with fixed h
-// | Gaussian | Wendland with computed h | FP64 adjoint, cubic:
+// and costs issue time (short groups, the final sums).  Pair stage in us with 1 and
+// 4 lanes, by sizes in waves of one query per thread (97,280 on 152 SMs); a tank's
+// walls count as queries, which end at once:
 //
-//   waves   G = 1                     G = 4                     G = 8
-//   0.05     57 |  92 |  76 |  77      28 |  32 |  29 |  41      18 |  22 |  25 |  31
-//   0.125    56 |  91 |  76 |  78      31 |  36 |  41 |  47      41 |  55 |  54 |  51
-//   0.49     63 | 108 | 119 | 106      60 |  87 | 107 | 110      97 | 130 | 144 | 133
-//   0.56     63 | 106 | 120 | 119      78 | 112 | 129 | 132     112 | 149 | 162 | 168
-//   1.02    118 | 218 | 227 | 226     125 | 172 | 205 | 229     187 | 249 | 271 | 312
-//   1.25    125 | 239 | 248 | 262     136 | 199 | 242 | 282     231 | 305 | 325 | 390
-//   1.75    141 | 271 | 312 | 324     186 | 271 | 331 | 363
-//   2.25    188 | 363 | 406 | 384     236 | 340 | 414 | 442
-//   3.9     274 | 532 | 661           402 | 566 | 694
+//   lattice  cubic, fixed h  Wendland, fixed h  cubic, computed h  Gaussian
+//   0.05         57  28            64  37             75  39          92  32
+//   0.125        56  31            64  37             75  39          91  36
+//   0.49         63  60            96  92            110 101         108  87
+//   0.52         63  76            96 110            111 115         108 107
+//   1.02        118 125           187 189            214 193         218 172
+//   1.25        125 136           201 212            230 228         239 199
+//   1.5         132 161           223 251            256 269         253 235
+//   2.25        188 236           324 369            371 388         363 340
+//   3.9         274 402           527 634            603 648         532 566
+//   tank
+//   0.97         81 108           151 167            171 192         155 177
+//   1.07        117 123           190 179            219 206         221 190
+//   1.2         130 131           238 205            272 236         277 217
+//   1.4         137 154           256 241            287 278         278 252
+//   1.75        143 184           267 287            302 329         286 301
+//   2.25        190 233           338 364            383 417         405 381
 //
-// (the adjoint's sizes are 1.16, 1.46, 1.91 and 2.35 from the row of 1.02 on).  So
-// G = 8 where the GPU is idle and the chain is the time, G = 4 up to half a
-// wave, and from there on G = 1 where the last wave is full enough: always with
-// the cubic and Wendland at a fixed h and in the adjoint; the Gaussian's long
-// pairs are worth sharing while the last wave is at most half full, up to 4 waves,
-// and a computed h's in the first quarter of the second wave (cubic at 1.02
-// waves 214 and 193 us).  The Gaussian's adjoint shares up to 4 waves: its mixed
-// form takes 217 us with one lane and 178 with 4 at 1.0 waves, 318 and 303 at
-// 1.8, 418 and 417 at 2.6, and its FP64 form differs by at most 3%.
+// With 8 lanes: cubic, fixed h 18, 41 and 97 at 0.05, 0.125 and 0.5.  So G = 8
+// where the GPU is idle and the chain is the time, G = 4 up to half a wave, and
+// from there on G = 1 where the last wave is full enough: always with the cubic
+// at a fixed h, whose pairs are short; the Gaussian's long pairs are worth sharing
+// while the last wave is at most half full, up to 4 waves, and the other forms'
+// in the first three eighths of the second wave.  The adjoint (cubic, FP64: 204
+// and 207 us at 1.03 waves, 263 and 282 at 1.46; mixed 123 and 161 at 1.46) does
+// not share, but for the Gaussian's: mixed, 217 and 178 us at 1.0 waves, 318 and
+// 303 at 1.8, 418 and 417 at 2.6, its FP64 form within 3%.
 inline int lanes_per_query(long long n, int kernel = SPH_KERNEL_CUBIC, bool uniform_h = true, bool adjoint = false) {
   const long long wave = (long long)sm_count() * kPairBlock * kPair64Blocks;
   if (n < wave / 8) return 8;
   if (n < wave / 2) return 4;
   if (n <= wave || n >= 4 * wave) return 1;
   if (kernel == SPH_KERNEL_GAUSSIAN) return adjoint || n % wave <= wave / 2 ? 4 : 1;
-  return !uniform_h && n <= wave + wave / 4 ? 4 : 1;
+  if (adjoint || (kernel == SPH_KERNEL_CUBIC && uniform_h)) return 1;
+  return n <= wave + 3 * wave / 8 ? 4 : 1;
 }
 
 // Exact size of the reference's neighbour set of a query whose own cell is
