@@ -323,13 +323,15 @@ __global__ void __launch_bounds__(kPairBlock, kListBlocks)
                 double *dt_hist) {
   step_kernel_entry();
   __shared__ unsigned int lists[ListCap<KERNEL>::value][kPairBlock];
-  const unsigned int cnt = *(volatile unsigned int *)&P.ctrl->fb_count;
+  const unsigned long long both = *(volatile unsigned long long *)&P.ctrl->fb_count;
+  const unsigned int cnt = (unsigned int)both;
+  // xsph_left, which is set in other steps only
+  const bool left = !XSPH && !pp.write_xsph && (both >> 32) != 0ull;
   // only the blocks that have entries take part (at least block 0, which
   // finishes the TimeStep when the list is empty); the rest leave at once.
   // A block that starts after the last participant emptied the list reads
   // 0 and leaves too: the list is emptied only once every participant,
   // itself included, has read the count.
-  const bool left = !XSPH && !pp.write_xsph && P.ctrl->xsph_left;  // set in other steps only
   const unsigned int parts = !left && cnt < gridDim.x ? (cnt > 0u ? cnt : 1u) : gridDim.x;
   if (blockIdx.x >= parts) return;
   if (left)

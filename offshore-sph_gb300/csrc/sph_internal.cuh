@@ -182,20 +182,23 @@ struct DevCtrl {
   // pair-kernel scheduling: next tile chunk and finished blocks of the tile
   // kernel; entries and finished blocks of the fallback list
   unsigned int tile_next, tile_done;
-  unsigned int fb_count, fb_done;
+  alignas(8) unsigned int fb_count;
+  // (read with fb_count in one load) a query had no neighbour in a step that
+  // writes the XSPH velocity of a run without XSPH, and kept what it was: from
+  // then on the steps between a run's first and last write it too (the query may
+  // have neighbours in one of them)
+  unsigned int xsph_left;
+  unsigned int fb_done;
   // non-empty tiles listed by the build (single-scene build): tl_heavy dense
   // tiles holding a boundary particle in their own list, tl_count other dense
   // ones from the front of the tile list, tl_back sparse ones from its back
   unsigned int tl_count, tl_back, tl_heavy;
   unsigned int bounds_done;  // finished blocks of the bounds pass (its last block sets the grid)
-  // a query had no neighbour in a step that writes the XSPH velocity of a run
-  // without XSPH, and kept what it was: from then on the steps between a run's
-  // first and last write it too (the query may have neighbours in one of them)
-  unsigned int xsph_left;
   double dt_ring[2][3];  // {dt, dt_c, dt_f} of the step with that parity
   GridKey grid_key;      // inputs of the grid in use
 };
 
+static_assert(offsetof(DevCtrl, xsph_left) == offsetof(DevCtrl, fb_count) + 4, "k_pair_list reads both at once");
 // the bound slots are consecutive (k_bounds indexes them from xmin)
 static_assert(offsetof(DevCtrl, xmax) == offsetof(DevCtrl, xmin) + 8 &&
                   offsetof(DevCtrl, ymin) == offsetof(DevCtrl, xmin) + 16 &&
