@@ -271,6 +271,23 @@ __device__ __forceinline__ unsigned long long square_hi(unsigned long long u) {
   return (unsigned long long)u1 * u1 + (((unsigned long long)u1 * u0) >> 31);
 }
 
+// q = r / h from the pair's squared distance, y = 1 / sqrt(v) and ih = 1 / h, in
+// units of 2^-61; q < 2 + 2^-40
+__device__ __forceinline__ unsigned long long q_q61(const Quad64 &v, unsigned long long y, const Fix64 &ih) {
+  // r = s 2^k, s in [1, 2) in units of 2^-61; q = (s ih.m) 2^(k + ih.e), the product in [1, 4)
+  return mul_hi(sqrt_q61(v, y) << 2, ih.m << 1) >> min(max(1 - v.k - ih.e, 0), 63);
+}
+
+// 1 - q / 2 for the Wendland kernel, 0 from q = 2 on: an exact difference of
+// integers, rounded once
+__device__ __forceinline__ double wendland_in(const Quad64 &v, const Fix64 &ih) {
+  const unsigned long long q = q_q61(v, rsqrt_q63(v), ih);  // units of 2^-62 for q / 2
+  if (q >= 1ull << 62) return 0.0;
+  const unsigned long long t = (1ull << 62) - q;
+  const int n = __clzll((long long)t);
+  return pack64<10>(t << (n - 1), 1024 - n);
+}
+
 // g(q) of the cubic spline's gradient factor -(al / h^2) g, q = r / h:
 // 3 - 2.25 q for q <= 1, 0.75 (2 - q)^2 / q up to 2, from the pair's squared
 // distance and ih = 1 / h, h; q < 2 + 2^-40.  Fixed point.  2 - q is an exact
@@ -279,9 +296,7 @@ __device__ __forceinline__ unsigned long long square_hi(unsigned long long u) {
 // 3 / q + 0.75 q - 3, it cancels there: 2e-8 off at q = 1.9999).
 __device__ __forceinline__ double cubic_g(const Quad64 &v, const Fix64 &ih, const Fix64 &h) {
   const unsigned long long y = rsqrt_q63(v);
-  // q = r ih in units of 2^-61: r = s 2^k, s in [1, 2) in units of 2^-61
-  const int sq = v.k + ih.e;  // q = (s ih.m) 2^sq, the product in [1, 4)
-  const unsigned long long q = mul_hi(sqrt_q61(v, y) << 2, ih.m << 1) >> min(max(1 - sq, 0), 63);
+  const unsigned long long q = q_q61(v, y, ih);
   constexpr unsigned long long one = 1ull << 61;
   unsigned long long g;  // the result is g 2^(e - 1086)
   int e;
@@ -389,9 +404,9 @@ struct Pair64 {
   double lim_lo, lim_hi;       // Gaussian: below / above, q <= 3 is decided
   double h2;                   // cubic: d2 <= h^2 is the inner piece.  Gaussian: d2 <= h2 has no gradient
   double o_t, o_r, o_rl;       // cubic, outer piece: (o_t / r) (2 + o_r r)^2, o_r = -1 / h in two parts
-  double i_r, i_0;             // inner piece: i_r r + i_0.  Wendland: (i_r r + i_0) (1 + o_r r)^5, o_r = -1 / (2 h)
+  double i_r, i_0;             // inner piece: i_r r + i_0.  Wendland: (i_r r + i_0) in^5, in = 1 + o_r r, o_r = -1 / (2 h)
   double g_d;                  // Gaussian: -2 / h^2, the gradient factor's derivative over r
-  double scale;                // of the gradient factor that is summed (cubic -al / h^2, Gaussian i_0, Wendland 1)
+  double scale;                // of the gradient factor that is summed (cubic -al / h^2, Gaussian and Wendland i_0)
   Fix64 hf, ihf, hb2f;         // h, 1/h, hb2
   Fix64 l2e;                   // log2(e) / h^2
   double al;                   // normalisation of W
@@ -445,7 +460,7 @@ inline Pair64 pair64_consts(const sph_config_t &cfg, const sph_wcsph_t &wc) {
   c.ihf = fix64_quot(1.0, 0.0, h, 0.0);
   c.hb2f = fix64(c.hb2);
   c.l2e = fix64_quot(0x1.71547652b82fep+0, 0x1.777d0ffda0d24p-56, hh, fma(h, h, -hh));  // log2(e) in two parts
-  c.scale = cfg.kernel == SPH_KERNEL_CUBIC ? -c.al / hh : (cfg.kernel == SPH_KERNEL_GAUSSIAN ? c.i_0 : 1.0);
+  c.scale = cfg.kernel == SPH_KERNEL_CUBIC ? -c.al / hh : c.i_0;
   c.pic = -wc.alpha * wc.co * h;  // -2 alpha c_ij h with c_ij = co / 2
   c.r02 = lj_reach(wc) * lj_reach(wc);
   c.lj_free = cfg.h_fixed > 0.0 && wc.r0 < 1.5 * h * (1.0 - 1e-9);

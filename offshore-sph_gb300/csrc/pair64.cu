@@ -67,28 +67,25 @@ __device__ __forceinline__ void pair64(Acc64 &s, const Query64 &q, const Pair64 
       } else {
         if (!le_bits(d2, c.lim)) return;  // W and its gradient are 0 at q >= 2
         const bool tiny = le_bits(d2, 1e-20);  // r < 1e-10: no gradient
-        double r = 0.0, ir;
-        if (KERNEL != SPH_KERNEL_CUBIC || c.xsph) sqrt_rsqrt64(geo.v, r, ir);
         if (KERNEL == SPH_KERNEL_CUBIC) {
           coef = cubic_g(geo.v, c.ihf, c.hf);  // scaled in the sum
-        } else {
-          const double in = fma(c.o_rl, r, fma(c.o_r, r, 1.0)), in2 = in * in;
-          coef = (in2 * in2) * (in * fma(c.i_r, r, c.i_0));
-        }
-        if (tiny) {
-          coef = 0.0;
-          r = 0.0;
-        }
-        if (c.xsph) {
-          const double qq = r * ih;
-          if (KERNEL == SPH_KERNEL_CUBIC) {
-            const double t = fma(c.o_rl, r, fma(c.o_r, r, 2.0));
+          if (c.xsph) {
+            double r, ir;
+            sqrt_rsqrt64(geo.v, r, ir);
+            if (tiny) r = 0.0;
+            const double qq = r * ih, t = fma(c.o_rl, r, fma(c.o_r, r, 2.0));
             w = le_bits(d2, c.h2) ? c.al * (1.0 - 1.5 * (qq * qq) * (1.0 - 0.5 * qq)) : c.al * 0.25 * (t * t * t);
-          } else {
-            const double in = fma(c.o_rl, r, fma(c.o_r, r, 1.0)), in2 = in * in;
+          }
+        } else {
+          // (1 + 2.5 q) = 6 - 5 in
+          const double in = wendland_in(geo.v, c.ihf), in2 = in * in;
+          coef = (in2 * in2) * (in * fma(-5.0, in, 6.0));  // scaled in the sum
+          if (c.xsph) {
+            const double qq = fma(-2.0, in, 2.0);
             w = c.al * (in2 * in2 * in2 * ((35.0 / 12.0) * qq * qq + 3.0 * qq + 1.0));
           }
         }
+        if (tiny) coef = 0.0;
       }
     } else {
       hij = half_exact(q.h + B.w);  // both positive or zero
@@ -266,7 +263,7 @@ __global__ void __launch_bounds__(kPairBlock, G == 8 ? 4 : kPair64Blocks)
     for_neighbours<G, kCap, kPairBlock>(sten, P.cstart, act, lists, near, [&](unsigned int j) {
       pair64<KERNEL, UH, kFix>(s, q, c, pp, kFix ? fix[j] : longlong2(), P.r64a[j], P.r64b[j]);
     });
-    if (UH && KERNEL != SPH_KERNEL_WENDLAND) {
+    if (UH) {
       s.dd *= c.scale;
       s.ax *= c.scale;
       s.ay *= c.scale;
