@@ -230,29 +230,30 @@ __device__ __forceinline__ void group_sum(T &v) {
 // walls count as queries, which end at once:
 //
 //   lattice  cubic, fixed h  Wendland, fixed h  cubic, computed h  Gaussian
-//   0.05         57  28            64  37             75  39          92  32
-//   0.125        56  31            64  37             75  39          91  36
-//   0.49         63  60            96  92            110 101         108  87
-//   0.52         63  76            96 110            111 115         108 107
-//   1.02        118 125           187 189            214 193         218 172
-//   1.25        125 136           201 212            230 228         239 199
-//   1.5         132 161           223 251            256 269         253 235
-//   2.25        188 236           324 369            371 388         363 340
-//   3.9         274 402           527 634            603 648         532 566
+//   0.05         56  28            57  29             75  31          91  34
+//   0.12         55  31            56  32             76  40          91  38
+//   0.49         65  60            72  70            110 101         109  88
+//   0.52         64  76            71  88            110 116         109 108
+//   1.02        117 124           140 146            214 195         220 174
+//   1.25        125 136           152 158            231 230         242 201
+//   1.5         131 162           165 187            256 270         250 237
+//   2.25        188 236           235 276            372 391         363 344
+//   3.9         272 403           352 475            603 652         533 570
 //   tank
-//   0.97         81 108           151 167            171 192         155 177
-//   1.07        117 123           190 179            219 206         221 190
-//   1.2         130 131           238 205            272 236         277 217
-//   1.4         137 154           256 241            287 278         278 252
-//   1.75        143 184           267 287            302 329         286 301
-//   2.25        190 233           338 364            383 417         405 381
+//   0.97         81 108           101 126            171 192         156 178
+//   1.07        117 123           138 141            222 204         227 190
+//   1.2         131 131           173 154            275 235         274 216
+//   1.4         136 154           179 181            288 278         280 252
+//   1.75        141 183           182 214            301 329         286 302
+//   2.25        189 232           247 272            375 418         406 381
 //
 // With 8 lanes: cubic, fixed h 18, 41 and 97 at 0.05, 0.125 and 0.5.  So G = 8
 // where the GPU is idle and the chain is the time, G = 4 up to half a wave, and
 // from there on G = 1 where the last wave is full enough: always with the cubic
 // at a fixed h, whose pairs are short; the Gaussian's long pairs are worth sharing
-// while the last wave is at most half full, up to 4 waves, and the other forms'
-// in the first three eighths of the second wave.  The adjoint (cubic, FP64: 204
+// while the last wave is at most half full, up to 4 waves, those of a computed h
+// in the first three eighths of the second wave, and Wendland's at a fixed h in
+// the first quarter.  The adjoint (cubic, FP64: 204
 // and 207 us at 1.03 waves, 263 and 282 at 1.46; mixed 123 and 161 at 1.46) does
 // not share, but for the Gaussian's: mixed, 217 and 178 us at 1.0 waves, 318 and
 // 303 at 1.8, 418 and 417 at 2.6, its FP64 form within 3%.
@@ -263,7 +264,7 @@ inline int lanes_per_query(long long n, int kernel = SPH_KERNEL_CUBIC, bool unif
   if (n <= wave || n >= 4 * wave) return 1;
   if (kernel == SPH_KERNEL_GAUSSIAN) return adjoint || n % wave <= wave / 2 ? 4 : 1;
   if (adjoint || (kernel == SPH_KERNEL_CUBIC && uniform_h)) return 1;
-  return n <= wave + 3 * wave / 8 ? 4 : 1;
+  return n <= wave + (uniform_h ? 2 : 3) * wave / 8 ? 4 : 1;
 }
 
 // Exact size of the reference's neighbour set of a query whose own cell is

@@ -35,14 +35,14 @@ def _lanes(n, wave, kernel=CUBIC, fixed=True, adjoint=False):
         return 4 if adjoint or n % wave <= wave // 2 else 1
     if adjoint or (kernel == CUBIC and fixed):
         return 1
-    return 4 if n <= wave + 3 * wave // 8 else 1
+    return 4 if n <= wave + (2 if fixed else 3) * wave // 8 else 1
 
 
 # (kernel, fixed h, XSPH, edge in eighths of a wave, n at the edge less the edge):
 # the last size on one side and the first on the other
 EDGES = [(k, f, x, e, -1) for k, f, x in ((CUBIC, True, False), (CUBIC, False, True), (GAUSS, True, True),
                                           (WEND, False, False), (WEND, True, True)) for e in (1, 4)]
-EDGES += [(CUBIC, False, True, 8, 0), (CUBIC, False, False, 11, 0), (WEND, False, True, 11, 0), (WEND, True, False, 11, 0),
+EDGES += [(CUBIC, False, True, 8, 0), (CUBIC, False, False, 11, 0), (WEND, False, True, 11, 0), (WEND, True, False, 10, 0),
           (GAUSS, True, False, 8, 0), (GAUSS, False, True, 12, 0), (GAUSS, True, True, 16, -1), (GAUSS, True, False, 28, 0)]
 
 
