@@ -47,7 +47,7 @@ TRAFFIC_FROM_PROFILE = {("dambreak1m", "mixed"): (63.5, "2026-12-05, k_pair_tile
 # what bounds the pair kernel instead of HBM, read off the same captures
 LIMITER_FROM_PROFILE = {"mixed": "instruction issue and the shared-memory pipe: 60.3% of active cycles issue, "
                                  "L1tex 77.4% of peak, DRAM 6.4% of peak (ncu, 2026-12-05)",
-                        "fp64": "latency at 20 warps per SM and the FP64 pipe: busy 64.7% of active cycles, DRAM 2.4% of "
+                        "fp64": "latency at 20 warps per SM and the FP64 pipe: busy 62.8% of active cycles, DRAM 2.5% of "
                                 "peak (ncu, 2026-12-05)"}
 
 

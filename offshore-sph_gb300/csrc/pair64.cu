@@ -18,8 +18,8 @@
 //     they contribute nothing).
 // A pair of the cubic spline so takes 11 FP64 operations instead of about 90.
 // 1M-fluid dam break, pair stage: 3.67 ms at 90, 1.27 ms at 31 (Halley steps and
-// launch-constant gradient polynomials in FP64), 0.66 ms now; the FP64 pipe
-// is busy 62% of it and 44% of the issue slots are used.  20 steps of 3200
+// launch-constant gradient polynomials in FP64), 0.65 ms now; the FP64 pipe
+// is busy 63% of it and 44% of the issue slots are used.  20 steps of 3200
 // fluid particles, where latency decides (several lanes per query): 2.40 ms,
 // 0.71 and 0.67.
 // A pair's terms are at least as close to the exact ones as the reference's

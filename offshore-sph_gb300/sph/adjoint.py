@@ -47,7 +47,7 @@ _STATE_ROWS = [FLOAT_FIELDS.index(k) for k in STATE_FIELDS]
 
 #: Largest size of the workspace copies that a forward keeps for its backward
 #: (20 steps of 130K particles; the replay that they save is about 7% of a
-#: forward and backward of 40 steps: 9.33 ms with it, 8.71 without, for 20K
+#: forward and backward of 40 steps: 9.26 ms with it, 8.63 without, for 20K
 #: particles).  A loss of a larger scene holds its checkpoints alone, as 20
 #: copies of a 1M-particle workspace are 8 GB.
 KEEP_BYTES = 1 << 30
